@@ -57,6 +57,7 @@ struct nbk_batch {
     TreeView v{};
     v.pos = arr.pos;
     v.posf = arr.posf;
+    v.posr = arr.posr;
     v.vel = arr.vel;
     v.perm = arr.perm;
     v.node = arr.node;
@@ -88,6 +89,7 @@ __global__ void k_maxabs(const double* p, int64_t n3, unsigned long long* out) {
 void free_arrays(nbk_batch* B) {
   dev_free(B->arr.pos, B->st);
   dev_free(B->arr.posf, B->st);
+  dev_free(B->arr.posr, B->st);
   dev_free(B->arr.perm, B->st);
   dev_free(B->arr.node, B->st);
   dev_free(B->arr.nodex, B->st);
@@ -162,6 +164,7 @@ int batch_build(nbk_batch* B, int b) {
   cudaStream_t st = B->st;
   NBK_TRY(dev_malloc((void**)&B->arr.pos, sizeof(P4) * std::max<int64_t>(n, 1), st));
   NBK_TRY(dev_malloc((void**)&B->arr.posf, sizeof(float4) * std::max<int64_t>(n, 1), st));
+  NBK_TRY(dev_malloc((void**)&B->arr.posr, sizeof(float4) * std::max<int64_t>(n, 1), st));
   NBK_TRY(dev_malloc((void**)&B->arr.perm, sizeof(int) * std::max<int64_t>(n, 1), st));
   NBK_TRY(dev_malloc((void**)&B->arr.node, sizeof(NodeRec) * std::max<int64_t>(nb, 1), st));
   NBK_TRY(dev_malloc((void**)&B->arr.nodex, sizeof(NodeX) * std::max<int64_t>(nb, 1), st));

@@ -1161,6 +1161,7 @@ struct PartOut {
   V4* vel;
   int* perm;
   float4* velf;  // ND = 6 only
+  float4* posr;  // ND = 3 only
 };
 
 template <int ND>
@@ -1453,8 +1454,13 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_build(
     p.z = cc[2 * K + q];
     p.m = m;
     po.pos[t] = p;
-    po.posf[t] = make_float4(__double2float_rn(p.x), __double2float_rn(p.y),
-                             __double2float_rn(p.z), 0.f);
+    const float4 f = make_float4(__double2float_rn(p.x), __double2float_rn(p.y),
+                                 __double2float_rn(p.z), 0.f);
+    po.posf[t] = f;
+    if (ND == 3)
+      po.posr[t] = make_float4(__double2float_rn(dsub(p.x, (double)f.x)),
+                               __double2float_rn(dsub(p.y, (double)f.y)),
+                               __double2float_rn(dsub(p.z, (double)f.z)), 0.f);
     po.perm[t] = ii;
     if (ND == 6) {
       po.vel[t] = make_v4(cc[3 * K + q], cc[4 * K + q], cc[5 * K + q], 0.0);
@@ -1830,7 +1836,7 @@ int build_forest(const std::vector<TreeSpec>& trees, int b, const double* d_pos_
                  const double* d_mass_in, const double* d_vel_in, BuiltArrays& out,
                  DevAlloc& alloc, cudaStream_t st, NodeX* root_out) {
   NodeOut<3> no{out.node, out.nodex};
-  PartOut<3> po{out.pos, out.posf, out.vel, out.perm, nullptr};
+  PartOut<3> po{out.pos, out.posf, out.vel, out.perm, nullptr, out.posr};
   const void* src = trees.empty() ? nullptr : (const void*)(out.nodex + trees[0].nbase);
   return build_forest_t<3>(trees, b, d_pos_in, d_mass_in, d_vel_in, no, po, alloc, st, root_out,
                            sizeof(NodeX), src);
@@ -1844,7 +1850,7 @@ int build_forest_phase(const std::vector<TreeSpec>& trees, int b, const double* 
     return NBK_ERR_INVALID;
   }
   NodeOut<6> no{out.nodes6, out.nodeb6, out.nodef6};
-  PartOut<6> po{out.pos, out.posf, out.vel, out.perm, out.velf};
+  PartOut<6> po{out.pos, out.posf, out.vel, out.perm, out.velf, nullptr};
   const void* src = trees.empty() ? nullptr : (const void*)(out.nodeb6 + trees[0].nbase);
   return build_forest_t<6>(trees, b, d_pos_in, d_mass_in, d_vel_in, no, po, alloc, st, root_out,
                            sizeof(NodeB6), src);

@@ -113,18 +113,20 @@ static int cached_kernel(int kerntype, int kernres, int nd, const KernelEntry** 
   return NBK_OK;
 }
 
-// Device image of a kernel table: [T | A | B] with W(q) = A[i] + B[i] q on cell i, the
+// Device image of a kernel table: [T | A | B | D] with W(q) = A[i] + B[i] q on cell i, the
 // same line through T[i] and T[i+1] as the reference's interpolation (one FMA per
-// neighbour instead of a division and five more operations).
+// neighbour instead of a division and five more operations), and D[i] = T[i+1] - T[i] the
+// line's slope in the table coordinate u = q / delta.
 void kernel_device_image(const std::vector<double>& T, std::vector<double>& img) {
   int kr = (int)T.size();
   double delta = 2.0 / (double)(kr - 1), inv_delta = 0.5 * (double)(kr - 1);
-  img.assign(3 * (size_t)kr, 0.0);
+  img.assign(4 * (size_t)kr, 0.0);
   for (int i = 0; i < kr; i++) {
     img[i] = T[i];
     double slope = i + 1 < kr ? (T[i + 1] - T[i]) * inv_delta : 0.0;
     img[kr + i] = T[i] - slope * (delta * i);
     img[2 * kr + i] = slope;
+    img[3 * kr + i] = i + 1 < kr ? T[i + 1] - T[i] : 0.0;
   }
 }
 
@@ -375,6 +377,7 @@ struct nbk_tree {
     TreeView v{};
     v.pos = arr.pos;
     v.posf = arr.posf;
+    v.posr = arr.posr;
     v.vel = arr.vel;
     v.perm = arr.perm;
     v.node = arr.node;
@@ -761,6 +764,7 @@ int nbk_create(const double* pos, const double* vel, const double* mass, int64_t
     size_t zeroed = block_bytes(parts);
     parts.push_back({(void**)&A.pos, sizeof(P4) * n});
     parts.push_back({(void**)&A.posf, sizeof(float4) * n});
+    if (!phs) parts.push_back({(void**)&A.posr, sizeof(float4) * n});
     parts.push_back({(void**)&A.perm, sizeof(int) * n});
     if (vel) parts.push_back({(void**)&A.vel, sizeof(V4) * n});
     if (phs) {
@@ -955,6 +959,7 @@ int nbk_knn(nbk_tree* t, int k, int variant, int periodic_mode, int32_t* nn, dou
   a.nq = (int)t->n;
   a.nn = dnn;
   a.d2 = dd2;
+  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, kEpiNN, t->st));
   NBK_TRY(S.finish());
   if (!t->dev()) NBK_TRY(check_err(t, "nbk_knn"));
@@ -1186,6 +1191,7 @@ static int density_common(nbk_tree* t, int k, int nsmooth, double* rho, double* 
   a.nsmooth = nsmooth;
   a.rho = trho;
   a.vden = tv;
+  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, epi, t->st));
   if (rho) NBK_TRY(scatter_to_input_order(trho, t->arr.perm, drho, t->n, 1, t->st));
   if (vden) NBK_TRY(scatter_to_input_order(tv, t->arr.perm, dv, t->n, 1, t->st));
@@ -1905,6 +1911,7 @@ int nbk_density_adjoint(nbk_tree* t, int k, const double* w, double* rho, double
   a.nq = (int)t->n;
   a.rho = trho;
   a.nn = nn;
+  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, kEpiDensSave, t->st));
   k_gather_d<<<(unsigned)((t->n + 255) / 256), 256, 0, t->st>>>(dw, t->arr.perm, tw, t->n);
   note_launch();

@@ -1,0 +1,970 @@
+// k-nearest-neighbour search of every particle of a tree, a compact group of particles per
+// warp: the kNN behind CalcDensity, CalcVelDensity and FindNearest of all particles
+// (KDTree::FindNearest(Int_t**, ...) and the loops of KDCalcSmoothQuantities.cxx:203-389).
+//
+// What bounds it, and why groups: with a warp per query (knn_wq.cuh) every query walks the
+// tree alone, about 4,200 warp instructions a query at k = 32, most of them traversal and
+// the sorted insertion of candidates that do not survive. Particles next to one another in
+// tree order have nearly the same neighbourhood, so here one warp walks the tree once for a
+// group of up to G particles, with a radius guessed from the density of the smallest node
+// around the group with more than K particles, stages the particles within that radius of
+// the group's box in shared memory, and every query only screens the staged ones, 32 lanes
+// wide, keeping those within the radius in a buffer of its own. The K nearest are then found
+// by selection (bisection over the FP32 squared distances), not by sorted insertion.
+//
+// Precision of the screen: a particle's coordinates are staged relative to the group's
+// middle particle, as (hi - hi_c) + (lo - lo_c) from the FP32 copy posf (hi) and its FP32
+// residual posr (lo). The error of a difference of two such offsets is bounded by a few
+// 2^-23 of the offsets themselves (not of the coordinates), so the FP32 squared distance s
+// and the true distance d satisfy |sqrt(s) - d| <= E + 2^-20 sqrt(s) with E of the order
+// of 1e-6 of the group's extent, and the selection leaves the K nearest and hardly ever
+// anything else; where it leaves more, FP64 distances (the reference's association
+// ((dx*dx + dy*dy) + dz*dz)) decide.
+//
+// A query that this cannot answer exactly -- fewer than K particles within the radius, a
+// candidate not provably at a non-zero distance (the target search skips zero distances,
+// KDLeafNode.cxx:19-21), more candidates than the buffer holds within the rounding of the
+// K-th, distances outside the FP32 range, a periodic query whose image gates could open --
+// and every query of a group whose box meets too many particles is appended to a list that
+// a second launch serves with the warp-per-query search.
+//
+// The FP64 pipe (two operations per SM clock: 16 cycles a warp instruction) is the bound of
+// the density sums. Per neighbour 12 FP64 instructions are left: 6 for the distance (fused;
+// nothing is decided by it), 2 for the square root, 1 each for the table coordinate, the
+// table line, the gathered and the scattered term. What belongs to a query and not to a
+// neighbour (1/h, h^-3, products with the mass) is computed for all queries of the group at
+// once, a lane per query, and the gathered terms are summed through shared memory, so these
+// cost a group what they would cost one query.
+//
+// Measured (2^20 clustered particles, one GB300; the warp-per-query form in brackets):
+// CalcDensity(32) 3.1 ms (6.0), 32768 uniform 0.098 ms (0.178), 256^3 with k = 64 70 + 69 ms
+// (166 + 176). Groups of 16 took 4.0 ms (18 instead of 32 warps per SM), radii of 1.2 and
+// 1.3 as the first 3.3; everything inlined 5.7 ms (instruction cache); first-pass failures
+// and mixed groups left to the second launch 4.6 ms.
+#include <algorithm>
+
+#include "knn_wq.cuh"
+
+namespace nbk {
+namespace {
+
+constexpr int kGrpChunk = 64;   // candidates staged before the queries screen them
+constexpr int kGrpStack = 192;  // frontier stack (node indices) per warp
+constexpr int kGrpWpb = 4;      // warps (groups) per block
+constexpr int kGrpSlack = 3;    // entries beyond the K-th a buffer cut may leave
+constexpr int kGrpStrict = 256;    // a group that stages more tests nodes query by query
+constexpr int kGrpStaged = 12288;  // and one that stages more takes the second launch
+// search radius of each pass in units of the expected K-th distance: a pass serves the
+// queries that the one before found fewer than K particles for
+constexpr int kGrpPasses = 3;
+__device__ __constant__ static const float kGrpRadius[kGrpPasses] = {1.25f, 2.0f, 3.0f};
+
+// S slots of 32 neighbours: K <= 32 S. Groups shrink as the buffers grow, so that a warp's
+// shared memory stays near 6 KB.
+template <int S>
+struct GrpCfg {
+  static constexpr int G = S == 1 ? 8 : (S == 2 ? 4 : 2);
+  static constexpr int cap = 64 * S;
+};
+
+template <int S>
+struct GrpSmem {
+  float4 ch[kGrpChunk + 32];  // staged candidates: offsets from the centre, tree index
+  // per query its candidates: FP32 squared distance and tree index; in the SPH sums the
+  // row of bs holds 32 S doubles instead
+  unsigned bs[GrpCfg<S>::G][GrpCfg<S>::cap];
+  int bi[GrpCfg<S>::G][GrpCfg<S>::cap];
+  float4 qs[GrpCfg<S>::G];  // the queries: offset from the centre, acceptance bound
+  int stk[kGrpStack];
+};
+
+// Largest of the warp's keys (non-negative doubles' bit patterns).
+__device__ __forceinline__ long long warp_max_key(long long k) {
+  const unsigned hi = (unsigned)(k >> 32);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
+  return (long long)(((unsigned long long)mh << 32) | ml);
+}
+
+// Keep threshold for the K-th smallest FP32 squared distance s: every particle whose true
+// distance is at most the true K-th has an FP32 squared distance at or below it, and it is
+// at or above the true K-th squared distance.
+__device__ __forceinline__ float grp_thresh(float s, float two_e) {
+  float r;  // within 2^-22 of the square root, inside the 2^-20 margin
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(s));
+  const float u = __fmul_ru(r, 1.0f + 1.0f / 1048576.0f);
+  const float t = __fadd_ru(u, two_e);
+  return __fmul_ru(__fmul_ru(t, t), 1.0f + 1.0f / 1048576.0f);
+}
+
+struct GrpCut {
+  float thr;   // bound of the cut (-1: the FP32 range does not resolve the distances)
+  float smin;  // the smallest squared distance
+  int cnt;     // entries left
+};
+
+// Cut a query's buffer of cnt >= K entries back to those within the bound of its K-th
+// smallest (or of one of the `slack` next ones). Not inlined: the kernel's hot loops must
+// stay within the instruction cache (inlined everywhere, ten of eleven issue slots waited
+// for instructions).
+template <int S>
+__device__ __noinline__ GrpCut grp_tighten(unsigned* bs, int* bi, int lane, int cnt, int K,
+                                           int slack, float two_e) {
+  const unsigned FULL = 0xffffffffu;
+  constexpr int R = 2 * S;
+  GrpCut out;
+  unsigned r[R];
+  __syncwarp();
+  unsigned lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+  for (int t = 0; t < R; t++) {
+    const int p = t * 32 + lane;
+    const bool in = p < cnt;
+    r[t] = in ? bs[p] : 0xffffffffu;
+    lo = min(lo, r[t]);
+    if (in) hi = max(hi, r[t]);
+  }
+  lo = __reduce_min_sync(FULL, lo);
+  hi = __reduce_max_sync(FULL, hi);
+  out.smin = __uint_as_float(lo);
+  out.cnt = cnt;
+  // invariant: at least K entries are <= hi; done as soon as K to K + slack are. The first
+  // pivot assumes counts growing as the volume, the next ones halve the interval of values
+  float pv = __uint_as_float(hi) * (0.3f + 0.7f * __fdividef((float)K, (float)cnt));
+#pragma unroll 1
+  while (lo < hi && cnt > K + slack) {
+    const unsigned mid = max(min(__float_as_uint(pv), hi - 1u), lo);
+    int c = 0;
+#pragma unroll
+    for (int t = 0; t < R; t++) c += __popc(__ballot_sync(FULL, r[t] <= mid));
+    if (c >= K) {
+      hi = mid;
+      if (c <= K + slack) break;
+    } else {
+      lo = mid + 1;
+    }
+    pv = 0.5f * (__uint_as_float(lo) + __uint_as_float(hi));
+  }
+  unsigned kth = 0u;
+#pragma unroll
+  for (int t = 0; t < R; t++)
+    if (r[t] <= hi) kth = max(kth, r[t]);
+  kth = __reduce_max_sync(FULL, kth);
+  if (kth < 0x0da24260u || kth >= 0x7e000000u) {  // below 1e-30, near overflow
+    out.thr = -1.f;
+    return out;
+  }
+  out.thr = grp_thresh(__uint_as_float(kth), two_e);
+  if (cnt == K) return out;
+  const unsigned tb = __float_as_uint(out.thr);
+  int id[R], n = 0;
+#pragma unroll
+  for (int t = 0; t < R; t++) id[t] = bi[t * 32 + lane];
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < R; t++) {
+    const bool keep = r[t] <= tb;
+    const unsigned pm = __ballot_sync(FULL, keep);
+    if (keep) {
+      const int d = n + __popc(pm & ((1u << lane) - 1u));
+      bs[d] = r[t];
+      bi[d] = id[t];
+    }
+    n += __popc(pm);
+  }
+  __syncwarp();
+  out.cnt = n;
+  return out;
+}
+
+// The per-lane state of the group's queries (lane q < gn holds query q).
+struct GrpLane {
+  float x, y, z;  // offset from the centre
+  float thr;      // FP32 squared distances above it are not taken; -1: the query takes the
+                  // second launch
+  int cnt;        // candidates in its buffer
+  bool act;       // served by this pass
+};
+
+// Order-preserving map of floats to signed integers, and its inverse (the same map).
+__device__ __forceinline__ int ford(float x) {
+  const int i = __float_as_int(x);
+  return i ^ ((i >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float ford_inv(int i) {
+  return __int_as_float(i ^ ((i >> 31) & 0x7fffffff));
+}
+
+// FP32 squared length, every use rounded the same way (explicit fused steps).
+__device__ __forceinline__ float sq3(float x, float y, float z) {
+  return __fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x)));
+}
+
+// Every live query screens the staged candidates [0, m).
+template <int S>
+__device__ __forceinline__ void grp_stream(GrpSmem<S>& w, GrpLane& L, int lane, int gs, int m, int K,
+                           float two_e) {
+  const unsigned FULL = 0xffffffffu;
+  constexpr int cap = GrpCfg<S>::cap;
+  // queries whose bound does not reach the box around the staged candidates skip them
+  float blo[3], bhi[3];
+  {
+    int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
+    int mx[3] = {(int)0x80000000, (int)0x80000000, (int)0x80000000};
+    for (int c0 = 0; c0 < m; c0 += 32) {
+      if (c0 + lane >= m) continue;
+      const float4 c = w.ch[c0 + lane];
+      const int v[3] = {ford(c.x), ford(c.y), ford(c.z)};
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        mn[d] = min(mn[d], v[d]);
+        mx[d] = max(mx[d], v[d]);
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      blo[d] = ford_inv(__reduce_min_sync(FULL, mn[d]));
+      bhi[d] = ford_inv(__reduce_max_sync(FULL, mx[d]));
+    }
+  }
+  const float gx = fmaxf(0.f, fmaxf(blo[0] - L.x, L.x - bhi[0]));
+  const float gy = fmaxf(0.f, fmaxf(blo[1] - L.y, L.y - bhi[1]));
+  const float gz = fmaxf(0.f, fmaxf(blo[2] - L.z, L.z - bhi[2]));
+  // the screen's own distance of any of them is at least this (the same roundings, monotone)
+  unsigned live = __ballot_sync(FULL, L.act && sq3(gx, gy, gz) <= L.thr);
+  while (live) {
+    const int q = __ffs(live) - 1;
+    live &= live - 1;
+    const float4 qs = w.qs[q];
+    float thr = qs.w;
+    int cnt = __shfl_sync(FULL, L.cnt, q);
+#pragma unroll 1
+    for (int c0 = 0; c0 < m; c0 += 32) {
+      const float4 c = w.ch[c0 + lane];
+      const int id = __float_as_int(c.w);
+      const float s = sq3(c.x - qs.x, c.y - qs.y, c.z - qs.z);
+      bool pass = c0 + lane < m && s <= thr && id != gs + q;
+      unsigned pm = __ballot_sync(FULL, pass);
+      if (!pm) continue;
+      if (cnt + __popc(pm) > cap) {
+        const GrpCut t = grp_tighten<S>(w.bs[q], w.bi[q], lane, cnt, K,
+                                        min(kGrpSlack, cap - 32 - K), two_e);
+        thr = fminf(thr, t.thr);
+        cnt = t.cnt;
+        pass = pass && s <= thr;
+        pm = __ballot_sync(FULL, pass);
+        if (cnt + __popc(pm) > cap) thr = -1.f;  // too many within the rounding of the K-th
+        if (lane == q) L.thr = thr;
+        if (lane == 0) w.qs[q].w = thr;
+        if (thr < 0.f) break;
+      }
+      if (pass) {
+        const int d = cnt + __popc(pm & ((1u << lane) - 1u));
+        w.bs[q][d] = __float_as_uint(s);
+        w.bi[q][d] = id;
+      }
+      cnt += __popc(pm);
+    }
+    if (lane == q) L.cnt = cnt;
+  }
+  __syncwarp();
+}
+
+// One group's constants.
+struct GrpGeom {
+  float qlo[3], qhi[3];  // box around the group's particles (FP32, widened)
+  float4 ch, cl;         // the centre particle: FP32 copy and residual
+  float reach;           // squared: particles farther from the box are of no use
+};
+
+__device__ __forceinline__ bool grp_near(const GrpGeom& ge, float lx, float ly, float lz, float hx,
+                                         float hy, float hz) {
+  const float gx = fmaxf(0.f, fmaxf(__fsub_rd(lx, ge.qhi[0]), __fsub_rd(ge.qlo[0], hx)));
+  const float gy = fmaxf(0.f, fmaxf(__fsub_rd(ly, ge.qhi[1]), __fsub_rd(ge.qlo[1], hy)));
+  const float gz = fmaxf(0.f, fmaxf(__fsub_rd(lz, ge.qhi[2]), __fsub_rd(ge.qlo[2], hz)));
+  return __fadd_rd(__fadd_rd(__fmul_rd(gx, gx), __fmul_rd(gy, gy)), __fmul_rd(gz, gz)) <= ge.reach;
+}
+
+// Append the particle ti (one per lane, valid lanes only) to the staged candidates when it
+// is within reach of the group's box.
+template <int S>
+__device__ __forceinline__ void grp_stage(GrpSmem<S>& w, const TreeView& tv, const GrpGeom& ge,
+                                          int lane, bool valid, int ti, int& chn) {
+  float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool in = false;
+  if (valid) {
+    c = tv.posf[ti];
+    in = grp_near(ge, c.x, c.y, c.z, c.x, c.y, c.z);
+  }
+  const unsigned pm = __ballot_sync(0xffffffffu, in);
+  if (in) {
+    const float4 r = tv.posr[ti];
+    w.ch[chn + __popc(pm & ((1u << lane) - 1u))] =
+        make_float4((c.x - ge.ch.x) + (r.x - ge.cl.x), (c.y - ge.ch.y) + (r.y - ge.cl.y),
+                    (c.z - ge.ch.z) + (r.z - ge.cl.z), __int_as_float(ti));
+  }
+  chn += __popc(pm);
+}
+
+// The nodes of one step tested query by query (a node per lane, `have` marks the lanes that
+// hold one): whether any active query's bound reaches the lane's node. A node of more than K
+// particles also bounds the K-th distance by its farthest corner, so a dense place inside a
+// large radius cuts the bound before its particles are staged. Gaps are narrowed, and
+// reaches widened, by the rounding of the offsets.
+template <int S>
+__device__ __forceinline__ bool grp_wanted(GrpSmem<S>& w, const GrpGeom& ge, GrpLane& L,
+                                           const NodeRec& r, bool have, unsigned act, int lane,
+                                           int K, float two_e) {
+  const float lx = (r.lo[0] - ge.ch.x) - ge.cl.x, hx = (r.hi[0] - ge.ch.x) - ge.cl.x;
+  const float ly = (r.lo[1] - ge.ch.y) - ge.cl.y, hy = (r.hi[1] - ge.ch.y) - ge.cl.y;
+  const float lz = (r.lo[2] - ge.ch.z) - ge.cl.z, hz = (r.hi[2] - ge.ch.z) - ge.cl.z;
+  const bool many = have && r.count > K;
+  bool any = false;
+#pragma unroll 1
+  for (; act; act &= act - 1) {
+    const int i = __ffs(act) - 1;
+    float4 q = w.qs[i];
+    const float ax = lx - q.x, bx = q.x - hx, ay = ly - q.y, by = q.y - hy, az = lz - q.z,
+                bz = q.z - hz;
+    // the farthest corner is at max(|lo - q|, |q - hi|) per dimension
+    const float f = many ? sq3(fmaxf(fabsf(ax), fabsf(bx)), fmaxf(fabsf(ay), fabsf(by)),
+                               fmaxf(fabsf(az), fabsf(bz)))
+                         : FLT_MAX;
+    const float fm = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(f)));
+    if (fm < q.w) {
+      // widened twice: the bound of a cut to K of these candidates stays within it
+      q.w = fminf(q.w, grp_thresh(grp_thresh(grp_thresh(fm, two_e), two_e), two_e));
+      if (lane == i) {
+        L.thr = q.w;
+        w.qs[i].w = q.w;
+      }
+    }
+    const float gx = fmaxf(0.f, fmaxf(ax, bx) - two_e);
+    const float gy = fmaxf(0.f, fmaxf(ay, by) - two_e);
+    const float gz = fmaxf(0.f, fmaxf(az, bz) - two_e);
+    any = any || sq3(gx, gy, gz) <= q.w * (1.0f + 1.0f / 65536.0f);
+  }
+  __syncwarp();
+  return have && any;
+}
+
+// Distance within which a box of extents e (sorted or not) with n particles is expected to
+// hold K of them, taken as the largest of the line, square and cube estimates (the cube's
+// unless the box is flat or thin).
+__device__ __forceinline__ float grp_radius(float ex, float ey, float ez, int n, int K) {
+  const float a = fmaxf(ex, fmaxf(ey, ez)), c = fminf(ex, fminf(ey, ez));
+  const float b = fmaxf(fminf(ex, ey), fminf(fmaxf(ex, ey), ez));
+  const float f = __fdividef((float)K, (float)n);
+  const float r1 = 0.5f * f * a;
+  const float r2 = sqrtf(f * a * b * 0.31831f);
+  const float r3 = exp2f(log2f(f * a * b * c * 0.23873f) * (1.0f / 3.0f));
+  return fmaxf(r1, fmaxf(r2, r3));
+}
+
+// One walk of the tree for the active queries: first home itself and the siblings of home
+// and of its ancestors, one per lane (at most 31 levels), then their subtrees, up to 32
+// nodes a step. Returns false when the queries have to take the second launch.
+template <int S>
+__device__ bool grp_walk(GrpSmem<S>& w, const TreeView& tv, GrpGeom& ge, GrpLane& L, int lane,
+                         int gs, int hh, int lev, int K, float two_e) {
+  const unsigned FULL = 0xffffffffu;
+  const unsigned act = __ballot_sync(FULL, L.act);
+  int chn = 0, nst = 0, sp = 0, m = lev + 1, h = hh;
+  if (lane > 0 && lane <= lev) {
+    const int a = ((hh + 1) >> (lane - 1)) - 1;
+    h = (a & 1) ? a + 1 : a - 1;
+  }
+  unsigned lm = 0;      // leaves of the last step not staged yet (a bit per lane)
+  NodeRec r{};
+  int st = 0, ct = 0;   // the leaf this half warp stages, and how much of it is left
+#pragma unroll 1
+  for (int guard = 0; guard < (1 << 24); guard++) {
+    const bool part = __any_sync(FULL, ct > 0);
+    const bool done = m == 0 && lm == 0 && !part;
+    // the queries screen the staged candidates when a further batch might not fit
+    if (chn > kGrpChunk || (done && chn > 0)) {
+      __syncwarp();
+      grp_stream<S>(w, L, lane, gs, chn, K, two_e);
+      nst += chn;
+      chn = 0;
+      // the bounds shrink as buffers are cut
+      const float far = __uint_as_float(
+          __reduce_max_sync(FULL, L.act && L.thr >= 0.f ? __float_as_uint(L.thr) : 0u));
+      ge.reach = fminf(ge.reach, grp_thresh(far, two_e));
+    }
+    if (done) return true;
+    if (part || lm) {
+      // two leaves at a time, one per half warp, 16 particles a step
+      if (!part) {
+        const int l0 = __ffs(lm) - 1;
+        lm &= lm - 1;
+        const int l1 = lm ? __ffs(lm) - 1 : -1;
+        lm &= lm - 1;
+        const int src = lane < 16 ? l0 : l1;
+        st = __shfl_sync(FULL, r.start, src & 31);
+        ct = __shfl_sync(FULL, r.count, src & 31);
+        if (src < 0) ct = 0;
+      }
+      grp_stage<S>(w, tv, ge, lane, (lane & 15) < ct, st + (lane & 15), chn);
+      st += 16;
+      ct -= 16;
+      continue;
+    }
+    // the next nodes
+    bool need = false;
+    if (lane < m) {
+      r = tv.node[tv.nbase + h];
+      need = grp_near(ge, r.lo[0], r.lo[1], r.lo[2], r.hi[0], r.hi[1], r.hi[2]);
+    }
+    // a group whose box meets a much denser place: nodes are tested query by query, so that
+    // its cost stays that of its queries
+    if (nst > kGrpStrict) need = grp_wanted<S>(w, ge, L, r, need, act, lane, K, two_e);
+    const bool leaf = need && r.count <= tv.b;
+    const unsigned inner = __ballot_sync(FULL, need && !leaf);
+    lm = __ballot_sync(FULL, leaf);
+    const int ne = __popc(inner);
+    if (sp + 2 * ne > kGrpStack || nst > kGrpStaged) return false;
+    if ((inner >> lane) & 1u) {
+      const int slot = sp + 2 * __popc((inner >> lane) >> 1);
+      w.stk[slot] = 2 * h + 2;
+      w.stk[slot + 1] = 2 * h + 1;
+    }
+    sp += 2 * ne;
+    __syncwarp();
+    // above kWqBatchLimit entries pop one node at a time: a depth-first descent from there
+    // adds at most the tree depth
+    m = sp <= kWqBatchLimit ? min(32, sp) : 1;
+    if (lane < m) h = w.stk[sp - 1 - lane];
+    sp -= m;
+    __syncwarp();
+  }
+  return false;
+}
+
+// One group: on return lane q < gn holds the state of query gs + q and its buffer holds
+// every particle whose FP32 squared distance is within thr.
+template <int S>
+__device__ void grp_search(GrpSmem<S>& w, const TreeView& tv, int lane, int g, int depth, int K,
+                           GrpLane& L, int& gs, int& gn, float& two_e) {
+  const unsigned FULL = 0xffffffffu;
+  constexpr int G = GrpCfg<S>::G;
+  // the group (the node at `depth` of the split rule, virtual below the leaves) and the
+  // smallest real node around it with more than K particles (home)
+  const int want = max(K + 1, G);
+  int s0 = 0, sz = tv.n;
+  int hh = 0, hn = tv.n, lev = 0;
+  for (int i = depth - 1; i >= 0; i--) {
+    const int ls = (sz - 1) / 2 + 1;  // KDTree.cxx:1012, 1025-1030
+    const bool real = sz > tv.b;
+    const int right = (g >> i) & 1;
+    if (right) s0 += ls;
+    sz = right ? sz - ls : ls;
+    if (real && sz >= want) {
+      hh = 2 * hh + 1 + right;
+      hn = sz;
+      lev++;
+    }
+  }
+  gs = tv.pstart + s0;
+  gn = sz;
+  GrpGeom ge;
+  ge.ch = tv.posf[gs + (gn >> 1)];
+  ge.cl = tv.posr[gs + (gn >> 1)];
+  const NodeRec home = tv.node[tv.nbase + hh];
+  const float rad = grp_radius(__fsub_ru(home.hi[0], home.lo[0]), __fsub_ru(home.hi[1], home.lo[1]),
+                               __fsub_ru(home.hi[2], home.lo[2]), hn, K);
+  // offsets of the queries from the group's middle particle
+  float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
+  L.thr = -1.f;
+  L.cnt = 0;
+  L.x = L.y = L.z = 0.f;
+  if (lane < gn) {
+    mine = tv.posf[gs + lane];
+    const float4 r = tv.posr[gs + lane];
+    L.x = (mine.x - ge.ch.x) + (r.x - ge.cl.x);
+    L.y = (mine.y - ge.ch.y) + (r.y - ge.cl.y);
+    L.z = (mine.z - ge.ch.z) + (r.z - ge.cl.z);
+  }
+  // 2E: an offset's error is at most 2^-23 of it plus the residuals' own rounding (2^-48 of
+  // the coordinates, far below 2^-20 eps); the parts proportional to the distance are in
+  // the relative margin of grp_thresh
+  const float far = __uint_as_float(__reduce_max_sync(
+      FULL, __float_as_uint(fmaxf(fabsf(L.x), fmaxf(fabsf(L.y), fabsf(L.z))))));
+  two_e = __fmul_ru(4.f, __fadd_ru(__fmul_ru(far, 1.f / 4194304.f),
+                                   __fmul_ru(tv.eps, 1.f / 524288.f)));
+  const float e2 = __fmul_ru(2.f, tv.eps);  // the queries' own rounding and the candidates'
+#pragma unroll 1
+  for (int pass = 0; pass < kGrpPasses; pass++) {
+    L.act = lane < gn && L.cnt < K;
+    if (!__any_sync(FULL, L.act)) break;
+    const float r = kGrpRadius[pass] * rad;
+    float lo[3], hi[3];
+    lo[0] = L.act ? __fsub_rd(mine.x, e2) : FLT_MAX;
+    lo[1] = L.act ? __fsub_rd(mine.y, e2) : FLT_MAX;
+    lo[2] = L.act ? __fsub_rd(mine.z, e2) : FLT_MAX;
+    hi[0] = L.act ? __fadd_ru(mine.x, e2) : -FLT_MAX;
+    hi[1] = L.act ? __fadd_ru(mine.y, e2) : -FLT_MAX;
+    hi[2] = L.act ? __fadd_ru(mine.z, e2) : -FLT_MAX;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      ge.qlo[d] = __shfl_sync(FULL, lo[d], 0);
+      ge.qhi[d] = __shfl_sync(FULL, hi[d], 0);
+    }
+    ge.reach = grp_thresh(r * r, two_e);
+    if (L.act) {
+      L.cnt = 0;
+      L.thr = r * r;
+      w.qs[lane] = make_float4(L.x, L.y, L.z, L.thr);
+    }
+    __syncwarp();
+    if (!grp_walk<S>(w, tv, ge, L, lane, gs, hh, lev, K, two_e)) {
+      if (L.act) L.thr = -1.f;
+      break;
+    }
+    if (L.act && L.thr < 0.f) L.cnt = K;  // given up: not tried again
+  }
+}
+
+// Ascending sort of the 32 S (key, index) pairs over the warp, position p = s * 32 + lane.
+template <int S>
+__device__ __forceinline__ void grp_sort(long long key[S], int idx[S], int lane) {
+  const unsigned FULL = 0xffffffffu;
+#pragma unroll
+  for (int size = 2; size <= 32 * S; size <<= 1) {
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      if (stride >= 32) {
+        const int ds = stride >> 5;
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+          if (s & ds) continue;
+          const bool up = ((s * 32) & size) == 0;
+          if ((key[s] > key[s + ds]) == up) {
+            const long long k = key[s];
+            key[s] = key[s + ds];
+            key[s + ds] = k;
+            const int i = idx[s];
+            idx[s] = idx[s + ds];
+            idx[s + ds] = i;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+          const long long ok = __shfl_xor_sync(FULL, key[s], stride);
+          const int oj = __shfl_xor_sync(FULL, idx[s], stride);
+          const bool up = ((s * 32 + lane) & size) == 0, lower = (lane & stride) == 0;
+          if ((lower == up) ? (ok < key[s]) : (ok > key[s])) {
+            key[s] = ok;
+            idx[s] = oj;
+          }
+        }
+      }
+    }
+  }
+}
+
+// Exact choice among the cnt > K candidates left in a query's buffer (at most 32 S + 32):
+// FP64 distances, the largest dropped until K are left, their indices back in the buffer.
+template <int S>
+__device__ __noinline__ void grp_drop(int* bi, const P4* pos, int lane, int self, int cnt, int K) {
+  const unsigned FULL = 0xffffffffu;
+  const P4 x = pos[self];
+  long long key[S + 1];
+  int idx[S + 1];
+#pragma unroll
+  for (int s = 0; s <= S; s++) {
+    const int p = s * 32 + lane;
+    key[s] = 0;
+    idx[s] = -1;
+    if (p < cnt) {
+      idx[s] = bi[p];
+      const P4 c = pos[idx[s]];
+      key[s] = dkey(dist2_exact(x.x, x.y, x.z, c.x, c.y, c.z));
+    }
+  }
+  for (int left = cnt; left > K; left--) {
+    long long mx = 0;
+#pragma unroll
+    for (int s = 0; s <= S; s++) mx = max(mx, key[s]);
+    mx = warp_max_key(mx);
+    int gone = 0;  // one holder of the largest leaves
+#pragma unroll
+    for (int s = 0; s <= S; s++) {
+      const unsigned b = gone ? 0u : __ballot_sync(FULL, idx[s] >= 0 && key[s] == mx);
+      if (b) {
+        gone = 1;
+        if (lane == __ffs(b) - 1) {
+          key[s] = 0;
+          idx[s] = -1;
+        }
+      }
+    }
+  }
+  int n = 0;
+  __syncwarp();
+#pragma unroll
+  for (int s = 0; s <= S; s++) {
+    const unsigned pm = __ballot_sync(FULL, idx[s] >= 0);
+    if (idx[s] >= 0) bi[n + __popc(pm & ((1u << lane) - 1u))] = idx[s];
+    n += __popc(pm);
+  }
+  __syncwarp();
+}
+
+// The neighbours of one query: its buffer cut to the K nearest (indices in bi[0 .. K)).
+// Returns false when the query has to take the second launch; thr returns an FP32 bound at
+// or above the K-th squared distance.
+template <int S>
+__device__ bool grp_select(GrpSmem<S>& w, const TreeView& tv, int lane, int q, int self, int cnt,
+                           int K, float two_e, float& thr) {
+  if (thr < 0.f || cnt < K) return false;
+  const GrpCut f = grp_tighten<S>(w.bs[q], w.bi[q], lane, cnt, K, 0, two_e);
+  // every particle within the bound must have been taken, and every neighbour must be
+  // provably at a non-zero distance: sqrt(s) (1 - 2^-20) > 2E
+  const float zero2 = __fmul_ru(__fmul_ru(two_e, two_e), 1.01f);
+  if (f.thr < 0.f || f.thr > thr || f.smin <= zero2 || f.cnt > 32 * S + 32) return false;
+  thr = f.thr;
+  if (f.cnt > K) grp_drop<S>(w.bi[q], tv.pos, lane, self, f.cnt, K);
+  return true;
+}
+
+// Sums of the G rows of 32 S doubles, 32 / G lanes a row: on return the first of row q's
+// lanes holds its sum.
+template <int S>
+__device__ __forceinline__ double grp_row_sums(GrpSmem<S>& w, int lane) {
+  constexpr int lanes = 32 / GrpCfg<S>::G, per = 32 * S / lanes;
+  static_assert((per & (per - 1)) == 0, "the rotation wraps");
+  const double* row =
+      reinterpret_cast<const double*>(w.bs[lane / lanes]) + (lane % lanes) * per;
+  double acc = 0.0;
+#pragma unroll
+  for (int t = 0; t < per; t++) acc = dadd(acc, row[(t + lane) & (per - 1)]);
+#pragma unroll
+  for (int o = 1; o < lanes; o <<= 1) acc = dadd(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+  return acc;
+}
+
+// Marks in a row of squared distances: the farthest neighbour sits at q = 2 exactly in the
+// reference's arithmetic (the table's last entry); no neighbour in this place.
+constexpr double kGrpFar = -1.0, kGrpNone = -2.0;
+
+// W of one row entry: u = sqrt(d2) c1 is the table coordinate (c1 = 1 / (h delta)).
+__device__ __forceinline__ double grp_w(double d2, double c1, int kr, const double* T) {
+  const int hi = __double2hiint(d2);
+  if (hi < 0) return d2 == kGrpFar ? T[kr - 1] : 0.0;
+  return w_at_u(dmul(sqrt_newton(d2), c1), kr, T);
+}
+
+// The group's density sums (CalcDensity, KDCalcSmoothQuantities.cxx:260-286): okm marks the
+// queries answered here, bi their neighbours. SAVE: the neighbour rows are kept too, the
+// farthest last.
+template <int S, bool SAVE>
+__device__ void grp_density(const KnnArgs& a, const TreeView& tv, GrpSmem<S>& w, int lane, int gs,
+                            unsigned okm, int K) {
+  const unsigned FULL = 0xffffffffu;
+  const int kr = a.kernres;
+  const double* T = a.kernel;
+  long long top = 0;
+#pragma unroll 1
+  for (unsigned left = okm; left; left &= left - 1) {
+    const int q = __ffs(left) - 1;
+    const P4 x = tv.pos[gs + q];
+    double* row = reinterpret_cast<double*>(w.bs[q]);
+    double d2[S];
+    long long mx = 0;
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const int p = s * 32 + lane;
+      d2[s] = kGrpNone;
+      if (p < K) {
+        const P4 c = tv.pos[w.bi[q][p]];
+        const double dx = dsub(x.x, c.x), dy = dsub(x.y, c.y), dz = dsub(x.z, c.z);
+        d2[s] = __fma_rn(dz, dz, __fma_rn(dy, dy, dmul(dx, dx)));
+        mx = max(mx, dkey(d2[s]));
+      }
+    }
+    mx = warp_max_key(mx);
+    if (lane == q) top = mx;
+    int at = K - 1;  // where the farthest is
+#pragma unroll
+    for (int s = S - 1; s >= 0; s--) {
+      const bool is = dkey(d2[s]) == mx;
+      if (SAVE) {
+        const unsigned b = __ballot_sync(FULL, is);
+        if (b) at = s * 32 + __ffs(b) - 1;
+      }
+      row[s * 32 + lane] = is ? kGrpFar : d2[s];
+    }
+    if (SAVE) {
+#pragma unroll
+      for (int s = 0; s < S; s++) {
+        const int p = s * 32 + lane;
+        if (p < K)
+          a.nn[(size_t)(gs + q - tv.pstart) * K + (p == at ? K - 1 : (p == K - 1 ? at : p))] =
+              w.bi[q][p];
+      }
+    }
+  }
+  // a lane per query: 1/h (h = sqrt(top) / 2), the table coordinate's scale, the weights
+  double c1 = 0.0, wn = 0.0, wm = 0.0;
+  if ((okm >> lane) & 1u) {
+    const double ih = two_rsqrt(__longlong_as_double(top));
+    c1 = dmul(ih, 0.5 * (double)(kr - 1));
+    wn = 0.5 * dmul(dmul(ih, ih), ih);
+    wm = dmul(wn, tv.pos[gs + lane].m);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (unsigned left = okm; left; left &= left - 1) {
+    const int q = __ffs(left) - 1;
+    const double c = __shfl_sync(FULL, c1, q), m = __shfl_sync(FULL, wm, q);
+    double* row = reinterpret_cast<double*>(w.bs[q]);
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const int p = s * 32 + lane;
+      double t = 0.0;
+      if (p < K) {
+        const int j = w.bi[q][p];
+        const double wq = grp_w(row[p], c, kr, T);
+        atomicAdd(&a.rho[j], dmul(wq, m));
+        t = dmul(wq, tv.pos[j].m);
+      }
+      row[p] = t;
+    }
+  }
+  __syncwarp();
+  const double acc = grp_row_sums<S>(w, lane);
+  constexpr int lanes = 32 / GrpCfg<S>::G;
+  const int q = lane / lanes;
+  const double n = __shfl_sync(FULL, wn, q);
+  if (lane % lanes == 0 && ((okm >> q) & 1u)) atomicAdd(&a.rho[gs + q], dmul(acc, n));
+  __syncwarp();
+}
+
+// The group's velocity densities (CalcVelDensity, KDCalcSmoothQuantities.cxx:354-383): the
+// nsmooth smallest |dv| of the neighbours, h = 0.5 max, sum Wsm(|dv|/h) h^-3, unit weights.
+template <int S>
+__device__ void grp_veldensity(const KnnArgs& a, const TreeView& tv, GrpSmem<S>& w, int lane,
+                               int gs, unsigned okm, int K) {
+  const unsigned FULL = 0xffffffffu;
+  const int kr = a.kernres, ns = a.nsmooth;
+  const double* T = a.kernel;
+  long long top = 0;
+#pragma unroll 1
+  for (unsigned left = okm; left; left &= left - 1) {
+    const int q = __ffs(left) - 1;
+    const V4 x = tv.vel[gs + q];
+    double* row = reinterpret_cast<double*>(w.bs[q]);
+    long long vk[S];
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const int p = s * 32 + lane;
+      vk[s] = kWqSent;
+      if (p < K) {
+        const V4 c = tv.vel[w.bi[q][p]];
+        const double dx = dsub(x.x, c.x), dy = dsub(x.y, c.y), dz = dsub(x.z, c.z);
+        vk[s] = dkey(__fma_rn(dz, dz, __fma_rn(dy, dy, dmul(dx, dx))));
+      }
+    }
+    bool sel[S];
+    if (ns < K) {
+      int rk[S];
+      wq_ranks<S>(vk, lane, K, rk);
+#pragma unroll
+      for (int s = 0; s < S; s++) sel[s] = s * 32 + lane < K && rk[s] < ns;
+    } else {
+#pragma unroll
+      for (int s = 0; s < S; s++) sel[s] = s * 32 + lane < K;
+    }
+    long long mx = 0;
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      if (sel[s]) mx = max(mx, vk[s]);
+    mx = warp_max_key(mx);
+    if (lane == q) top = mx;
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      row[s * 32 + lane] =
+          !sel[s] ? kGrpNone : (vk[s] == mx ? kGrpFar : __longlong_as_double(vk[s]));
+  }
+  double c1 = 0.0, wn = 0.0;
+  if ((okm >> lane) & 1u) {
+    const double ih = two_rsqrt(__longlong_as_double(top));
+    c1 = dmul(ih, 0.5 * (double)(kr - 1));
+    wn = dmul(dmul(ih, ih), ih);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (unsigned left = okm; left; left &= left - 1) {
+    const int q = __ffs(left) - 1;
+    const double c = __shfl_sync(FULL, c1, q);
+    double* row = reinterpret_cast<double*>(w.bs[q]);
+#pragma unroll
+    for (int s = 0; s < S; s++) row[s * 32 + lane] = grp_w(row[s * 32 + lane], c, kr, T);
+  }
+  __syncwarp();
+  const double acc = grp_row_sums<S>(w, lane);
+  constexpr int lanes = 32 / GrpCfg<S>::G;
+  const int q = lane / lanes;
+  const double n = __shfl_sync(FULL, wn, q);
+  if (lane % lanes == 0 && ((okm >> q) & 1u)) a.vden[gs + q] = dmul(acc, n);
+  __syncwarp();
+}
+
+// The warp-per-query search for the queries the group kernel left: a persistent grid over
+// the list fb[1 .. fb[0]] of tree indices.
+template <int S, int EPI>
+__global__ void __launch_bounds__(32 * kWqWpb, 4) k_knn_wq_list(KnnArgs a) {
+  __shared__ WqSmem ws[kWqWpb];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int count = min(a.fb[0], a.nq);
+  for (int i = blockIdx.x * kWqWpb + warp; i < count; i += gridDim.x * kWqWpb) {
+    const int self = a.fb[1 + i];
+    P4 p = a.tv.pos[self];
+    double x0[3] = {p.x, p.y, p.z};
+    wq_run<S, EPI>(a, a.tv, ws[warp], lane, self - a.q0, self, x0, a.kheap);
+    __syncwarp();
+  }
+}
+
+// K: neighbours other than the query itself. A periodic search (FindNearest) takes the
+// image passes in the second launch for the queries whose gates could open; for the rest
+// its k + 1 list is the query itself at zero distance, then the K = k nearest others.
+template <int S, int EPI>
+__global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int depth, int K) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int g = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
+  if (g >= (1 << depth)) return;
+  const TreeView& tv = a.tv;
+  GrpLane L;
+  int gs, gn;
+  float two_e;
+  grp_search<S>(w, tv, lane, g, depth, K, L, gs, gn, two_e);
+  unsigned okm = 0u;  // queries answered here; the others take the second launch
+#pragma unroll 1
+  for (int q = 0; q < gn; q++) {
+    float thr = __shfl_sync(FULL, L.thr, q);
+    const int cnt = __shfl_sync(FULL, L.cnt, q), self = gs + q;
+    bool ok = grp_select<S>(w, tv, lane, q, self, cnt, K, two_e, thr);
+    if (EPI == kEpiNN && ok && a.periodic) {
+      const float4 qf = tv.posf[self];
+      const float qeps = __fmul_ru(2.f, tv.eps);
+      const int near_sq = near_walls(qf, tv.period, qeps, thr);
+      const int near_lin = near_walls_lin(qf, tv.period, qeps, thr);
+      ok = near_sq == 0 && (a.min_image || __popc(near_lin) < 2);
+    }
+    if (!ok) continue;
+    okm |= 1u << q;
+    if (EPI == kEpiNN) {
+      const P4 x = tv.pos[self];
+      long long key[S];
+      int idx[S];
+#pragma unroll
+      for (int s = 0; s < S; s++) {
+        key[s] = kWqSent;
+        idx[s] = -1;
+        if (s * 32 + lane < K) {
+          idx[s] = w.bi[q][s * 32 + lane];
+          const P4 c = tv.pos[idx[s]];
+          key[s] = dkey(dist2_exact(x.x, x.y, x.z, c.x, c.y, c.z));
+        }
+      }
+      grp_sort<S>(key, idx, lane);
+      // a periodic list starts with the query itself, then the others; the row leaves out
+      // the nearest (FindNearest) or the largest (FindNearestPos) where one more was asked
+      const int off = (a.periodic ? 1 : 0) - (a.kheap - (a.drop_largest ? 1 : 0) - a.kout);
+      const size_t row = (size_t)(self - a.q0) * a.kout;
+#pragma unroll
+      for (int s = 0; s < S; s++) {
+        const int i = s * 32 + lane + off;
+        if (s * 32 + lane < K && i >= 0 && i < a.kout) {
+          a.nn[row + i] = idx[s];
+          a.d2[row + i] = __longlong_as_double(key[s]);
+        }
+      }
+      if (off > 0 && lane == 0) {
+        a.nn[row] = self;
+        a.d2[row] = 0.0;
+      }
+    }
+  }
+  __syncwarp();
+  if (EPI == kEpiDensity || EPI == kEpiDensVel || EPI == kEpiDensSave)
+    grp_density<S, EPI == kEpiDensSave>(a, tv, w, lane, gs, okm, K);
+  if (EPI == kEpiDensVel || EPI == kEpiVel) grp_veldensity<S>(a, tv, w, lane, gs, okm, K);
+  const unsigned am = ~okm & (gn >= 32 ? FULL : (1u << gn) - 1u);
+  if (am) {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&a.fb[0], __popc(am));
+    base = __shfl_sync(FULL, base, 0);
+    if ((am >> lane) & 1u) a.fb[1 + base + __popc(am & ((1u << lane) - 1u))] = gs + lane;
+  }
+}
+
+template <int S, int EPI>
+int launch_group(const KnnArgs& a, int K, cudaStream_t st) {
+  // groups of at most G particles, and enough of them to keep every SM's warps busy
+  int nsm = 0, dev = 0;
+  NBK_CUDA_TRY(cudaGetDevice(&dev));
+  NBK_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  int depth = 0;
+  while ((((int64_t)a.nq - 1) >> depth) + 1 > GrpCfg<S>::G) depth++;
+  while ((1 << depth) < 16 * nsm && (((int64_t)a.nq - 1) >> (depth + 1)) + 1 >= 2) depth++;
+  const size_t sm = sizeof(GrpSmem<S>) * kGrpWpb;
+  NBK_TRY(ensure_dyn_smem((const void*)k_knn_group<S, EPI>, (int)sm));
+  static const char* kNames[] = {"knn_nn", "knn_density", "knn_density_veldensity", "knn_veldensity",
+                                 "knn_density_particle", "knn_veldensity_particle", "knn_density_save"};
+  NBK_CUDA_TRY(cudaMemsetAsync(a.fb, 0, sizeof(int), st));
+  Phase ph(kNames[EPI], st);
+  const unsigned blocks = ((1u << depth) + kGrpWpb - 1) / kGrpWpb;
+  k_knn_group<S, EPI><<<blocks, 32 * kGrpWpb, sm, st>>>(a, depth, K); note_launch();
+  const unsigned lb = (unsigned)std::min<int64_t>(4 * nsm, ((int64_t)a.nq + kWqWpb - 1) / kWqWpb);
+  if (a.kheap <= 32) k_knn_wq_list<1, EPI><<<lb, 32 * kWqWpb, 0, st>>>(a);
+  else if (a.kheap <= 64) k_knn_wq_list<2, EPI><<<lb, 32 * kWqWpb, 0, st>>>(a);
+  else k_knn_wq_list<4, EPI><<<lb, 32 * kWqWpb, 0, st>>>(a);
+  note_launch();
+  NBK_CUDA_TRY(cudaGetLastError());
+  return NBK_OK;
+}
+
+template <int EPI>
+int launch_group_e(const KnnArgs& a, cudaStream_t st) {
+  const int K = a.periodic ? a.kheap - 1 : a.kheap;  // neighbours other than the query
+  if (K <= 32) return launch_group<1, EPI>(a, K, st);
+  if (K <= 64) return launch_group<2, EPI>(a, K, st);
+  return launch_group<4, EPI>(a, K, st);
+}
+
+}  // namespace
+
+bool group_search_serves(const KnnArgs& a) {
+  const int K = a.periodic ? a.kheap - 1 : a.kheap;
+  return a.qmode == 0 && a.fb && a.nq == a.tv.n && a.kheap <= 128 && K >= 1 &&
+         a.nq >= 4 * (K + 1) && a.tv.eps < 1e11f && (a.exclude_self || a.periodic);
+}
+
+int launch_knn_group(const KnnArgs& a, int epi, cudaStream_t st) {
+  switch (epi) {
+    case kEpiNN: return launch_group_e<kEpiNN>(a, st);
+    case kEpiDensity: return launch_group_e<kEpiDensity>(a, st);
+    case kEpiDensVel: return launch_group_e<kEpiDensVel>(a, st);
+    case kEpiVel: return launch_group_e<kEpiVel>(a, st);
+    case kEpiDensSave: return launch_group_e<kEpiDensSave>(a, st);
+  }
+  set_error("unknown kNN epilogue");
+  return NBK_ERR_INVALID;
+}
+
+}  // namespace nbk

@@ -702,12 +702,13 @@ __device__ __forceinline__ void wq_ranks(const long long v[S], int lane, int K, 
   }
 }
 
+static __device__ __noinline__ double two_rsqrt_call(double t) { return 1.0 / (0.5 * __dsqrt_rn(t)); }
 // 2 / sqrt(t) (the 1/h of h = sqrt(t) / 2) to about 2e-16 relative: the FP32 reciprocal
 // square root as the start and two Newton steps y (3/2 - t/2 y^2) in FP64. Outside the
 // FP32 normal range it takes the FP64 square root and division.
 __device__ __forceinline__ double two_rsqrt(double t) {
   const float tf = __double2float_rn(t);
-  if (!(tf > 1e-30f && tf < 1e30f)) return 1.0 / (0.5 * __dsqrt_rn(t));
+  if (!(tf > 1e-30f && tf < 1e30f)) return two_rsqrt_call(t);
   double y = (double)rsqrtf(tf);
   const double ht = 0.5 * t;
   y = dmul(y, __fma_rn(-ht, dmul(y, y), 1.5));
@@ -728,6 +729,131 @@ __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x = dadd(x, __shfl_xor_sync(0xffffffffu, x, o));
   return x;
+}
+
+constexpr int kWqWpb = 8;  // warps (queries) per block
+
+// What one query's k-list (L, topk: the key at position K - 1) becomes: neighbour rows
+// ascending in d2 (kEpiNN), or the SPH sums. `qi` indexes the per-query outputs and `self`
+// is the query's tree index. All lanes of the warp call this together.
+template <int S, int EPI>
+__device__ __forceinline__ void wq_epilogue(const KnnArgs& a, const TreeView& tv, int lane, int qi,
+                                            int self, int K, const WqList<S>& L, long long topk) {
+  const unsigned FULL = 0xffffffffu;
+  const int kr = a.kernres;
+  const double inv_delta = 0.5 * (double)(kr - 1);  // 1 / table step, exact
+  if (EPI == kEpiNN) {
+    // rows ascending in d2; the popped largest (FindNearestPos on a periodic tree) or the
+    // nearest (FindNearest on a periodic tree: k + 1 searched, k written) are left out
+    // exactly as the heap version pops them
+    int first = K - (a.drop_largest ? 1 : 0) - a.kout;
+    size_t row = (size_t)qi * a.kout;
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      int i = s * 32 + lane - first;
+      if (i >= 0 && i < a.kout) {
+        a.nn[row + i] = L.idx[s];
+        a.d2[row + i] = __longlong_as_double(L.key[s]);
+      }
+    }
+    return;
+  }
+  // density family: the list holds exactly the k neighbours (target search)
+  bool missing = false;
+#pragma unroll
+  for (int s = 0; s < S; s++) missing |= (s * 32 + lane < K) && L.idx[s] < 0;
+  if (__any_sync(FULL, missing)) {
+    if (lane == 0) atomicExch(a.err, kErrTooFew);
+    return;
+  }
+  const double* T = a.kernel;
+  if (EPI == kEpiDensity || EPI == kEpiDensVel || EPI == kEpiDensPart || EPI == kEpiDensSave) {
+    // KDCalcSmoothQuantities.cxx:260-286: one neighbour per lane. 1 / h with
+    // h = sqrt(top) / 2 (the reference divides by h) within a few ulps, far inside the
+    // 1e-12 density tolerance
+    const double me_m = tv.pos[self].m;
+    double ih = two_rsqrt(__longlong_as_double(topk));
+    double norm = dmul(dmul(ih, ih), ih);  // 1 / h^3 (the reference takes pow(h, 3))
+    double wnorm = EPI == kEpiDensPart ? norm : 0.5 * norm;
+    double acc = 0.0;
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      int p = s * 32 + lane;
+      if (p >= K) continue;
+      double d2 = __longlong_as_double(L.key[s]);
+      int j = L.idx[s];
+      // the farthest neighbour sits at q = 2 exactly in the reference's arithmetic (the
+      // table's last entry); the product with 1/h could land an ulp below it
+      double q = dmul(sqrt_newton(d2), ih);
+      double wq = L.key[s] == topk ? T[kr - 1] : wsm_line(q, kr, inv_delta, T);
+      double wij = dmul(wq, wnorm);
+      acc = dadd(acc, dmul(wij, tv.pos[j].m));
+      if (EPI != kEpiDensPart) {
+        atomicAdd(&a.rho[j], dmul(wij, me_m));
+        if (EPI == kEpiDensSave) a.nn[(size_t)(self - tv.pstart) * K + p] = j;
+      }
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) {
+      if (EPI == kEpiDensPart) a.rho[qi] = acc;
+      else atomicAdd(&a.rho[self], acc);
+    }
+  }
+  if (EPI == kEpiDensVel || EPI == kEpiVel || EPI == kEpiVelPart) {
+    // KDCalcSmoothQuantities.cxx:354-383: |dv| of the Nsearch neighbours, keep the
+    // Nsmooth smallest, h = 0.5 max, sum Wsm(|dv|/h) h^-3 with unit weights
+    V4 vi = tv.vel[self];
+    long long vk[S];
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      vk[s] = kWqSent;
+      if (s * 32 + lane < K) {
+        V4 vj = tv.vel[L.idx[s]];
+        vk[s] = dkey(sqrt_newton(dist2_exact(vi.x, vi.y, vi.z, vj.x, vj.y, vj.z)));
+      }
+    }
+    int ns = a.nsmooth;
+    bool sel[S];
+    if (ns < K) {
+      int rk[S];
+      wq_ranks<S>(vk, lane, K, rk);
+#pragma unroll
+      for (int s = 0; s < S; s++) sel[s] = s * 32 + lane < K && rk[s] < ns;
+    } else {
+#pragma unroll
+      for (int s = 0; s < S; s++) sel[s] = s * 32 + lane < K;
+    }
+    long long vmaxk = 0;
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      if (sel[s]) vmaxk = max(vmaxk, vk[s]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vmaxk = max(vmaxk, __shfl_xor_sync(FULL, vmaxk, o));
+    double ih = recip_newton(0.5 * __longlong_as_double(vmaxk));
+    double norm = dmul(dmul(ih, ih), ih);
+    double acc = 0.0;
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      if (!sel[s]) continue;
+      double q = dmul(__longlong_as_double(vk[s]), ih);
+      double wq = vk[s] == vmaxk ? T[kr - 1] : wsm_line(q, kr, inv_delta, T);  // q = 2
+      acc = dadd(acc, dmul(wq, norm));
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) {
+      if (EPI == kEpiVelPart) a.vden[qi] = acc;
+      else a.vden[self] = acc;
+    }
+  }
+}
+
+// One query's search and epilogue on one warp (as wq_epilogue).
+template <int S, int EPI, bool F32FIRST = false>
+__device__ void wq_run(const KnnArgs& a, const TreeView& tv, WqSmem& w, int lane, int qi,
+                       int self, const double x0[3], int K) {
+  WqQuery<S> Q;
+  wq_search<S, F32FIRST>(Q, w, a, tv, lane, self, x0, K, a.exclude_self != 0);
+  wq_epilogue<S, EPI>(a, tv, lane, qi, self, K, Q.L, Q.topk);
 }
 
 }  // namespace

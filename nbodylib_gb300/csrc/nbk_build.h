@@ -28,6 +28,7 @@ struct TreeSpec {
 struct BuiltArrays {
   P4* pos = nullptr;
   float4* posf = nullptr;
+  float4* posr = nullptr;     // physical / velocity trees
   V4* vel = nullptr;
   int* perm = nullptr;
   NodeRec* node = nullptr;    // physical / velocity trees
@@ -130,8 +131,12 @@ struct KnnArgs {
   double* vden;
   int* err;
   const double* qv;   // query velocities of coordinate queries (CalcVelDensityPosition)
+  int* fb;            // 1 + nq ints of scratch for the group search (null: a warp per query)
 };
 int launch_knn(const KnnArgs& a, int epi, cudaStream_t st);
+// The group search (knn_group.cu): every particle of a tree at once.
+bool group_search_serves(const KnnArgs& a);
+int launch_knn_group(const KnnArgs& a, int epi, cudaStream_t st);
 
 // ---- phase-space trees (phase.cu)
 enum PhaseEpi : int {

@@ -3,6 +3,7 @@
 // HBM layout of a built tree (all arrays in tree order unless noted):
 //   P4      pos[n]    x, y, z, mass as FP64 (32 B, two 16-B vector loads)
 //   float4  posf[n]   x, y, z rounded to nearest FP32 (candidate filter)
+//   float4  posr[n]   x - posf.x, ... rounded to FP32 (local offsets of the group search)
 //   V4 vel[n]    vx, vy, vz, 0 (only when velocities were given)
 //   int32   perm[n]   tree index -> input index
 //   NodeRec node[]    heap-indexed (root 0, children 2h+1 / 2h+2): FP32 bounding box
@@ -70,6 +71,7 @@ struct __align__(16) NodeF6 {  // the same box in FP32, rounded outward
 struct TreeView {
   const P4* pos;
   const float4* posf;
+  const float4* posr;    // physical / velocity trees
   const V4* vel;
   const int* perm;
   const NodeRec* node;
@@ -280,6 +282,15 @@ __device__ __forceinline__ double wsm_line(double q, int size, double inv_delta,
   return img[size - 1];
 }
 
+// W at the table coordinate u = q (size - 1) / 2 from the image's sections A and D: on cell
+// i = (int)u the line is A[i] + D[i] u. The cell comes from the bits of u (u < 2^20).
+__device__ __forceinline__ double w_at_u(double u, int size, const double* img) {
+  const int hi = __double2hiint(u), e = (hi >> 20) - 1023;
+  const int i = e < 0 ? 0 : ((hi & 0xfffff) | 0x100000) >> max(20 - e, 0);
+  if (i < size - 1) return __fma_rn(img[3 * size + i], u, img[size + i]);
+  return img[size - 1];
+}
+
 // ---- phase-space trees: depth bound of their per-thread walks, six-vector access
 constexpr int kPhDepth = 64;
 // v[d] of a six-vector indexed at run time (registers, no local memory)
@@ -355,17 +366,43 @@ __device__ __forceinline__ float pair_ub6f(const float q[6], const float c[6], c
   return s;
 }
 
-// sqrt(x) for the kernel interpolation, to about 2e-14 relative: the FP32 square root as
-// the start and one Newton-Raphson (Heron) step in FP64, q0 + (x - q0^2) / (2 q0), whose
-// correction uses an FP32 reciprocal (its error only scales the already small correction).
-// Outside the FP32 normal range it falls back to the FP64 square root.
+// FP32 value of a positive double in FP32's normal range, rounded to nearest, and a
+// positive normal float as a double, on the integer pipe (GB300's conversions to and from
+// FP64 share the FP64 pipe's two lanes).
+__device__ __forceinline__ float f32_of_bits(int hi, int lo) {
+  const unsigned m = ((unsigned)hi << 3) | ((unsigned)lo >> 29);
+  return __uint_as_float(m - ((1023u - 127u) << 23) + (((unsigned)lo >> 28) & 1u));
+}
+__device__ __forceinline__ double f64_of_f32(float f) {
+  const unsigned u = __float_as_uint(f);
+  return __hiloint2double((int)((u >> 3) + ((1023u - 127u) << 20)), (int)(u << 29));
+}
+
+// The FP64 square root out of line, for the rare paths of inlined code.
+static __device__ __noinline__ double dsqrt_call(double x) { return __dsqrt_rn(x); }
+
+// sqrt(x) for the kernel interpolation, to about one unit in the last place: x = xh + xl as
+// two floats, the FP32 reciprocal square root y of xh, q0 = xh y corrected in FP32 by
+// (x - q0^2) / (2 q0) (to 2^-44), and one Heron step in FP64. W falls off as (2 - q)^3, so
+// a relative error of q grows by 3 q / (2 - q) in the outermost neighbours' terms. Three
+// FP64 instructions. Outside 2^-70 .. 2^100 it falls back to the FP64 square root.
 __device__ __forceinline__ double sqrt_newton(double x) {
-  const float xf = __double2float_rn(x);
-  if (!(xf > 1e-30f && xf < 1e30f)) return __dsqrt_rn(x);
-  const float q0f = sqrtf(xf);
-  const double q0 = (double)q0f;
-  const double half_inv = (double)__fdividef(0.5f, q0f);
-  return __fma_rn(__fma_rn(-q0, q0, x), half_inv, q0);
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  if ((unsigned)(hi - ((1023 - 70) << 20)) > (unsigned)(170 << 20)) return dsqrt_call(x);
+  const float xh = f32_of_bits(hi, lo);
+  // x - xh: the 29 bits below, signed by the rounding, times 2^(e - 52)
+  const float xl = __fmul_rn((float)((int)((unsigned)lo << 3) >> 3),
+                             __int_as_float(((hi >> 20) - (1023 + 52 - 127)) << 23));
+  float y;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(xh));
+  const float q0 = __fmul_rn(xh, y), hy = __fmul_rn(0.5f, y);
+  const float q1 = __fmul_rn(__fadd_rn(__fmaf_rn(-q0, q0, xh), xl), hy);
+  // q1 may be negative or zero (then 2^-127, nothing to q0)
+  const unsigned u = __float_as_uint(q1);
+  const double d1 = __hiloint2double(
+      (int)((((u & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20)) | (u & 0x80000000u)), (int)(u << 29));
+  const double q = dadd(f64_of_f32(q0), d1);
+  return __fma_rn(__fma_rn(-q, q, x), f64_of_f32(hy), q);
 }
 
 // W(q) at q = sqrt(d2) / h with h = sqrt(top) / 2 (ih = 1/h): the farthest neighbour
