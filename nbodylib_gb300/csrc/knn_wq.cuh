@@ -1,6 +1,10 @@
-// Warp-per-query k-nearest-neighbour search for target queries (a query that is a
-// particle of the tree): the kNN behind CalcDensity, CalcVelDensity, CalcDensityParticle,
-// CalcVelDensityParticle and FindNearest / FindNearestPos of tree particles.
+// Warp-per-query k-nearest-neighbour search: the kNN behind CalcDensityParticle,
+// CalcVelDensityParticle, FindNearest / FindNearestPos of given tree particles, the coordinate
+// forms (FindNearest(x), CalcDensityPosition, CalcVelDensityPosition), and the queries that
+// the group search (knn_group.cu) leaves. A warp for 32 consecutive points walked the tree
+// for all of them at once: with points in no spatial order every lane's neighbourhood was
+// opened for the whole warp (250,007 points, k = 40, in 500,009 particles: 145 ms; a warp a
+// point does not depend on their order).
 //
 // Replaces the depth-first search of SplitNode/LeafNode::FindNearestPos(target)
 // (src/KDTree/KDSplitNode.cxx:15-41, KDLeafNode.cxx:15-28) with its bounded max-heap
@@ -527,15 +531,36 @@ __device__ __forceinline__ void wq_home(const TreeView& tv, int self, int want, 
   }
 }
 
+// The same for a query point that is no particle: the path follows the split planes
+// (SplitNode's left child holds the coordinates up to the split value).
+__device__ __forceinline__ void wq_home_point(const TreeView& tv, const double x[3], int want,
+                                              int& h, int& start, int& size) {
+  h = 0;
+  start = tv.pstart;
+  size = tv.n;
+  while (size > tv.b) {
+    const NodeX& nx = tv.nodex[tv.nbase + h];
+    const int d = nx.split_dim;
+    const double c = d == 0 ? x[0] : (d == 1 ? x[1] : x[2]);
+    const int ch = 2 * h + (c > nx.split_val ? 2 : 1);
+    const NodeRec& r = tv.node[tv.nbase + ch];
+    if (r.count < want) break;
+    h = ch;
+    start = r.start;
+    size = r.count;
+  }
+}
+
 // An FP32 upper bound of the k-th distance from the query's own subtree [hs, hs + hn):
 // a value T with at least K particles whose FP32 upper bound of the squared distance is
 // at or below T (bisection over the bit patterns, which order as the non-negative values
-// do), counting only particles provably at a non-zero distance and other than the query
-// (the target search skips those). Returns +inf when fewer than K qualify.
-// hn <= 2K + 1 <= 64 S + 1.
+// do), for a target search counting only particles provably at a non-zero distance and other
+// than the query (it skips those). Returns +inf when fewer than K qualify. A subtree larger
+// than 32 R particles (a large leaf) gives the bound of its first ones.
 template <int S>
 __device__ __forceinline__ float wq_home_bound(const WqQuery<S>& Q, const TreeView& tv, int lane,
-                                               int self, int hs, int hn, int K) {
+                                               int self, int hs, int hn, int K,
+                                               bool target) {
   const unsigned FULL = 0xffffffffu;
   constexpr int R = 2 * S + 1;
   unsigned hb[R];
@@ -548,7 +573,7 @@ __device__ __forceinline__ float wq_home_bound(const WqQuery<S>& Q, const TreeVi
       int ti = hs + c;
       float4 cf = tv.posf[ti];
       float lo = pair_d2_lo(Q.qx, Q.qy, Q.qz, cf.x, cf.y, cf.z, Q.two_eps);
-      if (ti != self && lo > 0.f) {
+      if (!target || (ti != self && lo > 0.f)) {
         hb[r] = __float_as_uint(pair_d2_hi(Q.qx, Q.qy, Q.qz, cf.x, cf.y, cf.z, Q.two_eps));
         mn = min(mn, hb[r]);
         mx = max(mx, hb[r]);
@@ -625,8 +650,8 @@ __device__ bool wq_search_f32(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int 
   return true;
 }
 
-// The search of one target query (tree index `self`, position x0): the direct pass
-// (seeded with the query's own subtree) and, on a periodic tree, the image passes with
+// The search of one query (tree index `self`, or -1 for a point; position x0): the direct
+// pass (seeded with the subtree around the query) and, on a periodic tree, the image passes with
 // the reference's gates. exclude_self: the target search of the direct pass skips the
 // query and zero distances (KDLeafNode.cxx:19-21). On return Q.L holds the K nearest.
 // F32FIRST: one-slot target searches without images take wq_search_f32 first (faster
@@ -645,12 +670,11 @@ __device__ void wq_search(WqQuery<S>& Q, WqSmem& w, const KnnArgs& a, const Tree
   Q.self = exclude_self ? self : -1;
   wq_set_point<S>(Q, tv, x0);
   int hh, hs, hn;
-  wq_home(tv, self, K + 1, hh, hs, hn);
-  if (exclude_self) Q.thr = fminf(Q.thr, wq_home_bound<S>(Q, tv, lane, self, hs, hn, K));
+  if (self >= 0) wq_home(tv, self, K + 1, hh, hs, hn);
+  else wq_home_point(tv, x0, K + 1, hh, hs, hn);
+  // the bound lets the rest of the tree be pruned at once
+  Q.thr = fminf(Q.thr, wq_home_bound<S>(Q, tv, lane, self, hs, hn, K, exclude_self));
   wq_range<S>(Q, w, tv, lane, hs, hn);
-  // with the bound the rest of the tree prunes at once; without it (coordinate search of
-  // the direct pass) the queue is flushed first so the k-th distance is known
-  if (!exclude_self) wq_drain<S>(Q, w, tv, lane);
   bool ok = hh == 0 || wq_traverse<S>(Q, w, tv, lane, hh);
   wq_drain<S>(Q, w, tv, lane);
   if (ok && a.periodic) {
@@ -771,7 +795,7 @@ __device__ __forceinline__ void wq_epilogue(const KnnArgs& a, const TreeView& tv
     // KDCalcSmoothQuantities.cxx:260-286: one neighbour per lane. 1 / h with
     // h = sqrt(top) / 2 (the reference divides by h) within a few ulps, far inside the
     // 1e-12 density tolerance
-    const double me_m = tv.pos[self].m;
+    const double me_m = EPI == kEpiDensPart ? 0.0 : tv.pos[self].m;
     double ih = two_rsqrt(__longlong_as_double(topk));
     double norm = dmul(dmul(ih, ih), ih);  // 1 / h^3 (the reference takes pow(h, 3))
     double wnorm = EPI == kEpiDensPart ? norm : 0.5 * norm;
@@ -802,7 +826,9 @@ __device__ __forceinline__ void wq_epilogue(const KnnArgs& a, const TreeView& tv
   if (EPI == kEpiDensVel || EPI == kEpiVel || EPI == kEpiVelPart) {
     // KDCalcSmoothQuantities.cxx:354-383: |dv| of the Nsearch neighbours, keep the
     // Nsmooth smallest, h = 0.5 max, sum Wsm(|dv|/h) h^-3 with unit weights
-    V4 vi = tv.vel[self];
+    const V4 vi = self >= 0 ? tv.vel[self]
+                            : make_v4(a.qv[3 * (size_t)qi], a.qv[3 * (size_t)qi + 1],
+                                      a.qv[3 * (size_t)qi + 2], 0.0);
     long long vk[S];
 #pragma unroll
     for (int s = 0; s < S; s++) {

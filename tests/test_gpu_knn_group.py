@@ -72,3 +72,20 @@ def test_periodic_rows(gpu, port_built, method, n, b, k):
     oi, od = o.knn(k, method)
     assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), oi, od,
                      f"method {method}")
+
+
+@pytest.mark.parametrize("n,b,k", [(40, 16, 8), (3001, 1000, 32), (5003, 16, 33), (5003, 1, 64),
+                                   (5003, 16, 65), (4099, 16, 127)])
+def test_points(gpu, port_built, n, b, k):
+    """Points anywhere: on particles (zero distances count), beside them, outside the box."""
+    pos, mass, _ = inputs("clustered", n)
+    rng = np.random.default_rng(5)
+    x = np.concatenate([pos[:101], pos[::-1][:100] + rng.normal(size=(min(n, 100), 3)) * 1e-3,
+                        rng.random((99, 3)) * 3.0 - 1.0])
+    for per in (None, [1.0, 1.0, 1.0]):
+        o = oracle.OracleTree(pos, None, mass, b, 0, 0, 1000, per, backend="port", nthreads=8)
+        t = KDTree(pos, None, mass, b, kerntype=0, period=per)
+        nn, d2 = t.FindNearestPosPoints(x, k)
+        assert np.all(np.diff(d2, axis=1) >= 0)
+        oi, od = o.knn_pos(x, k)
+        assert_knn_equal(to_ids(nn, t.GetPerm()), d2, oi, od, f"points, period {per}")
