@@ -1360,8 +1360,6 @@ static int smooth_common(nbk_tree* t, int which, int qmode, const int32_t* targe
   if (weight) NBK_TRY(S.in(weight, t->n, &dw));
   if (mean) NBK_TRY(S.in(mean, nq, &dmean));
   NBK_TRY(S.out(out, (size_t)width * nq, &dout));
-  if (qmode == 0 && which != kSmVelPhys)
-    NBK_CUDA_TRY(cudaMemsetAsync(dout, 0, sizeof(double) * width * nq, t->st));
   NBK_TRY(clear_err(t));
   KnnArgs a = base_args(t);
   a.tv.periodic = 0;  // the smoothing functions search without images, as CalcDensity
@@ -1374,7 +1372,7 @@ static int smooth_common(nbk_tree* t, int which, int qmode, const int32_t* targe
   a.nq = (int)nq;
   a.nsmooth = nsmooth;
   SmoothArgs sa{a, nsmooth, drho, dsv, ddisp, dw, dmean, dout};
-  NBK_TRY(launch_smooth(sa, which, t->st));
+  NBK_TRY(launch_smooth(sa, which, S.alloc, t->st));
   NBK_TRY(S.finish());
   if (!t->dev()) NBK_TRY(check_err(t, "smoothing"));
   return NBK_OK;

@@ -153,7 +153,8 @@ int launch_wq(const KnnArgs& a, cudaStream_t st) {
   unsigned blocks = (unsigned)((a.nq + kWqWpb - 1) / kWqWpb);
   if (blocks == 0) return NBK_OK;
   static const char* kNames[] = {"knn_nn", "knn_density", "knn_density_veldensity", "knn_veldensity",
-                                 "knn_density_particle", "knn_veldensity_particle", "knn_density_save"};
+                                 "knn_density_particle", "knn_veldensity_particle", "knn_density_save",
+                                 "knn_save"};
   Phase ph(kNames[EPI], st);
   k_knn_wq<S, EPI><<<blocks, 32 * kWqWpb, 0, st>>>(a); note_launch();
   NBK_CUDA_TRY(cudaGetLastError());
@@ -256,6 +257,7 @@ int launch_knn(const KnnArgs& a, int epi, cudaStream_t st) {
     case kEpiDensPart: return launch_e<kEpiDensPart>(a, st);
     case kEpiVelPart: return launch_e<kEpiVelPart>(a, st);
     case kEpiDensSave: return launch_e<kEpiDensSave>(a, st);
+    case kEpiSave: return launch_e<kEpiSave>(a, st);
   }
   set_error("unknown kNN epilogue");
   return NBK_ERR_INVALID;

@@ -621,20 +621,22 @@ __device__ __noinline__ void grp_drop(int* bi, const P4* pos, int lane, int self
 }
 
 // The neighbours of one query: its buffer cut to the K nearest (indices in bi[0 .. K)).
-// Returns false when the query has to take the second launch; thr returns an FP32 bound at
-// or above the K-th squared distance.
+// Returns 0 when the query has to take the second launch, 2 when FP64 distances chose (the
+// buffer's squared distances are then no longer those of its indices), else 1; thr returns an
+// FP32 bound at or above the K-th squared distance.
 template <int S>
-__device__ bool grp_select(GrpSmem<S>& w, const TreeView& tv, int lane, int q, int self, int cnt,
+__device__ int grp_select(GrpSmem<S>& w, const TreeView& tv, int lane, int q, int self, int cnt,
                            int K, float two_e, float& thr) {
-  if (thr < 0.f || cnt < K) return false;
+  if (thr < 0.f || cnt < K) return 0;
   const GrpCut f = grp_tighten<S>(w.bs[q], w.bi[q], lane, cnt, K, 0, two_e);
   // every particle within the bound must have been taken, and every neighbour must be
   // provably at a non-zero distance: sqrt(s) (1 - 2^-20) > 2E
   const float zero2 = __fmul_ru(__fmul_ru(two_e, two_e), 1.01f);
-  if (f.thr < 0.f || f.thr > thr || f.smin <= zero2 || f.cnt > 32 * S + 32) return false;
+  if (f.thr < 0.f || f.thr > thr || f.smin <= zero2 || f.cnt > 32 * S + 32) return 0;
   thr = f.thr;
-  if (f.cnt > K) grp_drop<S>(w.bi[q], tv.pos, lane, self, f.cnt, K);
-  return true;
+  if (f.cnt == K) return 1;
+  grp_drop<S>(w.bi[q], tv.pos, lane, self, f.cnt, K);
+  return 2;
 }
 
 // Sums of the G rows of 32 S doubles, 32 / G lanes a row: on return the first of row q's
@@ -820,6 +822,58 @@ __device__ void grp_veldensity(const KnnArgs& a, const TreeView& tv, GrpSmem<S>&
   __syncwarp();
 }
 
+// One query's neighbour row, the farthest last. The FP32 squared distances name it unless
+// another one is within their rounding of it; then FP64 distances do.
+template <int S>
+__device__ __forceinline__ void grp_save(const KnnArgs& a, const TreeView& tv, GrpSmem<S>& w,
+                                         int lane, int q, int self, int how, int K, float two_e) {
+  const unsigned FULL = 0xffffffffu;
+  int idx[S];
+  unsigned sb[S], mx = 0u;
+#pragma unroll
+  for (int s = 0; s < S; s++) {
+    const int p = s * 32 + lane;
+    idx[s] = p < K ? w.bi[q][p] : 0;
+    sb[s] = p < K ? w.bs[q][p] : 0u;
+    mx = max(mx, sb[s]);
+  }
+  mx = __reduce_max_sync(FULL, mx);
+  int at = 0, c = 0;
+#pragma unroll
+  for (int s = 0; s < S; s++) {
+    const unsigned b = __ballot_sync(
+        FULL, s * 32 + lane < K &&
+                  grp_thresh(__uint_as_float(sb[s]), two_e) >= __uint_as_float(mx));
+    if (b) at = s * 32 + __ffs(b) - 1;
+    c += __popc(b);
+  }
+  if (how == 2 || c != 1) {
+    const P4 x = tv.pos[self];
+    long long key[S], km = 0;
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      key[s] = 0;
+      if (s * 32 + lane < K) {
+        const P4 y = tv.pos[idx[s]];
+        key[s] = dkey(dist2_exact(x.x, x.y, x.z, y.x, y.y, y.z));
+      }
+      km = max(km, key[s]);
+    }
+    km = warp_max_key(km);
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const unsigned b = __ballot_sync(FULL, s * 32 + lane < K && key[s] == km);
+      if (b) at = s * 32 + __ffs(b) - 1;
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < S; s++) {
+    const int p = s * 32 + lane;
+    if (p < K)
+      a.nn[(size_t)(self - a.q0) * K + (p == at ? K - 1 : (p == K - 1 ? at : p))] = idx[s];
+  }
+}
+
 // The warp-per-query search for the queries the group kernel left: a persistent grid over
 // the list fb[1 .. fb[0]] of tree indices.
 template <int S, int EPI>
@@ -845,8 +899,9 @@ __global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int de
   GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int g = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
-  if (g >= (1 << depth)) return;
+  int g = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
+  if (g >= (1 << (depth - a.slices))) return;
+  g += a.slice << (depth - a.slices);
   const TreeView& tv = a.tv;
   GrpLane L;
   int gs, gn;
@@ -857,7 +912,8 @@ __global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int de
   for (int q = 0; q < gn; q++) {
     float thr = __shfl_sync(FULL, L.thr, q);
     const int cnt = __shfl_sync(FULL, L.cnt, q), self = gs + q;
-    bool ok = grp_select<S>(w, tv, lane, q, self, cnt, K, two_e, thr);
+    const int how = grp_select<S>(w, tv, lane, q, self, cnt, K, two_e, thr);
+    bool ok = how != 0;
     if (EPI == kEpiNN && ok && a.periodic) {
       const float4 qf = tv.posf[self];
       const float qeps = __fmul_ru(2.f, tv.eps);
@@ -867,6 +923,7 @@ __global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int de
     }
     if (!ok) continue;
     okm |= 1u << q;
+    if (EPI == kEpiSave) grp_save<S>(a, tv, w, lane, q, self, how, K, two_e);
     if (EPI == kEpiNN) {
       const P4 x = tv.pos[self];
       long long key[S];
@@ -920,15 +977,17 @@ int launch_group(const KnnArgs& a, int K, cudaStream_t st) {
   NBK_CUDA_TRY(cudaGetDevice(&dev));
   NBK_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   int depth = 0;
-  while ((((int64_t)a.nq - 1) >> depth) + 1 > GrpCfg<S>::G) depth++;
-  while ((1 << depth) < 16 * nsm && (((int64_t)a.nq - 1) >> (depth + 1)) + 1 >= 2) depth++;
+  const int64_t n = a.tv.n;
+  while (((n - 1) >> depth) + 1 > GrpCfg<S>::G) depth++;
+  while ((1 << depth) < 16 * nsm && ((n - 1) >> (depth + 1)) + 1 >= 2) depth++;
   const size_t sm = sizeof(GrpSmem<S>) * kGrpWpb;
   NBK_TRY(ensure_dyn_smem((const void*)k_knn_group<S, EPI>, (int)sm));
   static const char* kNames[] = {"knn_nn", "knn_density", "knn_density_veldensity", "knn_veldensity",
-                                 "knn_density_particle", "knn_veldensity_particle", "knn_density_save"};
+                                 "knn_density_particle", "knn_veldensity_particle", "knn_density_save",
+                                 "knn_save"};
   NBK_CUDA_TRY(cudaMemsetAsync(a.fb, 0, sizeof(int), st));
   Phase ph(kNames[EPI], st);
-  const unsigned blocks = ((1u << depth) + kGrpWpb - 1) / kGrpWpb;
+  const unsigned blocks = ((1u << (depth - a.slices)) + kGrpWpb - 1) / kGrpWpb;
   k_knn_group<S, EPI><<<blocks, 32 * kGrpWpb, sm, st>>>(a, depth, K); note_launch();
   const unsigned lb = (unsigned)std::min<int64_t>(4 * nsm, ((int64_t)a.nq + kWqWpb - 1) / kWqWpb);
   if (a.kheap <= 32) k_knn_wq_list<1, EPI><<<lb, 32 * kWqWpb, 0, st>>>(a);
@@ -951,8 +1010,8 @@ int launch_group_e(const KnnArgs& a, cudaStream_t st) {
 
 bool group_search_serves(const KnnArgs& a) {
   const int K = a.periodic ? a.kheap - 1 : a.kheap;
-  return a.qmode == 0 && a.fb && a.nq == a.tv.n && a.kheap <= 128 && K >= 1 &&
-         a.nq >= 4 * (K + 1) && a.tv.eps < 1e11f && (a.exclude_self || a.periodic);
+  return a.qmode == 0 && a.fb && (a.nq == a.tv.n || a.slices > 0) && a.kheap <= 128 && K >= 1 &&
+         a.tv.n >= 4 * (K + 1) && a.tv.eps < 1e11f && (a.exclude_self || a.periodic);
 }
 
 int launch_knn_group(const KnnArgs& a, int epi, cudaStream_t st) {
@@ -962,6 +1021,7 @@ int launch_knn_group(const KnnArgs& a, int epi, cudaStream_t st) {
     case kEpiDensVel: return launch_group_e<kEpiDensVel>(a, st);
     case kEpiVel: return launch_group_e<kEpiVel>(a, st);
     case kEpiDensSave: return launch_group_e<kEpiDensSave>(a, st);
+    case kEpiSave: return launch_group_e<kEpiSave>(a, st);
   }
   set_error("unknown kNN epilogue");
   return NBK_ERR_INVALID;

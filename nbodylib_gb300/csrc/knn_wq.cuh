@@ -788,6 +788,13 @@ __device__ __forceinline__ void wq_epilogue(const KnnArgs& a, const TreeView& tv
   for (int s = 0; s < S; s++) missing |= (s * 32 + lane < K) && L.idx[s] < 0;
   if (__any_sync(FULL, missing)) {
     if (lane == 0) atomicExch(a.err, kErrTooFew);
+    if (EPI == kEpiSave && lane == 0) a.nn[(size_t)qi * K + K - 1] = -1;  // no row
+    return;
+  }
+  if (EPI == kEpiSave) {
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      if (s * 32 + lane < K) a.nn[(size_t)qi * K + s * 32 + lane] = L.idx[s];
     return;
   }
   const double* T = a.kernel;

@@ -107,6 +107,7 @@ enum Epi : int {
   kEpiDensPart = 4,    // CalcDensityParticle (gather only)
   kEpiVelPart = 5,     // CalcVelDensityParticle
   kEpiDensSave = 6,    // CalcDensity scatter + save neighbour lists (adjoint forward)
+  kEpiSave = 7,        // neighbour indices only, the farthest last (smoothing)
 };
 
 struct KnnArgs {
@@ -132,6 +133,8 @@ struct KnnArgs {
   int* err;
   const double* qv;   // query velocities of coordinate queries (CalcVelDensityPosition)
   int* fb;            // 1 + nq ints of scratch for the group search (null: a warp per query)
+  int slices, slice;  // kEpiSave over the particles [q0, q0 + nq) of the slice-th of 2^slices
+                      // nodes of one level (0, 0: the whole tree)
 };
 int launch_knn(const KnnArgs& a, int epi, cudaStream_t st);
 // The group search (knn_group.cu): every particle of a tree at once.
@@ -173,9 +176,9 @@ struct SmoothArgs {
   const double* disp;     // input order [n][9]
   const double* weight;   // input order [n]
   const double* mean;     // query order [nq]
-  double* out;            // input order (every-particle forms, zeroed) or query order
+  double* out;            // input order (every-particle forms) or query order
 };
-int launch_smooth(const SmoothArgs& s, int which, cudaStream_t st);
+int launch_smooth(const SmoothArgs& s, int which, DevAlloc& alloc, cudaStream_t st);
 
 // ---- batched path: many trees, one persistent launch
 struct WorkItem {

@@ -4,257 +4,390 @@
 //   CalcVelDensityWithPhysDensity[Particle] (:393-478, :922-990);
 //   CalcSmoothVel/CalcSmoothVelDisp {Particle,Position} (:992-1091, :1209-1306) and
 //   CalcSmoothLocalMean/CalcSmoothLocalDisp {Particle,Position} (:1539-1700), one-sided.
-// Each is an epilogue of the warp search of knn_core.cuh: the lane's heap holds its
-// neighbours when the search returns, so no neighbour list is stored. Per-particle inputs
-// (densities, mean velocities, dispersions, weights) and the every-particle outputs are in
-// input order and addressed through the tree's permutation; the scattered sums use FP64
-// atomics, so their summation order (not their terms) differs from the reference's.
-#include "knn_core.cuh"
+//
+// The neighbours come from the kNN search (the group search for every particle, a warp per
+// query else) as rows of indices with the farthest last; a thread per query then runs over
+// its row. What belongs to a particle and not to a pair is prepared once per particle in
+// tree order (m / rho, the mean velocity, the inverse powers of the dispersion: divisions
+// and permutations out of the pair loop), and the every-particle sums are gathered with FP64
+// atomics in tree order, where neighbours are close in memory, then permuted. The summation
+// order (not the terms) differs from the reference's. A row costs 4 B per neighbour each way;
+// trees of more than kSliceMax particles go slice by slice, so that the rows stay small.
+//
+// What bounds it: the FP64 pipe, 19 instructions a pair for CalcSmoothVel and 37 for
+// CalcSmoothVelDisp (its nine sums are six, the matrix being symmetric). As epilogues of a
+// lane-per-query search with all divisions per pair the two took 8.2 ms each at 2^20
+// clustered particles, Nsmooth = 32.
+#include <algorithm>
+
+#include "knn_wq.cuh"
 
 namespace nbk {
 
 namespace {
 
-// 1 / x^1.5 as the reference's pow(x, 1.5) in the denominator of the skewness.
-__device__ __forceinline__ double inv_pow15(double x) { return 1.0 / dmul(x, __dsqrt_rn(x)); }
+constexpr int64_t kSliceMax = int64_t(1) << 23;  // queries per slice of rows
 
-template <int KMAX, int SM>
-__device__ void smooth_warp(const SmoothArgs& s, const TreeView& tv, WarpSmem<KMAX>& w, int lane,
-                            bool valid, int qi, int self, const double x0[3], int K) {
-  const KnnArgs& a = s.k;
-  double top = knn_search<KMAX>(a, tv, w, lane, valid, self, x0, K);
-  if (!valid) return;
-  for (int q = 0; q < K; q++)
-    if (w.hi[q][lane] < 0) {
-      atomicExch(a.err, kErrTooFew);
-      return;
-    }
-  const int kr = a.kernres;
-  const double inv_delta = 0.5 * (double)(kr - 1);
-  const double* T = a.kernel;
+// One particle's share of the pair terms, tree order.
+struct SmoothPrep {
+  const double* mr;  // m / rho
+  const V4* sv;      // mean velocity (moment forms)
+  const V4* iv;      // inverse power of the dispersion's diagonal (skewness, kurtosis)
+  const double* wt;  // weights (local mean and dispersion)
+};
 
-  if (SM == kSmVelPhys) {
-    // |dv| of the Nsearch neighbours, the Nsmooth smallest kept (as CalcVelDensity); the
-    // physical h is half the largest *squared* distance, as the reference computes it
-    // (:428); a table index past the end gives the table's last entry (the reference
-    // reads past its table there).
-    V4 vi = tv.vel[self];
-    P4 pi = tv.pos[self];
-    for (int q = 0; q < K; q++) {
-      V4 vj = tv.vel[w.hi[q][lane]];
-      w.hd[q][lane] = __dsqrt_rn(dist2_exact(vi.x, vi.y, vi.z, vj.x, vj.y, vj.z));
+__global__ void k_smooth_prep(SmoothArgs s, int n, int which, double* mr, V4* sv, V4* iv,
+                              double* wt) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int64_t id = s.k.tv.perm[t];
+  mr[t] = s.k.tv.pos[t].m / s.rho[id];
+  if (sv) sv[t] = make_v4(s.smvel[3 * id], s.smvel[3 * id + 1], s.smvel[3 * id + 2], 0.0);
+  if (iv) {
+    double v[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const double d = s.disp[9 * id + 4 * k];
+      // the reference's 1 / pow(d, 1.5), and 1 / (d d)
+      v[k] = which == kSmVelSkew ? 1.0 / dmul(d, __dsqrt_rn(d)) : 1.0 / dmul(d, d);
     }
-    int ns = min(s.nsmooth, K);
-    if (ns < K) {
-      for (int q = ns / 2 - 1; q >= 0; q--) {
-        double d = w.hd[q][lane];
-        int j = w.hi[q][lane];
-        heap_sift<KMAX>(w, lane, ns, q, d, j);
-      }
-      for (int q = ns; q < K; q++) {
-        double d = w.hd[q][lane];
-        if (dkey(d) < dkey(w.hd[0][lane])) heap_sift<KMAX>(w, lane, ns, 0, d, w.hi[q][lane]);
-      }
-    }
-    long long vmaxk = 0;
-    for (int q = 0; q < ns; q++) vmaxk = max(vmaxk, dkey(w.hd[q][lane]));
-    double vih = 1.0 / (0.5 * __longlong_as_double(vmaxk));
-    double vnorm = dmul(dmul(vih, vih), vih);
-    double ih = 1.0 / (0.5 * top);
-    double norm = dmul(dmul(ih, ih), ih);
-    double ri = s.rho[tv.perm[self]];
-    double acc = 0.0;
-    for (int q = 0; q < ns; q++) {
-      int j = w.hi[q][lane];
-      P4 pj = tv.pos[j];
-      double rij = __dsqrt_rn(dist2_exact(pi.x, pi.y, pi.z, pj.x, pj.y, pj.z));
-      const double vd = w.hd[q][lane];  // the largest |dv| is at q = 2 exactly
-      double vw = dmul(dkey(vd) == vmaxk ? T[kr - 1] : wsm_line(dmul(vd, vih), kr, inv_delta, T),
-                       vnorm);
-      double wij = dmul(wsm_line(dmul(rij, ih), kr, inv_delta, T), norm);
-      acc = dadd(acc, dmul(vw, dmul(wij / ri, pi.m)));
-    }
-    if (a.qmode == 0) s.out[tv.perm[self]] = acc;
-    else s.out[qi] = acc;
-    return;
+    iv[t] = make_v4(v[0], v[1], v[2], 0.0);
   }
-
-  // the SPH weights of the Nsmooth nearest: h = half the largest distance
-  double ih = 1.0 / (0.5 * __dsqrt_rn(top));
-  const long long topk = dkey(top);
-  double norm = dmul(dmul(ih, ih), ih);
-  constexpr bool kSym = SM == kSmVel || SM == kSmVelDisp || SM == kSmVelSkew || SM == kSmVelKurt;
-  double wnorm = kSym ? 0.5 * norm : norm;  // the symmetric forms carry the 1/2
-
-  if (kSym) {
-    const int id = tv.perm[self];
-    P4 pi = tv.pos[self];
-    V4 vi = tv.vel[self];
-    const double vi3[3] = {vi.x, vi.y, vi.z};
-    const double tb0 = pi.m / s.rho[id];  // the target's weight factor, times W_ij
-    double svi[3] = {0, 0, 0}, ddi[3] = {1, 1, 1};
-    if (SM != kSmVel)
-      for (int k = 0; k < 3; k++) svi[k] = s.smvel[3 * (size_t)id + k];
-    if (SM == kSmVelSkew || SM == kSmVelKurt)
-      for (int k = 0; k < 3; k++) ddi[k] = s.disp[9 * (size_t)id + 4 * k];
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int q = 0; q < K; q++) {
-      int j = w.hi[q][lane];
-      int jd = tv.perm[j];
-      double wij = dmul(w_at_d2(w.hd[q][lane], topk, ih, kr, inv_delta, T), wnorm);
-      P4 pj = tv.pos[j];
-      V4 vj = tv.vel[j];
-      const double vj3[3] = {vj.x, vj.y, vj.z};
-      double ta = dmul(wij / s.rho[jd], pj.m);  // Wij / rho_j * m_j, summed into the target
-      double tb = dmul(wij, tb0) ;              // Wij / rho_i * m_i, summed into neighbour j
-      if (SM == kSmVel) {
-        for (int k = 0; k < 3; k++) {
-          acc[k] = dadd(acc[k], dmul(ta, vj3[k]));
-          atomicAdd(&s.out[3 * (size_t)jd + k], dmul(tb, vi3[k]));
-        }
-      } else if (SM == kSmVelDisp) {
-        double svj[3];
-        for (int k = 0; k < 3; k++) svj[k] = s.smvel[3 * (size_t)jd + k];
-        for (int k = 0; k < 3; k++)
-          for (int l = 0; l < 3; l++) {
-            acc[3 * k + l] = dadd(acc[3 * k + l],
-                                  dmul(dmul(ta, dsub(vj3[k], svi[k])), dsub(vj3[l], svi[l])));
-            atomicAdd(&s.out[9 * (size_t)jd + 3 * k + l],
-                      dmul(dmul(tb, dsub(vi3[k], svj[k])), dsub(vi3[l], svj[l])));
-          }
-      } else {
-        for (int k = 0; k < 3; k++) {
-          double dv = dsub(vj3[k], svi[k]);
-          double du = dsub(vi3[k], s.smvel[3 * (size_t)jd + k]);
-          double djk = s.disp[9 * (size_t)jd + 4 * k];
-          if (SM == kSmVelSkew) {
-            acc[k] = dadd(acc[k], dmul(dmul(dmul(ta, dv), dv), dv) * inv_pow15(ddi[k]));
-            atomicAdd(&s.out[3 * (size_t)jd + k],
-                      dmul(dmul(dmul(tb, du), du), du) * inv_pow15(djk));
-          } else {
-            // the reference subtracts 3 in every neighbour's term
-            acc[k] = dadd(acc[k], dsub(dmul(dmul(dmul(dmul(ta, dv), dv), dv), dv) /
-                                           dmul(ddi[k], ddi[k]), 3.0));
-            atomicAdd(&s.out[3 * (size_t)jd + k],
-                      dsub(dmul(dmul(dmul(dmul(tb, du), du), du), du) / dmul(djk, djk), 3.0));
-          }
-        }
-      }
-    }
-    const int width = SM == kSmVelDisp ? 9 : 3;
-    for (int k = 0; k < width; k++) atomicAdd(&s.out[(size_t)width * id + k], acc[k]);
-    return;
-  }
-
-  // one-sided forms: the query's own sums
-  double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  double sv[3] = {0, 0, 0};
-  if (SM == kSmVelDispOne)
-    for (int k = 0; k < 3; k++) sv[k] = s.smvel[3 * (size_t)qi + k];
-  const double mean = SM == kSmDispOne ? s.mean[qi] : 0.0;
-  for (int q = 0; q < K; q++) {
-    int j = w.hi[q][lane];
-    int jd = tv.perm[j];
-    double wij = dmul(w_at_d2(w.hd[q][lane], topk, ih, kr, inv_delta, T), wnorm);
-    double ta = dmul(wij / s.rho[jd], tv.pos[j].m);
-    if (SM == kSmVelOne || SM == kSmVelDispOne) {
-      V4 vj = tv.vel[j];
-      const double vj3[3] = {vj.x, vj.y, vj.z};
-      if (SM == kSmVelOne) {
-        for (int k = 0; k < 3; k++) acc[k] = dadd(acc[k], dmul(ta, vj3[k]));
-      } else {
-        for (int k = 0; k < 3; k++)
-          for (int l = 0; l < 3; l++)
-            acc[3 * k + l] = dadd(acc[3 * k + l],
-                                  dmul(dmul(ta, dsub(vj3[k], sv[k])), dsub(vj3[l], sv[l])));
-      }
-    } else if (SM == kSmMeanOne) {
-      acc[0] = dadd(acc[0], dmul(ta, s.weight[jd]));
-    } else {
-      double dl = dsub(s.weight[jd], mean);
-      acc[0] = dadd(acc[0], dmul(dmul(ta, dl), dl));
-    }
-  }
-  const int width = SM == kSmVelDispOne ? 9 : (SM == kSmVelOne ? 3 : 1);
-  for (int k = 0; k < width; k++) s.out[(size_t)width * qi + k] = acc[k];
+  if (wt) wt[t] = s.weight[id];
 }
 
-template <int KMAX, int SM>
-__global__ void __launch_bounds__(32 * warps_per_block<KMAX>()) k_smooth(SmoothArgs s) {
-  constexpr int WPB = warps_per_block<KMAX>();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  WarpSmem<KMAX>* ws = reinterpret_cast<WarpSmem<KMAX>*>(smem_raw);
+// Sums per particle in tree order to input order; the dispersion's six to its nine.
+template <int W>
+__global__ void k_smooth_out(const double* acc, const int* perm, double* out, int n) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int64_t id = perm[t];
+  if (W == 6) {
+    const int at[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+#pragma unroll
+    for (int c = 0; c < 9; c++) out[9 * id + c] = acc[6 * (int64_t)t + at[c]];
+  } else {
+#pragma unroll
+    for (int c = 0; c < W; c++) out[W * id + c] = acc[W * (int64_t)t + c];
+  }
+}
+
+template <int SM>
+__global__ void __launch_bounds__(128) k_smooth_rows(SmoothArgs s, SmoothPrep P, int K,
+                                                     double* acc_out) {
   const KnnArgs& a = s.k;
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int gw = blockIdx.x * WPB + warp;
-  int qi = gw * 32 + lane;
-  if (gw * 32 >= a.nq) return;
   const TreeView& tv = a.tv;
-  bool valid = qi < a.nq;
+  const int qi = blockIdx.x * blockDim.x + threadIdx.x;
+  if (qi >= a.nq) return;
+  const int* row = a.nn + (size_t)qi * K;
+  constexpr bool kSym = SM == kSmVel || SM == kSmVelDisp || SM == kSmVelSkew || SM == kSmVelKurt;
   int self = -1;
-  double x0[3] = {0, 0, 0};
-  if (valid) {
-    if (a.qmode == 0) self = a.q0 + qi;
-    else if (a.qmode == 2) self = a.qidx[qi];
-    if (a.qmode == 2 && (self < 0 || self >= tv.n)) {
-      atomicExch(a.err, kErrTarget);
-      valid = false;
-      self = 0;
-    }
-    if (a.qmode == 1) {
-      x0[0] = a.qx[3 * (size_t)qi];
-      x0[1] = a.qx[3 * (size_t)qi + 1];
-      x0[2] = a.qx[3 * (size_t)qi + 2];
+  double x, y, z;
+  if (a.qmode == 1) {
+    x = a.qx[3 * (size_t)qi];
+    y = a.qx[3 * (size_t)qi + 1];
+    z = a.qx[3 * (size_t)qi + 2];
+  } else {
+    self = a.qmode == 0 ? a.q0 + qi : a.qidx[qi];
+    if (self < 0 || self >= tv.n) return;  // reported by the search
+    const P4 p = tv.pos[self];
+    x = p.x;
+    y = p.y;
+    z = p.z;
+  }
+  if (row[K - 1] < 0) return;  // too few neighbours: reported by the search
+  const int kr = a.kernres;
+  const double* T = a.kernel;
+  // the weights of the neighbours: h = half the largest distance
+  double top;
+  {
+    const P4 c = tv.pos[row[K - 1]];
+    const double dx = dsub(x, c.x), dy = dsub(y, c.y), dz = dsub(z, c.z);
+    top = __fma_rn(dz, dz, __fma_rn(dy, dy, dmul(dx, dx)));
+  }
+  const double ih = two_rsqrt(top), c1 = dmul(ih, 0.5 * (double)(kr - 1));
+  const double norm = dmul(dmul(ih, ih), ih);
+  const double wnorm = kSym ? 0.5 * norm : norm;  // the symmetric forms carry the 1/2
+  V4 vi = make_v4(0, 0, 0, 0), si = vi;
+  double wi = 0.0;  // this particle's factor in its neighbours' sums
+  if (kSym) {
+    vi = tv.vel[self];
+    wi = dmul(wnorm, P.mr[self]);
+    if (SM != kSmVel) si = P.sv[self];
+  }
+  V4 ivi = make_v4(0, 0, 0, 0);
+  if (SM == kSmVelSkew || SM == kSmVelKurt) ivi = P.iv[self];
+  if (SM == kSmVelDispOne)
+    si = make_v4(s.smvel[3 * (size_t)qi], s.smvel[3 * (size_t)qi + 1], s.smvel[3 * (size_t)qi + 2],
+                 0.0);
+  const double mean = SM == kSmDispOne ? s.mean[qi] : 0.0;
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  for (int q = 0; q < K; q++) {
+    const int j = row[q];
+    const P4 c = tv.pos[j];
+    const double dx = dsub(x, c.x), dy = dsub(y, c.y), dz = dsub(z, c.z);
+    const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dmul(dx, dx)));
+    // the farthest neighbour sits at q = 2 exactly: the table's last entry
+    const double w = d2 == top ? T[kr - 1] : w_at_u(dmul(sqrt_newton(d2), c1), kr, T);
+    const double ta = dmul(dmul(w, wnorm), P.mr[j]);  // W_ij m_j / rho_j, into the query
+    const double tb = dmul(w, wi);                    // W_ij m_i / rho_i, into neighbour j
+    if (SM == kSmMeanOne) {
+      acc[0] = __fma_rn(ta, P.wt[j], acc[0]);
+    } else if (SM == kSmDispOne) {
+      const double dl = dsub(P.wt[j], mean);
+      acc[0] = __fma_rn(dmul(ta, dl), dl, acc[0]);
+    } else if (SM == kSmVel || SM == kSmVelOne) {
+      const V4 vj = tv.vel[j];
+      acc[0] = __fma_rn(ta, vj.x, acc[0]);
+      acc[1] = __fma_rn(ta, vj.y, acc[1]);
+      acc[2] = __fma_rn(ta, vj.z, acc[2]);
+      if (SM == kSmVel) {
+        double* o = acc_out + 3 * (size_t)j;
+        atomicAdd(o, dmul(tb, vi.x));
+        atomicAdd(o + 1, dmul(tb, vi.y));
+        atomicAdd(o + 2, dmul(tb, vi.z));
+      }
     } else {
-      P4 p = tv.pos[self];
-      x0[0] = p.x;
-      x0[1] = p.y;
-      x0[2] = p.z;
+      const V4 vj = tv.vel[j];
+      const double d[3] = {dsub(vj.x, si.x), dsub(vj.y, si.y), dsub(vj.z, si.z)};
+      if (SM == kSmVelDisp || SM == kSmVelDispOne) {
+        const double e[3] = {dmul(ta, d[0]), dmul(ta, d[1]), dmul(ta, d[2])};
+        acc[0] = __fma_rn(e[0], d[0], acc[0]);
+        acc[1] = __fma_rn(e[0], d[1], acc[1]);
+        acc[2] = __fma_rn(e[0], d[2], acc[2]);
+        acc[3] = __fma_rn(e[1], d[1], acc[3]);
+        acc[4] = __fma_rn(e[1], d[2], acc[4]);
+        acc[5] = __fma_rn(e[2], d[2], acc[5]);
+      }
+      if (kSym) {
+        const V4 sj = P.sv[j];
+        const double u[3] = {dsub(vi.x, sj.x), dsub(vi.y, sj.y), dsub(vi.z, sj.z)};
+        if (SM == kSmVelDisp) {
+          const double f[3] = {dmul(tb, u[0]), dmul(tb, u[1]), dmul(tb, u[2])};
+          double* o = acc_out + 6 * (size_t)j;
+          atomicAdd(o, dmul(f[0], u[0]));
+          atomicAdd(o + 1, dmul(f[0], u[1]));
+          atomicAdd(o + 2, dmul(f[0], u[2]));
+          atomicAdd(o + 3, dmul(f[1], u[1]));
+          atomicAdd(o + 4, dmul(f[1], u[2]));
+          atomicAdd(o + 5, dmul(f[2], u[2]));
+        } else {
+          const V4 ivj = P.iv[j];
+          const double ii[3] = {ivi.x, ivi.y, ivi.z}, ij[3] = {ivj.x, ivj.y, ivj.z};
+          double* o = acc_out + 3 * (size_t)j;
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            const double a3 = dmul(dmul(dmul(ta, d[k]), d[k]), d[k]);
+            const double b3 = dmul(dmul(dmul(tb, u[k]), u[k]), u[k]);
+            if (SM == kSmVelSkew) {
+              acc[k] = __fma_rn(a3, ii[k], acc[k]);
+              atomicAdd(o + k, dmul(b3, ij[k]));
+            } else {
+              // the reference subtracts 3 in every neighbour's term
+              acc[k] = dadd(acc[k], dsub(dmul(dmul(a3, d[k]), ii[k]), 3.0));
+              atomicAdd(o + k, dsub(dmul(dmul(b3, u[k]), ij[k]), 3.0));
+            }
+          }
+        }
+      }
     }
   }
-  smooth_warp<KMAX, SM>(s, tv, ws[warp], lane, valid, qi, self, x0, a.kheap);
+  constexpr int kAcc = SM == kSmVelDisp || SM == kSmVelDispOne ? 6
+                       : SM == kSmMeanOne || SM == kSmDispOne  ? 1
+                                                               : 3;
+  if (kSym) {
+#pragma unroll
+    for (int k = 0; k < kAcc; k++) atomicAdd(acc_out + kAcc * (size_t)self + k, acc[k]);
+  } else if (SM == kSmVelDispOne) {
+    const int at[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+#pragma unroll
+    for (int c = 0; c < 9; c++) s.out[9 * (size_t)qi + c] = acc[at[c]];
+  } else {
+#pragma unroll
+    for (int k = 0; k < kAcc; k++) s.out[kAcc * (size_t)qi + k] = acc[k];
+  }
 }
 
-template <int KMAX, int SM>
-int launch_st(const SmoothArgs& s, cudaStream_t st) {
-  constexpr int WPB = warps_per_block<KMAX>();
-  size_t sm = sizeof(WarpSmem<KMAX>) * WPB;
-  NBK_TRY(ensure_dyn_smem((const void*)k_smooth<KMAX, SM>, (int)sm));
-  int blocks = ((s.k.nq + 31) / 32 + WPB - 1) / WPB;
-  if (blocks == 0) return NBK_OK;
-  Phase ph("smooth", st);
-  k_smooth<KMAX, SM><<<blocks, 32 * WPB, sm, st>>>(s); note_launch();
+// CalcVelDensityWithPhysDensity: a warp per query, a neighbour per lane and slot. |dv| of the
+// Nsearch neighbours, the Nsmooth smallest kept (as CalcVelDensity); the physical h is half
+// the largest *squared* distance, as the reference computes it (:428); a table index past the
+// end gives the table's last entry (the reference reads past its table there).
+template <int S>
+__global__ void __launch_bounds__(256) k_smooth_velphys(SmoothArgs s, SmoothPrep P, int K) {
+  const unsigned FULL = 0xffffffffu;
+  const KnnArgs& a = s.k;
+  const TreeView& tv = a.tv;
+  const int lane = threadIdx.x & 31;
+  const int qi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (qi >= a.nq) return;
+  const int self = a.qmode == 0 ? a.q0 + qi : a.qidx[qi];
+  if (self < 0 || self >= tv.n) return;  // reported by the search
+  const int kr = a.kernres;
+  const double* T = a.kernel;
+  const int* row = a.nn + (size_t)qi * K;
+  if (row[K - 1] < 0) return;  // too few neighbours: reported by the search
+  const P4 x = tv.pos[self];
+  const V4 v = tv.vel[self];
+  double d2[S];
+  long long vk[S], top = 0;
+#pragma unroll
+  for (int q = 0; q < S; q++) {
+    const int p = q * 32 + lane;
+    vk[q] = kWqSent;
+    d2[q] = 0.0;
+    if (p < K) {
+      const int j = row[p];
+      const V4 vj = tv.vel[j];
+      const P4 c = tv.pos[j];
+      vk[q] = dkey(sqrt_newton(dist2_exact(v.x, v.y, v.z, vj.x, vj.y, vj.z)));
+      d2[q] = dist2_exact(x.x, x.y, x.z, c.x, c.y, c.z);
+      top = max(top, dkey(d2[q]));
+    }
+  }
+  const int ns = min(s.nsmooth, K);
+  int rk[S];
+  if (ns < K) wq_ranks<S>(vk, lane, K, rk);
+  bool sel[S];
+  long long vmax = 0;
+#pragma unroll
+  for (int q = 0; q < S; q++) {
+    sel[q] = q * 32 + lane < K && (ns == K || rk[q] < ns);
+    if (sel[q]) vmax = max(vmax, vk[q]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    vmax = max(vmax, __shfl_xor_sync(FULL, vmax, o));
+    top = max(top, __shfl_xor_sync(FULL, top, o));
+  }
+  const double vih = recip_newton(0.5 * __longlong_as_double(vmax));
+  const double vnorm = dmul(dmul(vih, vih), vih);
+  const double ih = recip_newton(0.5 * __longlong_as_double(top));
+  const double norm = dmul(dmul(ih, ih), ih);
+  const double hk = 0.5 * (double)(kr - 1), mr = P.mr[self];
+  double acc = 0.0;
+#pragma unroll
+  for (int q = 0; q < S; q++) {
+    if (!sel[q]) continue;
+    const double vw = vk[q] == vmax  // the largest |dv| is at q = 2 exactly
+                          ? T[kr - 1]
+                          : w_at_u(dmul(dmul(__longlong_as_double(vk[q]), vih), hk), kr, T);
+    const double w = w_at_u(dmul(dmul(sqrt_newton(d2[q]), ih), hk), kr, T);
+    acc = __fma_rn(dmul(vw, vnorm), dmul(dmul(w, norm), mr), acc);
+  }
+  acc = warp_sum(acc);
+  if (lane == 0) s.out[a.qmode == 0 ? tv.perm[self] : qi] = acc;
+}
+
+// Start and size of the slice-th of the 2^levels nodes of a level (KDTree.cxx:1012).
+void slice_range(int64_t n, int levels, int slice, int64_t* start, int64_t* size) {
+  int64_t s = 0;
+  for (int i = levels - 1; i >= 0; i--) {
+    const int64_t l = (n - 1) / 2 + 1;
+    if ((slice >> i) & 1) {
+      s += l;
+      n -= l;
+    } else {
+      n = l;
+    }
+  }
+  *start = s;
+  *size = n;
+}
+
+template <int SM>
+int rows_pass(const SmoothArgs& s, const SmoothPrep& P, int K, double* acc, cudaStream_t st) {
+  k_smooth_rows<SM><<<(unsigned)((s.k.nq + 127) / 128), 128, 0, st>>>(s, P, K, acc);
+  note_launch();
   NBK_CUDA_TRY(cudaGetLastError());
   return NBK_OK;
 }
 
-template <int SM>
-int launch_s(const SmoothArgs& s, cudaStream_t st) {
-  int k = s.k.kheap;
-  if (k <= 16) return launch_st<16, SM>(s, st);
-  if (k <= 33) return launch_st<33, SM>(s, st);
-  if (k <= 65) return launch_st<65, SM>(s, st);
-  if (k <= 128) return launch_st<128, SM>(s, st);
-  set_error("smoothing over more than 128 neighbours is not supported");
-  return NBK_ERR_UNSUPPORTED;
-}
-
 }  // namespace
 
-int launch_smooth(const SmoothArgs& s, int which, cudaStream_t st) {
-  switch (which) {
-    case kSmVel: return launch_s<kSmVel>(s, st);
-    case kSmVelDisp: return launch_s<kSmVelDisp>(s, st);
-    case kSmVelSkew: return launch_s<kSmVelSkew>(s, st);
-    case kSmVelKurt: return launch_s<kSmVelKurt>(s, st);
-    case kSmVelPhys: return launch_s<kSmVelPhys>(s, st);
-    case kSmVelOne: return launch_s<kSmVelOne>(s, st);
-    case kSmVelDispOne: return launch_s<kSmVelDispOne>(s, st);
-    case kSmMeanOne: return launch_s<kSmMeanOne>(s, st);
-    case kSmDispOne: return launch_s<kSmDispOne>(s, st);
+int launch_smooth(const SmoothArgs& s0, int which, DevAlloc& alloc, cudaStream_t st) {
+  const int K = s0.k.kheap;
+  if (which < kSmVel || which > kSmDispOne) {
+    set_error("unknown smoothing quantity");
+    return NBK_ERR_INVALID;
   }
-  set_error("unknown smoothing quantity");
-  return NBK_ERR_INVALID;
+  if (K > 128) {
+    set_error("smoothing over more than 128 neighbours is not supported");
+    return NBK_ERR_UNSUPPORTED;
+  }
+  if (s0.k.nq == 0) return NBK_OK;
+  const int n = s0.k.tv.n;
+  const int64_t nq = s0.k.nq;
+  const bool sym = which <= kSmVelKurt, every = s0.k.qmode == 0;
+  const int width = which == kSmVelDisp ? 6 : 3;
+  // slices of the queries: nodes of one level for every particle, plain ranges else
+  int levels = 0;
+  while (every && (nq >> levels) > kSliceMax) levels++;
+  const int64_t step = every ? (((nq - 1) >> levels) + 1) : std::min(nq, kSliceMax);
+  const int slices = every ? 1 << levels : (int)((nq + step - 1) / step);
+  double *mr, *acc = nullptr, *wt = nullptr;
+  V4 *sv = nullptr, *iv = nullptr;
+  int *rows, *fb = nullptr;
+  std::vector<DevPart> parts{{(void**)&mr, sizeof(double) * n},
+                             {(void**)&rows, sizeof(int) * step * K}};
+  if (sym) parts.push_back({(void**)&acc, sizeof(double) * width * n});
+  if (sym && which != kSmVel) parts.push_back({(void**)&sv, sizeof(V4) * n});
+  if (which == kSmVelSkew || which == kSmVelKurt) parts.push_back({(void**)&iv, sizeof(V4) * n});
+  if (which == kSmMeanOne || which == kSmDispOne) parts.push_back({(void**)&wt, sizeof(double) * n});
+  if (every) parts.push_back({(void**)&fb, sizeof(int) * (step + 1)});
+  NBK_TRY(alloc.get_block(parts));
+  if (sym) NBK_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(double) * width * n, st));
+  Phase ph("smooth", st);
+  const unsigned nb = (unsigned)((n + 255) / 256);
+  k_smooth_prep<<<nb, 256, 0, st>>>(s0, n, which, mr, sv, iv, wt);
+  note_launch();
+  const SmoothPrep P{mr, sv, iv, wt};
+  for (int i = 0; i < slices; i++) {
+    SmoothArgs s = s0;
+    s.k.nn = rows;
+    s.k.fb = fb;
+    if (every) {
+      int64_t start, size;
+      slice_range(nq, levels, i, &start, &size);
+      s.k.q0 = (int)start;
+      s.k.nq = (int)size;
+      s.k.slices = levels;
+      s.k.slice = i;
+    } else {
+      const int64_t o = i * step;
+      s.k.nq = (int)std::min(step, nq - o);
+      if (s.k.qidx) s.k.qidx += o;
+      if (s.k.qx) s.k.qx += 3 * o;
+      if (s.smvel) s.smvel += 3 * o;
+      if (s.mean) s.mean += o;
+      s.out += o * (which == kSmVelDispOne ? 9 : which == kSmVelOne ? 3 : 1);
+    }
+    NBK_TRY(launch_knn(s.k, kEpiSave, st));
+    switch (which) {
+      case kSmVel: NBK_TRY(rows_pass<kSmVel>(s, P, K, acc, st)); break;
+      case kSmVelDisp: NBK_TRY(rows_pass<kSmVelDisp>(s, P, K, acc, st)); break;
+      case kSmVelSkew: NBK_TRY(rows_pass<kSmVelSkew>(s, P, K, acc, st)); break;
+      case kSmVelKurt: NBK_TRY(rows_pass<kSmVelKurt>(s, P, K, acc, st)); break;
+      case kSmVelOne: NBK_TRY(rows_pass<kSmVelOne>(s, P, K, acc, st)); break;
+      case kSmVelDispOne: NBK_TRY(rows_pass<kSmVelDispOne>(s, P, K, acc, st)); break;
+      case kSmMeanOne: NBK_TRY(rows_pass<kSmMeanOne>(s, P, K, acc, st)); break;
+      case kSmDispOne: NBK_TRY(rows_pass<kSmDispOne>(s, P, K, acc, st)); break;
+      default: {
+        const unsigned blocks = (unsigned)((s.k.nq + 7) / 8);
+        if (K <= 32) k_smooth_velphys<1><<<blocks, 256, 0, st>>>(s, P, K);
+        else if (K <= 64) k_smooth_velphys<2><<<blocks, 256, 0, st>>>(s, P, K);
+        else k_smooth_velphys<4><<<blocks, 256, 0, st>>>(s, P, K);
+        note_launch();
+        NBK_CUDA_TRY(cudaGetLastError());
+      }
+    }
+  }
+  if (sym) {
+    if (width == 6) k_smooth_out<6><<<nb, 256, 0, st>>>(acc, s0.k.tv.perm, s0.out, n);
+    else k_smooth_out<3><<<nb, 256, 0, st>>>(acc, s0.k.tv.perm, s0.out, n);
+    note_launch();
+    NBK_CUDA_TRY(cudaGetLastError());
+  }
+  return NBK_OK;
 }
 
 }  // namespace nbk
