@@ -6,8 +6,10 @@
 //  - build: every group is one tree of a forest; one build_forest call builds them all
 //    (groups of <= 1024 particles are finished by one CTA each, larger groups go through
 //    the level-synchronous phase together).
-//  - search: one persistent launch; its warps pull (group, query bucket) work items, the
-//    largest groups first, from an atomic counter.
+//  - search: the group search of knn_group.cu over the whole forest, a warp for at most 8
+//    neighbouring particles of one group; or (query mapping 0) one persistent launch whose
+//    warps pull (group, query bucket) work items, the largest groups first, from an atomic
+//    counter and serve a query per lane.
 //  - the zeroing, the search and the scatter back to input order are captured once into
 //    a CUDA graph per (k, output) and replayed.
 //  - leaf size and query-bucket size are chosen by a small autotuner (bucket_size <= 0 at
@@ -39,8 +41,13 @@ struct nbk_batch {
   double* d_mass_in = nullptr;
   bool own_inputs = false;
   TreeInfo* d_trees = nullptr;
-  WorkItem* d_items = nullptr;
+  WorkItem* d_items = nullptr;  // lane-per-query form only: made at its first use
   int nitems = 0;
+  int* d_goff = nullptr;    // first search group of each tree for groups of 8, 4, 2; pstart
+  int ntrees = 0;           // non-empty trees (the entries of d_trees)
+  int64_t ngrp[3] = {0, 0, 0};
+  int nsm = 0;
+  int* d_fb = nullptr;      // queries the group kernel leaves
   int* d_counter = nullptr;
   int* d_err = nullptr;
   double* d_kernel = nullptr;
@@ -95,9 +102,12 @@ void free_arrays(nbk_batch* B) {
   dev_free(B->arr.nodex, B->st);
   dev_free(B->d_trees, B->st);
   dev_free(B->d_items, B->st);
+  dev_free(B->d_goff, B->st);
   B->arr = BuiltArrays();
   B->d_trees = nullptr;
   B->d_items = nullptr;
+  B->d_goff = nullptr;
+  B->nitems = 0;
 }
 
 void drop_graphs(nbk_batch* B) {
@@ -114,36 +124,49 @@ void batch_release(nbk_batch* B) {
     dev_free(B->d_pos_in, B->st);
     dev_free(B->d_mass_in, B->st);
   }
-  void* owned[] = {B->d_kernel, B->d_counter, B->d_err, B->d_rho_tree, B->d_rho_out};
+  void* owned[] = {B->d_kernel, B->d_counter, B->d_err, B->d_rho_tree, B->d_rho_out, B->d_fb};
   for (void* p : owned) dev_free(p, B->st);
   B->d_pos_in = B->d_mass_in = B->d_kernel = B->d_rho_tree = B->d_rho_out = nullptr;
-  B->d_counter = B->d_err = nullptr;
+  B->d_counter = B->d_err = B->d_fb = nullptr;
   if (B->st) cudaStreamSynchronize(B->st);
   if (B->own_stream && B->st) cudaStreamDestroy(B->st);
   B->st = nullptr;
   B->own_stream = false;
 }
 
-// Work items: (tree, q0, count) buckets of qb queries, largest trees first.
-int make_items(nbk_batch* B, int qb) {
-  std::vector<int> order(B->ngroups);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(),
-                   [&](int a, int c) { return B->trees[a].n > B->trees[c].n; });
+// Work items of the lane-per-query form: (tree, q0, count) buckets of qb queries, largest
+// trees first (tree: entry of d_trees).
+int make_items(nbk_batch* B) {
+  if (B->d_items) return NBK_OK;
+  const int qb = B->qb;
+  std::vector<int> order;
+  std::vector<int64_t> size;
+  for (auto& t : B->trees)
+    if (t.n > 0) {
+      order.push_back((int)order.size());
+      size.push_back(t.n);
+    }
+  std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return size[a] > size[c]; });
   std::vector<WorkItem> items;
-  items.reserve(B->ntot / qb + B->ngroups);
+  items.reserve(B->ntot / qb + order.size());
   for (int g : order)
-    for (int64_t q = 0; q < B->trees[g].n; q += qb)
-      items.push_back({g, (int)q, (int)std::min<int64_t>(qb, B->trees[g].n - q), 0});
-  dev_free(B->d_items, B->st);
+    for (int64_t q = 0; q < size[g]; q += qb)
+      items.push_back({g, (int)q, (int)std::min<int64_t>(qb, size[g] - q), 0});
   NBK_TRY(dev_malloc((void**)&B->d_items, sizeof(WorkItem) * std::max<size_t>(1, items.size()), B->st));
   NBK_CUDA_TRY(cudaMemcpyAsync(B->d_items, items.data(), sizeof(WorkItem) * items.size(),
                                cudaMemcpyHostToDevice, B->st));
   NBK_CUDA_TRY(cudaStreamSynchronize(B->st));
   B->nitems = (int)items.size();
-  B->qb = qb;
-  drop_graphs(B);
   return NBK_OK;
+}
+
+// Another query-bucket size: its items are made at the next lane-per-query search.
+void set_query_bucket(nbk_batch* B, int qb) {
+  B->qb = qb;
+  dev_free(B->d_items, B->st);
+  B->d_items = nullptr;
+  B->nitems = 0;
+  drop_graphs(B);
 }
 
 // (Re)build every tree with leaf size b.
@@ -153,13 +176,28 @@ int batch_build(nbk_batch* B, int b) {
   B->b = b;
   int64_t nb = 0;
   B->trees.resize(B->ngroups);
-  std::vector<TreeInfo> info(B->ngroups);
+  std::vector<TreeInfo> info;
+  std::vector<int> goff[3], pstart;
+  info.reserve(B->ngroups);
+  pstart.reserve(B->ngroups);
+  for (auto& v : goff) v.reserve(B->ngroups);
+  for (int64_t& c : B->ngrp) c = 0;
   for (int64_t g = 0; g < B->ngroups; g++) {
     int64_t n = B->off[g + 1] - B->off[g];
     B->trees[g] = {B->off[g], n, (int)nb};
-    info[g] = {(int)B->off[g], (int)n, (int)nb, 0};
-    nb += n > 0 ? heap_slots(n, b) : 0;
+    if (n == 0) continue;
+    info.push_back({(int)B->off[g], (int)n, (int)nb, 0});
+    pstart.push_back((int)B->off[g]);
+    for (int i = 0; i < 3; i++) {
+      // the node level of the split rule whose nodes hold at most 8, 4 or 2 particles
+      goff[i].push_back((int)B->ngrp[i]);
+      int64_t c = 1;
+      while (((n - 1) / c + 1) > (8 >> i)) c *= 2;
+      B->ngrp[i] += c;
+    }
+    nb += heap_slots(n, b);
   }
+  B->ntrees = (int)info.size();
   int64_t n = B->ntot;
   cudaStream_t st = B->st;
   NBK_TRY(dev_malloc((void**)&B->arr.pos, sizeof(P4) * std::max<int64_t>(n, 1), st));
@@ -172,13 +210,20 @@ int batch_build(nbk_batch* B, int b) {
   NBK_TRY(dev_malloc((void**)&B->d_trees, sizeof(TreeInfo) * std::max<int64_t>(B->ngroups, 1), st));
   NBK_CUDA_TRY(cudaMemcpyAsync(B->d_trees, info.data(), sizeof(TreeInfo) * info.size(),
                                cudaMemcpyHostToDevice, st));
+  std::vector<int> idx;  // [goff 8 | goff 4 | goff 2 | pstart]
+  idx.reserve(4 * info.size());
+  for (auto& v : goff) idx.insert(idx.end(), v.begin(), v.end());
+  idx.insert(idx.end(), pstart.begin(), pstart.end());
+  NBK_TRY(dev_malloc((void**)&B->d_goff, sizeof(int) * std::max<size_t>(idx.size(), 1), st));
+  NBK_CUDA_TRY(cudaMemcpyAsync(B->d_goff, idx.data(), sizeof(int) * idx.size(),
+                               cudaMemcpyHostToDevice, st));
   DevAlloc alloc;
   alloc.st = st;
   std::vector<TreeSpec> nonempty;
   for (auto& t : B->trees)
     if (t.n > 0) nonempty.push_back(t);
   NBK_TRY(build_forest(nonempty, b, B->d_pos_in, B->d_mass_in, nullptr, B->arr, alloc, st));
-  return make_items(B, B->qb);
+  return NBK_OK;  // the build has synchronised the stream: the host arrays may go
 }
 
 KnnArgs batch_args(nbk_batch* B, int k) {
@@ -191,6 +236,8 @@ KnnArgs batch_args(nbk_batch* B, int k) {
   a.kernres = B->kernres;
   a.rho = B->d_rho_tree;
   a.err = B->d_err;
+  a.nq = (int)B->ntot;
+  a.fb = B->d_fb;
   return a;
 }
 
@@ -199,7 +246,11 @@ int density_sequence(nbk_batch* B, int k, double* out) {
   NBK_CUDA_TRY(cudaMemsetAsync(B->d_rho_tree, 0, sizeof(double) * B->ntot, B->st));
   NBK_CUDA_TRY(cudaMemsetAsync(B->d_counter, 0, sizeof(int), B->st));
   KnnArgs a = batch_args(B, k);
-  BatchArgs ba{B->d_items, B->d_trees, B->nitems, B->d_counter, B->wpq};
+  if (!B->wpq) NBK_TRY(make_items(B));
+  const int i = batch_group_size(k, B->ngrp, B->nsm);
+  BatchArgs ba{B->d_items, B->d_trees, B->nitems, B->d_counter, B->wpq,
+               B->d_goff + (size_t)i * B->ntrees, B->d_goff + (size_t)3 * B->ntrees,
+               B->ntrees, (int)B->ngrp[i], 8 >> i, B->nsm};
   NBK_TRY(launch_knn_batch(a, ba, B->st));
   NBK_TRY(scatter_to_input_order(B->d_rho_tree, B->arr.perm, out, B->ntot, 1, B->st));
   return NBK_OK;
@@ -286,7 +337,7 @@ int autotune(nbk_batch* B) {
     }
     float build_ms = median3(tb[0], tb[1], tb[2]);
     for (int qb : qbs) {
-      NBK_TRY(make_items(B, qb));
+      set_query_bucket(B, qb);
       for (int wpq : wpqs) {
         B->wpq = wpq;
         NBK_TRY(density_sequence(B, 32, B->d_rho_out));  // warm
@@ -404,6 +455,12 @@ int nbk_batch_create(const double* pos, const double* mass, const int64_t* offse
                                sizeof(double) * B->h_kernel_img.size(), cudaMemcpyHostToDevice, st));
   NBK_TRY(dev_malloc((void**)&B->d_counter, sizeof(int), st));
   NBK_TRY(dev_malloc((void**)&B->d_err, sizeof(int), st));
+  NBK_TRY(dev_malloc((void**)&B->d_fb, sizeof(int) * (n + 1), st));
+  {
+    int dev = 0;
+    NBK_CUDA_TRY(cudaGetDevice(&dev));
+    NBK_CUDA_TRY(cudaDeviceGetAttribute(&B->nsm, cudaDevAttrMultiProcessorCount, dev));
+  }
   NBK_CUDA_TRY(cudaMemsetAsync(B->d_err, 0, sizeof(int), st));
   NBK_TRY(dev_malloc((void**)&B->d_rho_tree, sizeof(double) * n, st));
   NBK_TRY(dev_malloc((void**)&B->d_rho_out, sizeof(double) * n, st));
@@ -526,6 +583,7 @@ static int pertree(nbk_batch* B, int k, double* rho, bool build) {
       NBK_TRY(build_forest(one, B->b, B->d_pos_in, B->d_mass_in, nullptr, B->arr, alloc, st));
     }
     KnnArgs a = batch_args(B, std::min<int64_t>(k, ts.n - 1));
+    a.fb = nullptr;  // a warp per query: the plain method
     a.tv.n = (int)ts.n;
     a.tv.pstart = (int)ts.pstart;
     a.tv.nbase = ts.nbase;

@@ -116,38 +116,6 @@ __global__ void __launch_bounds__(32 * kWqWpb, 4) k_knn_wq(KnnArgs a) {
   wq_run<S, EPI>(a, tv, ws[warp], lane, qi, self, x0, a.kheap);
 }
 
-// Batched density, warp per query: the persistent grid's warps pull (tree, query bucket)
-// work items and serve the bucket's queries one after another.
-// 6 blocks per SM (42 registers): for the many small trees of a batch the occupancy pays
-// more than for one large tree (20,000 power-law groups: 17.98 ms against 20.59 ms at 4).
-// The batch's one-slot searches run FP32 first (knn_wq.cuh wq_search_f32: 16.2 ms)
-template <int S>
-__global__ void __launch_bounds__(32 * kWqWpb, 6) k_knn_batch_wq(KnnArgs a, BatchArgs b) {
-  __shared__ WqSmem ws[kWqWpb];
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int guard = 0; guard < b.nitems + 1; guard++) {
-    int item = 0;
-    if (lane == 0) item = atomicAdd(b.counter, 1);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= b.nitems) break;
-    WorkItem it = b.items[item];
-    TreeInfo ti = b.trees[it.tree];
-    TreeView tv = a.tv;
-    tv.n = ti.n;
-    tv.pstart = ti.pstart;
-    tv.nbase = ti.nbase;
-    int K = min(a.kheap, ti.n - 1);
-    if (K < 1) continue;
-    for (int q = 0; q < it.count; q++) {
-      int self = ti.pstart + it.q0 + q;
-      P4 p = tv.pos[self];
-      double x0[3] = {p.x, p.y, p.z};
-      wq_run<S, kEpiDensity, true>(a, tv, ws[warp], lane, self, self, x0, K);
-      __syncwarp();
-    }
-  }
-}
-
 template <int S, int EPI>
 int launch_wq(const KnnArgs& a, cudaStream_t st) {
   unsigned blocks = (unsigned)((a.nq + kWqWpb - 1) / kWqWpb);
@@ -205,41 +173,8 @@ int launch_batch_t(const KnnArgs& a, const BatchArgs& b, cudaStream_t st) {
 
 }  // namespace
 
-// Persistent warp-per-query batch kernel: every resident block of this device.
-template <int S>
-int launch_batch_wq_t(const KnnArgs& a, const BatchArgs& b, cudaStream_t st) {
-  static std::mutex mu;
-  static std::map<int, int> grids;
-  int dev = 0, grid = 0;
-  NBK_CUDA_TRY(cudaGetDevice(&dev));
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = grids.find(dev);
-    if (it != grids.end()) grid = it->second;
-  }
-  if (grid == 0) {
-    int nsm = 0, per = 0;
-    NBK_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    NBK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_knn_batch_wq<S>,
-                                                               32 * kWqWpb, 0));
-    grid = nsm * (per > 0 ? per : 1);
-    std::lock_guard<std::mutex> lk(mu);
-    grids[dev] = grid;
-  }
-  int blocks = std::min(grid, (b.nitems + kWqWpb - 1) / kWqWpb);
-  if (blocks <= 0) return NBK_OK;
-  Phase ph("knn_density_batch", st);
-  k_knn_batch_wq<S><<<blocks, 32 * kWqWpb, 0, st>>>(a, b); note_launch();
-  NBK_CUDA_TRY(cudaGetLastError());
-  return NBK_OK;
-}
-
 int launch_knn_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st) {
-  if (b.warp_per_query) {
-    if (a.kheap <= 32) return launch_batch_wq_t<1>(a, b, st);
-    if (a.kheap <= 64) return launch_batch_wq_t<2>(a, b, st);
-    if (a.kheap <= 128) return launch_batch_wq_t<4>(a, b, st);
-  }
+  if (b.warp_per_query && a.kheap <= 128) return launch_knn_group_batch(a, b, st);
   if (a.kheap <= 16) return launch_batch_t<16>(a, b, st);
   if (a.kheap <= 33) return launch_batch_t<33>(a, b, st);
   if (a.kheap <= 65) return launch_batch_t<65>(a, b, st);

@@ -53,7 +53,9 @@ constexpr int kGrpStack = 192;  // frontier stack (node indices) per warp
 constexpr int kGrpWpb = 4;      // warps (groups) per block
 constexpr int kGrpSlack = 3;    // entries beyond the K-th a buffer cut may leave
 constexpr int kGrpStrict = 256;    // a group that stages more tests nodes query by query
-constexpr int kGrpStaged = 12288;  // and one that stages more takes the second launch
+constexpr int kGrpStaged = 1024;   // and one that stages more takes the second launch (12288:
+                                   // 2^20 particles with a group that stages that many 5.4 ms, else 3.0;
+                                   // 1024: 3.3 and 3.2)
 // search radius of each pass in units of the expected K-th distance: a pass serves the
 // queries that the one before found fewer than K particles for
 constexpr int kGrpPasses = 3;
@@ -471,8 +473,12 @@ __device__ void grp_search(GrpSmem<S>& w, const TreeView& tv, int lane, int g, i
   ge.ch = tv.posf[gs + (gn >> 1)];
   ge.cl = tv.posr[gs + (gn >> 1)];
   const NodeRec home = tv.node[tv.nbase + hh];
-  const float rad = grp_radius(__fsub_ru(home.hi[0], home.lo[0]), __fsub_ru(home.hi[1], home.lo[1]),
-                               __fsub_ru(home.hi[2], home.lo[2]), hn, K);
+  // a tree that fits the buffers is taken whole
+  const float rad = tv.n <= GrpCfg<S>::cap
+                        ? 1e18f
+                        : grp_radius(__fsub_ru(home.hi[0], home.lo[0]),
+                                     __fsub_ru(home.hi[1], home.lo[1]),
+                                     __fsub_ru(home.hi[2], home.lo[2]), hn, K);
   // offsets of the queries from the group's middle particle
   float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
   L.thr = -1.f;
@@ -894,15 +900,9 @@ __global__ void __launch_bounds__(32 * kWqWpb, 4) k_knn_wq_list(KnnArgs a) {
 // image passes in the second launch for the queries whose gates could open; for the rest
 // its k + 1 list is the query itself at zero distance, then the K = k nearest others.
 template <int S, int EPI>
-__global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int depth, int K) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
+__device__ __forceinline__ void grp_serve(const KnnArgs& a, const TreeView& tv, GrpSmem<S>& w,
+                                          int lane, int g, int depth, int K) {
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  int g = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
-  if (g >= (1 << (depth - a.slices))) return;
-  g += a.slice << (depth - a.slices);
-  const TreeView& tv = a.tv;
   GrpLane L;
   int gs, gn;
   float two_e;
@@ -971,6 +971,86 @@ __global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int de
 }
 
 template <int S, int EPI>
+__global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int depth, int K) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
+  const int g = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
+  if (g >= (1 << (depth - a.slices))) return;
+  grp_serve<S, EPI>(a, a.tv, w, threadIdx.x & 31, g + (a.slice << (depth - a.slices)), depth, K);
+}
+
+// ---- batched density: every particle of every tree of a forest, k = min(k, n_tree - 1)
+
+// Last entry of the ascending v[0 .. n) that is <= x.
+__device__ __forceinline__ int last_at_most(const int* v, int n, int x) {
+  int lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (v[mid] <= x) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+template <int S>
+__global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group_batch(KnnArgs a, BatchArgs b) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
+  if (i >= b.ngroups) return;
+  const int t = last_at_most(b.goff, b.ntrees, i);
+  const TreeInfo ti = b.trees[t];
+  TreeView tv = a.tv;
+  tv.n = ti.n;
+  tv.pstart = ti.pstart;
+  tv.nbase = ti.nbase;
+  const int K = min(a.kheap, ti.n - 1), q = (ti.n - 1) / b.gmax;
+  if (K < 1) return;
+  if (tv.eps >= 1e11f) {  // squares could leave the FP32 range: everything takes the list
+    if (i == b.goff[t])
+      for (int p = lane; p < ti.n; p += 32) a.fb[1 + atomicAdd(&a.fb[0], 1)] = ti.pstart + p;
+    return;
+  }
+  grp_serve<S, kEpiDensity>(a, tv, w, lane, i - b.goff[t], 32 - __clz(q), K);
+}
+
+// The batch's queries that the group kernel left (as k_knn_wq_list), each in its own tree.
+template <int S>
+__global__ void __launch_bounds__(32 * kWqWpb, 4) k_knn_wq_list_batch(KnnArgs a, BatchArgs b) {
+  __shared__ WqSmem ws[kWqWpb];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int count = min(a.fb[0], a.nq);
+  for (int i = blockIdx.x * kWqWpb + warp; i < count; i += gridDim.x * kWqWpb) {
+    const int self = a.fb[1 + i];
+    const TreeInfo ti = b.trees[last_at_most(b.pstart, b.ntrees, self)];
+    TreeView tv = a.tv;
+    tv.n = ti.n;
+    tv.pstart = ti.pstart;
+    tv.nbase = ti.nbase;
+    P4 p = tv.pos[self];
+    double x0[3] = {p.x, p.y, p.z};
+    wq_run<S, kEpiDensity>(a, tv, ws[warp], lane, self, self, x0, min(a.kheap, ti.n - 1));
+    __syncwarp();
+  }
+}
+
+template <int S>
+int launch_group_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st) {
+  const size_t sm = sizeof(GrpSmem<S>) * kGrpWpb;
+  NBK_TRY(ensure_dyn_smem((const void*)k_knn_group_batch<S>, (int)sm));
+  NBK_CUDA_TRY(cudaMemsetAsync(a.fb, 0, sizeof(int), st));
+  if (b.ngroups == 0) return NBK_OK;
+  Phase ph("knn_density_batch", st);
+  k_knn_group_batch<S><<<(b.ngroups + kGrpWpb - 1) / kGrpWpb, 32 * kGrpWpb, sm, st>>>(a, b);
+  note_launch();
+  const unsigned lb = (unsigned)std::min<int64_t>(4 * b.nsm, ((int64_t)a.nq + kWqWpb - 1) / kWqWpb);
+  k_knn_wq_list_batch<S><<<lb, 32 * kWqWpb, 0, st>>>(a, b); note_launch();
+  NBK_CUDA_TRY(cudaGetLastError());
+  return NBK_OK;
+}
+
+template <int S, int EPI>
 int launch_group(const KnnArgs& a, int K, cudaStream_t st) {
   // groups of at most G particles, and enough of them to keep every SM's warps busy
   int nsm = 0, dev = 0;
@@ -1007,6 +1087,20 @@ int launch_group_e(const KnnArgs& a, cudaStream_t st) {
 }
 
 }  // namespace
+
+// Particles per group of a batch: the largest of 8, 4 and 2 that the buffers for k take and
+// that leaves enough groups to keep every SM's warps busy (index into the prefix arrays).
+int batch_group_size(int k, const int64_t ngroups[3], int nsm) {
+  int i = k <= 32 ? 0 : k <= 64 ? 1 : 2;
+  while (i < 2 && ngroups[i] < 16 * nsm) i++;
+  return i;
+}
+
+int launch_knn_group_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st) {
+  if (a.kheap <= 32) return launch_group_batch<1>(a, b, st);
+  if (a.kheap <= 64) return launch_group_batch<2>(a, b, st);
+  return launch_group_batch<4>(a, b, st);
+}
 
 bool group_search_serves(const KnnArgs& a) {
   const int K = a.periodic ? a.kheap - 1 : a.kheap;

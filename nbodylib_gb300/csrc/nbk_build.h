@@ -188,12 +188,17 @@ struct TreeInfo {
   int pstart, n, nbase, pad;
 };
 struct BatchArgs {
-  const WorkItem* items;
-  const TreeInfo* trees;
+  const WorkItem* items;  // lane-per-query form
+  const TreeInfo* trees;  // non-empty trees, ascending pstart
   int nitems;
-  int* counter;         // zeroed before each launch
-  int warp_per_query;   // 1: a warp serves one query at a time; 0: a lane per query
+  int* counter;           // zeroed before each launch
+  int warp_per_query;     // 1: a warp serves a group of queries; 0: a lane per query
+  const int* goff;        // group search: first group of each tree (groups of at most gmax)
+  const int* pstart;      // first particle of each tree
+  int ntrees, ngroups, gmax, nsm;
 };
+int batch_group_size(int k, const int64_t ngroups[3], int nsm);
+int launch_knn_group_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st);
 // Density of every particle of every tree (a.kheap = k, clamped per tree to n-1).
 int launch_knn_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st);
 
