@@ -886,7 +886,7 @@ int nbk_get_kernel(const nbk_tree* t, double* table, double* kernnorm) {
 // FindNearest(x) for qmode 1 (six values per point), through the reference's own walk
 // (phase.cu). A periodic target search grows the heap by one and drops its nearest entry
 // (KDFindNearest.cxx:250, 310).
-static int phase_nn(nbk_tree* t, int qmode, const int* dq, const double* dx, int64_t nq, int k,
+static int phase_nn(nbk_tree* t, Stage& S, int qmode, const int* dq, const double* dx, int64_t nq, int k,
                     int* dnn, double* dd2, bool metric) {
   PhaseArgs pa{};
   pa.k = base_args(t);
@@ -902,7 +902,7 @@ static int phase_nn(nbk_tree* t, int qmode, const int* dq, const double* dx, int
   pa.metric = metric ? 1 : 0;
   pa.spacing_periodic = t->periodic ? 1 : 0;
   pa.epi = kPhNN;
-  return launch_phase(pa, t->st);
+  return launch_phase(pa, S.alloc, t->st);
 }
 
 static int knn_variant_ok(const nbk_tree* t, int variant, const char* what) {
@@ -940,7 +940,7 @@ int nbk_knn(nbk_tree* t, int k, int variant, int periodic_mode, int32_t* nn, dou
   NBK_TRY(S.out(d2, (size_t)t->n * k, &dd2));
   NBK_TRY(clear_err(t));
   if (t->treetype == NBK_TPHS) {
-    NBK_TRY(phase_nn(t, 0, nullptr, nullptr, t->n, k, dnn, dd2,
+    NBK_TRY(phase_nn(t, S, 0, nullptr, nullptr, t->n, k, dnn, dd2,
                      t->aniso == 0 && variant != NBK_FINDNEARESTPHASE));
     NBK_TRY(S.finish());
     if (!t->dev()) NBK_TRY(check_err(t, "nbk_knn"));
@@ -992,7 +992,7 @@ int nbk_knn_targets(nbk_tree* t, const int32_t* targets, int64_t nt, int k, int 
   NBK_TRY(S.out(d2, (size_t)nt * k, &dd2));
   NBK_TRY(clear_err(t));
   if (t->treetype == NBK_TPHS) {
-    NBK_TRY(phase_nn(t, 2, dt, nullptr, nt, k, dnn, dd2,
+    NBK_TRY(phase_nn(t, S, 2, dt, nullptr, nt, k, dnn, dd2,
                      t->aniso == 0 && variant != NBK_FINDNEARESTPHASE));
     NBK_TRY(S.finish());
     if (!t->dev()) NBK_TRY(check_err(t, "nbk_knn_targets"));
@@ -1074,7 +1074,7 @@ int nbk_knn_coords(nbk_tree* t, const double* x, int64_t nq, int k, int32_t* nn,
   NBK_TRY(S.out(d2, (size_t)nq * k, &dd2));
   NBK_TRY(clear_err(t));
   if (t->treetype == NBK_TPHS) {
-    NBK_TRY(phase_nn(t, 1, nullptr, dx, nq, k, dnn, dd2, t->aniso == 0));
+    NBK_TRY(phase_nn(t, S, 1, nullptr, dx, nq, k, dnn, dd2, t->aniso == 0));
   } else {  // velocity tree (never periodic): FindNearestVel(x) over the swapped arrays
     KnnArgs a = base_args(t);
     a.kheap = k;
@@ -1112,7 +1112,7 @@ int nbk_knn_phase_points(nbk_tree* t, const double* x, int64_t nq, int k, int32_
   NBK_TRY(S.out(nn, (size_t)nq * k, &dnn));
   NBK_TRY(S.out(d2, (size_t)nq * k, &dd2));
   NBK_TRY(clear_err(t));
-  NBK_TRY(phase_nn(t, 1, nullptr, dx, nq, k, dnn, dd2, false));
+  NBK_TRY(phase_nn(t, S, 1, nullptr, dx, nq, k, dnn, dd2, false));
   NBK_TRY(S.finish());
   if (!t->dev()) NBK_TRY(check_err(t, "nbk_knn_phase_points"));
   return NBK_OK;
@@ -1121,7 +1121,7 @@ int nbk_knn_phase_points(nbk_tree* t, const double* x, int64_t nq, int k, int32_
 
 // CalcDensity / CalcDensityParticle on a phase-space tree with the local metric: qmode 0
 // scatters into `trho` (tree order), qmode 2 gathers into `out` (query order).
-static int phase_density(nbk_tree* t, int qmode, const int* dq, int64_t nq, int k, double* rho) {
+static int phase_density(nbk_tree* t, Stage& S, int qmode, const int* dq, int64_t nq, int k, double* rho) {
   if (t->aniso != 0) {
     set_error("phase-space density needs the local metric (Aniso 0); with Aniso -1 the "
               "reference multiplies uninitialised metric arrays");
@@ -1143,7 +1143,7 @@ static int phase_density(nbk_tree* t, int qmode, const int* dq, int64_t nq, int 
   pa.metric = 1;
   pa.spacing_periodic = 0;
   pa.epi = qmode == 0 ? kPhDensity : kPhDensPart;
-  return launch_phase(pa, t->st);
+  return launch_phase(pa, S.alloc, t->st);
 }
 
 static int density_common(nbk_tree* t, int k, int nsmooth, double* rho, double* vden, int epi) {
@@ -1175,7 +1175,7 @@ static int density_common(nbk_tree* t, int k, int nsmooth, double* rho, double* 
   if (vden) NBK_TRY(S.alloc.get((void**)&tv, sizeof(double) * t->n));
   NBK_TRY(clear_err(t));
   if (t->treetype == NBK_TPHS) {
-    NBK_TRY(phase_density(t, 0, nullptr, t->n, k, trho));
+    NBK_TRY(phase_density(t, S, 0, nullptr, t->n, k, trho));
     NBK_TRY(scatter_to_input_order(trho, t->arr.perm, drho, t->n, 1, t->st));
     NBK_TRY(S.finish());
     if (!t->dev()) NBK_TRY(check_err(t, "density"));
@@ -1268,7 +1268,7 @@ static int particles_common(nbk_tree* t, const int32_t* targets, int64_t nt, int
   NBK_TRY(S.out(out, nt, &dout));
   NBK_TRY(clear_err(t));
   if (t->treetype == NBK_TPHS) {
-    NBK_TRY(phase_density(t, 2, dt, nt, k, dout));
+    NBK_TRY(phase_density(t, S, 2, dt, nt, k, dout));
     NBK_TRY(S.finish());
     if (!t->dev()) NBK_TRY(check_err(t, "particle density"));
     return NBK_OK;

@@ -43,7 +43,7 @@
 // and mixed groups left to the second launch 4.6 ms.
 #include <algorithm>
 
-#include "knn_wq.cuh"
+#include "knn_select.cuh"
 
 namespace nbk {
 namespace {
@@ -51,7 +51,6 @@ namespace {
 constexpr int kGrpChunk = 64;   // candidates staged before the queries screen them
 constexpr int kGrpStack = 192;  // frontier stack (node indices) per warp
 constexpr int kGrpWpb = 4;      // warps (groups) per block
-constexpr int kGrpSlack = 3;    // entries beyond the K-th a buffer cut may leave
 constexpr int kGrpStrict = 256;    // a group that stages more tests nodes query by query
 constexpr int kGrpStaged = 1024;   // and one that stages more takes the second launch (12288:
                                    // 2^20 particles with a group that stages that many 5.4 ms, else 3.0;
@@ -60,14 +59,6 @@ constexpr int kGrpStaged = 1024;   // and one that stages more takes the second 
 // queries that the one before found fewer than K particles for
 constexpr int kGrpPasses = 3;
 __device__ __constant__ static const float kGrpRadius[kGrpPasses] = {1.25f, 2.0f, 3.0f};
-
-// S slots of 32 neighbours: K <= 32 S. Groups shrink as the buffers grow, so that a warp's
-// shared memory stays near 6 KB.
-template <int S>
-struct GrpCfg {
-  static constexpr int G = S == 1 ? 8 : (S == 2 ? 4 : 2);
-  static constexpr int cap = 64 * S;
-};
 
 template <int S>
 struct GrpSmem {
@@ -79,105 +70,6 @@ struct GrpSmem {
   float4 qs[GrpCfg<S>::G];  // the queries: offset from the centre, acceptance bound
   int stk[kGrpStack];
 };
-
-// Largest of the warp's keys (non-negative doubles' bit patterns).
-__device__ __forceinline__ long long warp_max_key(long long k) {
-  const unsigned hi = (unsigned)(k >> 32);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
-  return (long long)(((unsigned long long)mh << 32) | ml);
-}
-
-// Keep threshold for the K-th smallest FP32 squared distance s: every particle whose true
-// distance is at most the true K-th has an FP32 squared distance at or below it, and it is
-// at or above the true K-th squared distance.
-__device__ __forceinline__ float grp_thresh(float s, float two_e) {
-  float r;  // within 2^-22 of the square root, inside the 2^-20 margin
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(s));
-  const float u = __fmul_ru(r, 1.0f + 1.0f / 1048576.0f);
-  const float t = __fadd_ru(u, two_e);
-  return __fmul_ru(__fmul_ru(t, t), 1.0f + 1.0f / 1048576.0f);
-}
-
-struct GrpCut {
-  float thr;   // bound of the cut (-1: the FP32 range does not resolve the distances)
-  float smin;  // the smallest squared distance
-  int cnt;     // entries left
-};
-
-// Cut a query's buffer of cnt >= K entries back to those within the bound of its K-th
-// smallest (or of one of the `slack` next ones). Not inlined: the kernel's hot loops must
-// stay within the instruction cache (inlined everywhere, ten of eleven issue slots waited
-// for instructions).
-template <int S>
-__device__ __noinline__ GrpCut grp_tighten(unsigned* bs, int* bi, int lane, int cnt, int K,
-                                           int slack, float two_e) {
-  const unsigned FULL = 0xffffffffu;
-  constexpr int R = 2 * S;
-  GrpCut out;
-  unsigned r[R];
-  __syncwarp();
-  unsigned lo = 0xffffffffu, hi = 0u;
-#pragma unroll
-  for (int t = 0; t < R; t++) {
-    const int p = t * 32 + lane;
-    const bool in = p < cnt;
-    r[t] = in ? bs[p] : 0xffffffffu;
-    lo = min(lo, r[t]);
-    if (in) hi = max(hi, r[t]);
-  }
-  lo = __reduce_min_sync(FULL, lo);
-  hi = __reduce_max_sync(FULL, hi);
-  out.smin = __uint_as_float(lo);
-  out.cnt = cnt;
-  // invariant: at least K entries are <= hi; done as soon as K to K + slack are. The first
-  // pivot assumes counts growing as the volume, the next ones halve the interval of values
-  float pv = __uint_as_float(hi) * (0.3f + 0.7f * __fdividef((float)K, (float)cnt));
-#pragma unroll 1
-  while (lo < hi && cnt > K + slack) {
-    const unsigned mid = max(min(__float_as_uint(pv), hi - 1u), lo);
-    int c = 0;
-#pragma unroll
-    for (int t = 0; t < R; t++) c += __popc(__ballot_sync(FULL, r[t] <= mid));
-    if (c >= K) {
-      hi = mid;
-      if (c <= K + slack) break;
-    } else {
-      lo = mid + 1;
-    }
-    pv = 0.5f * (__uint_as_float(lo) + __uint_as_float(hi));
-  }
-  unsigned kth = 0u;
-#pragma unroll
-  for (int t = 0; t < R; t++)
-    if (r[t] <= hi) kth = max(kth, r[t]);
-  kth = __reduce_max_sync(FULL, kth);
-  if (kth < 0x0da24260u || kth >= 0x7e000000u) {  // below 1e-30, near overflow
-    out.thr = -1.f;
-    return out;
-  }
-  out.thr = grp_thresh(__uint_as_float(kth), two_e);
-  if (cnt == K) return out;
-  const unsigned tb = __float_as_uint(out.thr);
-  int id[R], n = 0;
-#pragma unroll
-  for (int t = 0; t < R; t++) id[t] = bi[t * 32 + lane];
-  __syncwarp();
-#pragma unroll
-  for (int t = 0; t < R; t++) {
-    const bool keep = r[t] <= tb;
-    const unsigned pm = __ballot_sync(FULL, keep);
-    if (keep) {
-      const int d = n + __popc(pm & ((1u << lane) - 1u));
-      bs[d] = r[t];
-      bi[d] = id[t];
-    }
-    n += __popc(pm);
-  }
-  __syncwarp();
-  out.cnt = n;
-  return out;
-}
 
 // The per-lane state of the group's queries (lane q < gn holds query q).
 struct GrpLane {
@@ -539,50 +431,10 @@ __device__ void grp_search(GrpSmem<S>& w, const TreeView& tv, int lane, int g, i
   }
 }
 
-// Ascending sort of the 32 S (key, index) pairs over the warp, position p = s * 32 + lane.
-template <int S>
-__device__ __forceinline__ void grp_sort(long long key[S], int idx[S], int lane) {
-  const unsigned FULL = 0xffffffffu;
-#pragma unroll
-  for (int size = 2; size <= 32 * S; size <<= 1) {
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride >= 32) {
-        const int ds = stride >> 5;
-#pragma unroll
-        for (int s = 0; s < S; s++) {
-          if (s & ds) continue;
-          const bool up = ((s * 32) & size) == 0;
-          if ((key[s] > key[s + ds]) == up) {
-            const long long k = key[s];
-            key[s] = key[s + ds];
-            key[s + ds] = k;
-            const int i = idx[s];
-            idx[s] = idx[s + ds];
-            idx[s + ds] = i;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int s = 0; s < S; s++) {
-          const long long ok = __shfl_xor_sync(FULL, key[s], stride);
-          const int oj = __shfl_xor_sync(FULL, idx[s], stride);
-          const bool up = ((s * 32 + lane) & size) == 0, lower = (lane & stride) == 0;
-          if ((lower == up) ? (ok < key[s]) : (ok > key[s])) {
-            key[s] = ok;
-            idx[s] = oj;
-          }
-        }
-      }
-    }
-  }
-}
-
 // Exact choice among the cnt > K candidates left in a query's buffer (at most 32 S + 32):
 // FP64 distances, the largest dropped until K are left, their indices back in the buffer.
 template <int S>
 __device__ __noinline__ void grp_drop(int* bi, const P4* pos, int lane, int self, int cnt, int K) {
-  const unsigned FULL = 0xffffffffu;
   const P4 x = pos[self];
   long long key[S + 1];
   int idx[S + 1];
@@ -597,33 +449,7 @@ __device__ __noinline__ void grp_drop(int* bi, const P4* pos, int lane, int self
       key[s] = dkey(dist2_exact(x.x, x.y, x.z, c.x, c.y, c.z));
     }
   }
-  for (int left = cnt; left > K; left--) {
-    long long mx = 0;
-#pragma unroll
-    for (int s = 0; s <= S; s++) mx = max(mx, key[s]);
-    mx = warp_max_key(mx);
-    int gone = 0;  // one holder of the largest leaves
-#pragma unroll
-    for (int s = 0; s <= S; s++) {
-      const unsigned b = gone ? 0u : __ballot_sync(FULL, idx[s] >= 0 && key[s] == mx);
-      if (b) {
-        gone = 1;
-        if (lane == __ffs(b) - 1) {
-          key[s] = 0;
-          idx[s] = -1;
-        }
-      }
-    }
-  }
-  int n = 0;
-  __syncwarp();
-#pragma unroll
-  for (int s = 0; s <= S; s++) {
-    const unsigned pm = __ballot_sync(FULL, idx[s] >= 0);
-    if (idx[s] >= 0) bi[n + __popc(pm & ((1u << lane) - 1u))] = idx[s];
-    n += __popc(pm);
-  }
-  __syncwarp();
+  grp_keep<S>(key, idx, bi, lane, cnt, K);
 }
 
 // The neighbours of one query: its buffer cut to the K nearest (indices in bi[0 .. K)).
@@ -643,33 +469,6 @@ __device__ int grp_select(GrpSmem<S>& w, const TreeView& tv, int lane, int q, in
   if (f.cnt == K) return 1;
   grp_drop<S>(w.bi[q], tv.pos, lane, self, f.cnt, K);
   return 2;
-}
-
-// Sums of the G rows of 32 S doubles, 32 / G lanes a row: on return the first of row q's
-// lanes holds its sum.
-template <int S>
-__device__ __forceinline__ double grp_row_sums(GrpSmem<S>& w, int lane) {
-  constexpr int lanes = 32 / GrpCfg<S>::G, per = 32 * S / lanes;
-  static_assert((per & (per - 1)) == 0, "the rotation wraps");
-  const double* row =
-      reinterpret_cast<const double*>(w.bs[lane / lanes]) + (lane % lanes) * per;
-  double acc = 0.0;
-#pragma unroll
-  for (int t = 0; t < per; t++) acc = dadd(acc, row[(t + lane) & (per - 1)]);
-#pragma unroll
-  for (int o = 1; o < lanes; o <<= 1) acc = dadd(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-  return acc;
-}
-
-// Marks in a row of squared distances: the farthest neighbour sits at q = 2 exactly in the
-// reference's arithmetic (the table's last entry); no neighbour in this place.
-constexpr double kGrpFar = -1.0, kGrpNone = -2.0;
-
-// W of one row entry: u = sqrt(d2) c1 is the table coordinate (c1 = 1 / (h delta)).
-__device__ __forceinline__ double grp_w(double d2, double c1, int kr, const double* T) {
-  const int hi = __double2hiint(d2);
-  if (hi < 0) return d2 == kGrpFar ? T[kr - 1] : 0.0;
-  return w_at_u(dmul(sqrt_newton(d2), c1), kr, T);
 }
 
 // The group's density sums (CalcDensity, KDCalcSmoothQuantities.cxx:260-286): okm marks the
@@ -731,31 +530,7 @@ __device__ void grp_density(const KnnArgs& a, const TreeView& tv, GrpSmem<S>& w,
     wm = dmul(wn, tv.pos[gs + lane].m);
   }
   __syncwarp();
-#pragma unroll 1
-  for (unsigned left = okm; left; left &= left - 1) {
-    const int q = __ffs(left) - 1;
-    const double c = __shfl_sync(FULL, c1, q), m = __shfl_sync(FULL, wm, q);
-    double* row = reinterpret_cast<double*>(w.bs[q]);
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-      const int p = s * 32 + lane;
-      double t = 0.0;
-      if (p < K) {
-        const int j = w.bi[q][p];
-        const double wq = grp_w(row[p], c, kr, T);
-        atomicAdd(&a.rho[j], dmul(wq, m));
-        t = dmul(wq, tv.pos[j].m);
-      }
-      row[p] = t;
-    }
-  }
-  __syncwarp();
-  const double acc = grp_row_sums<S>(w, lane);
-  constexpr int lanes = 32 / GrpCfg<S>::G;
-  const int q = lane / lanes;
-  const double n = __shfl_sync(FULL, wn, q);
-  if (lane % lanes == 0 && ((okm >> q) & 1u)) atomicAdd(&a.rho[gs + q], dmul(acc, n));
-  __syncwarp();
+  grp_sums<S>(w.bs, w.bi, tv.pos, a.rho + gs, a.rho, T, kr, lane, okm, K, c1, wn, wm);
 }
 
 // The group's velocity densities (CalcVelDensity, KDCalcSmoothQuantities.cxx:354-383): the
@@ -820,7 +595,7 @@ __device__ void grp_veldensity(const KnnArgs& a, const TreeView& tv, GrpSmem<S>&
     for (int s = 0; s < S; s++) row[s * 32 + lane] = grp_w(row[s * 32 + lane], c, kr, T);
   }
   __syncwarp();
-  const double acc = grp_row_sums<S>(w, lane);
+  const double acc = grp_row_sums<S>(w.bs, lane);
   constexpr int lanes = 32 / GrpCfg<S>::G;
   const int q = lane / lanes;
   const double n = __shfl_sync(FULL, wn, q);
@@ -971,12 +746,12 @@ __device__ __forceinline__ void grp_serve(const KnnArgs& a, const TreeView& tv, 
 }
 
 template <int S, int EPI>
-__global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group(KnnArgs a, int depth, int K) {
+__global__ void __launch_bounds__(32 * kGrpWpb, 7) k_knn_group(KnnArgs a, int depth, int K) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
   const int g = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
   if (g >= (1 << (depth - a.slices))) return;
-  grp_serve<S, EPI>(a, a.tv, w, threadIdx.x & 31, g + (a.slice << (depth - a.slices)), depth, K);
+  grp_serve<S, EPI>(a, a.tv, w, lane_id(), g + (a.slice << (depth - a.slices)), depth, K);
 }
 
 // ---- batched density: every particle of every tree of a forest, k = min(k, n_tree - 1)
@@ -993,10 +768,10 @@ __device__ __forceinline__ int last_at_most(const int* v, int n, int x) {
 }
 
 template <int S>
-__global__ void __launch_bounds__(32 * kGrpWpb, 8) k_knn_group_batch(KnnArgs a, BatchArgs b) {
+__global__ void __launch_bounds__(32 * kGrpWpb, 7) k_knn_group_batch(KnnArgs a, BatchArgs b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
+  const int lane = lane_id();
   const int i = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
   if (i >= b.ngroups) return;
   const int t = last_at_most(b.goff, b.ntrees, i);

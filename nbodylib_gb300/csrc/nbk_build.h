@@ -153,8 +153,13 @@ struct PhaseArgs {
   int metric;            // 1: local metric (Aniso 0), 0: plain phase distance (Aniso -1)
   int spacing_periodic;  // the metric spacing searches the images (FindNearest's copy)
   int epi;               // PhaseEpi
+  const int* count;      // device: the number of listed queries (k.qidx), null: k.nq
 };
-int launch_phase(const PhaseArgs& a, cudaStream_t st);
+int launch_phase(const PhaseArgs& pa, DevAlloc& alloc, cudaStream_t st);
+// A lane per query (phase.cu), and a warp per group of tree particles (phase_group.cu).
+int launch_phase_lanes(const PhaseArgs& pa, cudaStream_t st);
+bool phase_group_serves(const PhaseArgs& pa);
+int launch_phase_group(const PhaseArgs& pa, DevAlloc& alloc, cudaStream_t st);
 
 // ---- SPH smoothing over the nearest neighbours (smooth.cu)
 enum Smooth : int {

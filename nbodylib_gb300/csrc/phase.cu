@@ -38,7 +38,7 @@
 // screened the same way (pair_lb6f) before their FP64 distance is computed. The reference's unscaled pruning opens far more of the tree
 // than the metric needs (the whole tree, for small velocity offsets), so this bound does
 // most of the pruning while the result stays the reference's.
-#include "nbk_build.h"
+#include "phase_core.cuh"
 
 namespace nbk {
 namespace {
@@ -81,29 +81,6 @@ __device__ __forceinline__ void ph_fill(PhHeap<KMAX, NT>& H, int t, int K) {
     H.d[s][t] = kMaxValue;
     H.i[s][t] = -1;
   }
-}
-
-// PhaseDistSqd (DistFunc.h:41-49): ((((dx^2 + dy^2) + dz^2) + dvx^2) + dvy^2) + dvz^2.
-__device__ __forceinline__ double phase_d2(const double x[6], const P4& p, const V4& v) {
-  double a = dsub(x[0], p.x), b = dsub(x[1], p.y), c = dsub(x[2], p.z);
-  double e = dsub(x[3], v.x), f = dsub(x[4], v.y), g = dsub(x[5], v.z);
-  double s = dadd(dmul(a, a), dmul(b, b));
-  s = dadd(s, dmul(c, c));
-  s = dadd(s, dmul(e, e));
-  s = dadd(s, dmul(f, f));
-  return dadd(s, dmul(g, g));
-}
-// MetricDistSqd (DistFunc.h:58-65): total += (metric[i] * d) * d from 0, dimension order.
-__device__ __forceinline__ double metric_d2(const double x[6], const P4& p, const V4& v,
-                                            const double m[6]) {
-  const double y[6] = {p.x, p.y, p.z, v.x, v.y, v.z};
-  double total = 0.0;
-#pragma unroll
-  for (int k = 0; k < 6; k++) {
-    double d = dsub(x[k], y[k]);
-    total = dadd(total, dmul(dmul(m[k], d), d));
-  }
-  return total;
 }
 
 // One depth-first walk of the reference's search from x (a phase-space point). metric:
@@ -437,9 +414,11 @@ __global__ void __launch_bounds__(32 * ph_warps_per_block<KMAX>()) k_phase(Phase
   PhWarp<KMAX>& w = reinterpret_cast<PhWarp<KMAX>*>(smem)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int gw = blockIdx.x * WPB + (threadIdx.x >> 5);
-  if (gw * 32 >= a.nq) return;  // whole warps only
+  // the queries: all nq, or (second launch of the group search) the first *count of a list
+  const int nq = pa.count ? min(*pa.count, a.nq) : a.nq;
+  if (gw * 32 >= nq) return;  // whole warps only
   const int q = gw * 32 + lane;
-  bool valid = q < a.nq;
+  bool valid = q < nq;
   // the query: a tree particle (qmode 0: q0 + q; 2: qidx[q]) or a phase-space point
   int self = -1;
   double x[6] = {0, 0, 0, 0, 0, 0};
@@ -522,10 +501,11 @@ __global__ void __launch_bounds__(32 * ph_warps_per_block<KMAX>()) k_phase(Phase
         id[b - 1] = ti;
       }
     const int skip = K - a.kout;
+    const size_t row = (size_t)(pa.count ? a.qidx[q] : q) * a.kout;
     for (int s = 0; s < a.kout; s++) {
       int j = id[skip + s];
-      a.nn[(size_t)q * a.kout + s] = j >= 0 ? j - tv.pstart : -1;
-      a.d2[(size_t)q * a.kout + s] = d[skip + s];
+      a.nn[row + s] = j >= 0 ? j - tv.pstart : -1;
+      a.d2[row + s] = d[skip + s];
     }
     return;
   }
@@ -582,7 +562,7 @@ int launch_phase_t(const PhaseArgs& pa, cudaStream_t st) {
 
 }  // namespace
 
-int launch_phase(const PhaseArgs& pa, cudaStream_t st) {
+int launch_phase(const PhaseArgs& pa, DevAlloc& alloc, cudaStream_t st) {
   if (pa.k.nq <= 0) return NBK_OK;
   Phase ph(pa.epi == kPhNN ? "phase_knn" : "phase_density", st);
   int K = pa.k.kheap;
@@ -590,6 +570,12 @@ int launch_phase(const PhaseArgs& pa, cudaStream_t st) {
     set_error("phase-space search: heap size must be in [1, 128]");
     return NBK_ERR_UNSUPPORTED;
   }
+  if (phase_group_serves(pa)) return launch_phase_group(pa, alloc, st);
+  return launch_phase_lanes(pa, st);
+}
+
+int launch_phase_lanes(const PhaseArgs& pa, cudaStream_t st) {
+  const int K = pa.k.kheap;
   // heaps hold at least the 8 entries of the metric spacing
   if (K <= 16) return launch_phase_t<16>(pa, st);
   if (K <= 32) return launch_phase_t<32>(pa, st);
