@@ -103,13 +103,12 @@ __global__ void k_prelink(FofArgs a) {
 }
 
 constexpr int kStack = 64;    // depth-first stack of the criterion search (one lane)
-constexpr int kWpb = 8;
+constexpr int kWpb = 4;
 constexpr int kFStack = 512;  // frontier stack of the link search (one warp)
 constexpr int kBatchLimit = kFStack - 128;
 
 struct FofSmem {
-  float4 sf[32];
-  int par[32];  // parents of the staged leaf particles, read once per leaf
+  float4 q[32];  // the warp's query points of this pass (FP32)
   int stk[kFStack];
 };
 
@@ -155,25 +154,37 @@ __device__ __forceinline__ bool crit_cmp(int cmp, const double* p, const double 
 // overlap. Surviving inner nodes that are not compact are expanded at once; surviving
 // leaves and compact nodes are then tested against every lane's own query.
 //
+// The particles of opened leaves are tested a lane each, two leaves at a time, against one
+// query after another of those that want the leaf: with a query per lane instead, half the
+// lanes had no query that wanted the leaf. A round-to-nearest distance decides outside a
+// band of its own rounding error around the linking length (squared: `near2` and `far2`);
+// pairs inside the band take FP64.
+//
 // CRIT3D: FOFCriterion with FOF3d inside its search region, run as FOF with
 // ll^2 = params[6]; the FP32 decisions are the same (their 2^-20 margins cover the
 // rounding of the comparator's divisions) and the pairs left to FP64 take the comparator.
 template <bool CRIT3D>
-__global__ void __launch_bounds__(32 * kWpb, 4) k_link(FofArgs a) {
+__global__ void __launch_bounds__(32 * kWpb, 10) k_link(FofArgs a) {
   __shared__ FofSmem sm[kWpb];
   const unsigned FULL = 0xffffffffu;
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   FofSmem& w = sm[warp];
   const TreeView& tv = a.tv;
-  int q = (blockIdx.x * kWpb + warp) * 32 + lane;
-  if ((blockIdx.x * kWpb + warp) * 32 >= tv.n) return;
-  bool valid = q < tv.n;
+  const int q0 = (blockIdx.x * kWpb + warp) * a.qpw, q = q0 + lane;
+  if (q0 >= tv.n) return;
+  const bool valid = lane < a.qpw && q < tv.n;
   int self = tv.pstart + (valid ? q : 0);
   P4 me = tv.pos[self];
   double x0[3] = {me.x, me.y, me.z};
   float thr = thresh_hi(a.ll2), ll2_lo = thresh_lo(a.ll2);
   long long ll2k = a.ll2 > 0.0 ? dkey(a.ll2) : 0;  // no link for ll2 <= 0 or NaN
-  float eps = tv.eps, two_eps = __fmul_ru(2.f, tv.eps);
+  float eps = tv.eps;
+  // |sqrt(s) - d| <= e + 2^-21 d for the round-to-nearest s of a pair at distance d: each
+  // coordinate difference is off by at most 2 eps, sqrt(3) of it in the distance
+  const float e = __fmul_ru(tv.eps, 3.4642f);
+  const float lf = __fadd_ru(__fsqrt_ru(thr), e), ln = __fsub_rd(__fsqrt_rd(ll2_lo), e);
+  const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 524288.0f);
+  const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 524288.0f) : 0.f;
   int myroot = find_root(a.parent, self, a.err);  // cached; refreshed when it goes stale
   int npass = tv.periodic ? 8 : 1;
   int near = tv.periodic && valid ? near_walls(tv.posf[self], tv.period, eps, thr) : 0;
@@ -208,8 +219,59 @@ __global__ void __launch_bounds__(32 * kWpb, 4) k_link(FofArgs a) {
     }
     int sp = 1;
     if (lane == 0) w.stk[0] = 0;
+    w.q[lane] = make_float4(qx, qy, qz, 0.f);
     __syncwarp();
-    const int first = tv.pstart + (blockIdx.x * kWpb + warp) * 32;  // lane 0's particle
+    const int first = tv.pstart + q0;  // lane 0's particle
+    // leaves waiting for their pair tests: this lane's half holds (st, ct) wanted by `mk`
+    int st = 0, ct = 0, pend = 0;
+    unsigned mk = 0, m0 = 0, m1 = 0;
+    auto pairs = [&]() {
+      for (; __any_sync(FULL, ct > 0); st += 16, ct -= 16) {
+        const int ti = st + (lane & 15);
+        const bool ok = (lane & 15) < ct;
+        float4 cf = make_float4(0.f, 0.f, 0.f, 0.f);
+        int pj = 0;
+        if (ok) {
+          cf = tv.posf[ti];
+          pj = ld_parent(a.parent, ti);
+        }
+#pragma unroll 1
+        for (unsigned qm = m0 | m1; qm; qm &= qm - 1) {
+          const int i = __ffs(qm) - 1, sq = first + i;
+          const int rq = __shfl_sync(FULL, myroot, i);
+          // direct pass: the test is symmetric, so each pair is handled once; a parent equal
+          // to the query's root proves one component for good (links and path halving never
+          // separate a component)
+          bool in = ok && ((mk >> i) & 1u) && (pass != 0 || ti > sq) && pj != rq && ti != rq;
+          if (!__any_sync(FULL, in)) continue;
+          const float4 qf = w.q[i];
+          const float dx = cf.x - qf.x, dy = cf.y - qf.y, dz = cf.z - qf.z;
+          const float s = dx * dx + dy * dy + dz * dz;
+          in = in && !(s >= far2);  // (a NaN is left to FP64)
+          const bool band = in && !(s < near2);
+          if (__any_sync(FULL, band)) {
+            double xi[3];
+#pragma unroll
+            for (int d = 0; d < 3; d++) xi[d] = __shfl_sync(FULL, xq[d], i);
+            if (band) {
+              const P4 c = tv.pos[ti];
+              if (CRIT3D) in = crit_cmp(0, a.params, xi, make_v4(0, 0, 0, 0), c, make_v4(0, 0, 0, 0));
+              else in = dkey(dist2_exact(xi[0], xi[1], xi[2], c.x, c.y, c.z)) < ll2k;
+            }
+          }
+          if (!__any_sync(FULL, in)) continue;
+          if (in) {
+            pj = find_root(a.parent, pj, a.err);
+            if (pj != rq && pj != find_root(a.parent, rq, a.err)) unite(a.parent, sq, ti, a.err);
+          }
+          __syncwarp();
+          if (lane == i) myroot = find_root(a.parent, self, a.err);
+        }
+      }
+      pend = 0;
+      ct = 0;
+      mk = m0 = m1 = 0;
+    };
     for (int guard = 0; sp > 0 && guard < (1 << 26); guard++) {
       // above kBatchLimit entries pop one node at a time: a depth-first descent from
       // there adds at most the tree depth, so the stack never exceeds kFStack
@@ -269,46 +331,17 @@ __global__ void __launch_bounds__(32 * kWpb, 4) k_link(FofArgs a) {
           expand |= 1u << j;
           continue;
         }
-        for (int c0 = 0; c0 < rj.count; c0 += 32) {
-          int mm = min(32, rj.count - c0);
-          if (lane < mm) {
-            w.sf[lane] = tv.posf[rj.start + c0 + lane];
-            w.par[lane] = ld_parent(a.parent, rj.start + c0 + lane);
-          }
-          __syncwarp();
-          if (need) {
-            for (int jj = 0; jj < mm; jj++) {
-              int ti = rj.start + c0 + jj;
-              // direct pass: the test is symmetric, so each pair is handled once
-              if (pass == 0 && ti <= self) continue;
-              // a staged parent equal to our root proves one component for good (links
-              // and path halving never separate a component), so no root chase is needed
-              int pj = w.par[jj];
-              if (pj == myroot || ti == myroot) continue;
-              float4 cf = w.sf[jj];
-              if (pair_d2_lo(qx, qy, qz, cf.x, cf.y, cf.z, two_eps) < thr) {
-                // decided in FP32 when the upper bound is already inside; only pairs
-                // within a few FP32 ulps of the linking length take the FP64 test
-                bool in = pair_d2_hi(qx, qy, qz, cf.x, cf.y, cf.z, two_eps) < ll2_lo;
-                if (!in) {
-                  P4 c = tv.pos[ti];
-                  if (CRIT3D) in = crit_cmp(0, a.params, xq, make_v4(0, 0, 0, 0), c, make_v4(0, 0, 0, 0));
-                  else in = dkey(dist2_exact(xq[0], xq[1], xq[2], c.x, c.y, c.z)) < ll2k;
-                }
-                if (in) {
-                  int rt = find_root(a.parent, pj, a.err);
-                  if (rt != myroot) myroot = find_root(a.parent, myroot, a.err);
-                  if (rt != myroot) {
-                    unite(a.parent, self, ti, a.err);
-                    myroot = find_root(a.parent, self, a.err);
-                  }
-                }
-              }
-            }
-          }
-          __syncwarp();
+        const unsigned nm = __ballot_sync(FULL, need);
+        if (pend == 0) m0 = nm;
+        else m1 = nm;
+        if ((lane >> 4) == pend) {
+          st = rj.start;
+          ct = rj.count;
+          mk = nm;
         }
+        if (++pend == 2) pairs();
       }
+      if (pend) pairs();
       // children of the expanded nodes: lane i pushes those of its own node
       int ne = __popc(expand);
       if (sp + 2 * ne > kFStack) {
@@ -461,8 +494,7 @@ __global__ void __launch_bounds__(128) k_crit_link(FofArgs a) {
 constexpr int kCritStack = 512;  // frontier stack of the phase-space link search (one warp)
 constexpr int kCritBatchLimit = kCritStack - 128;
 struct CritSmem {
-  float4 sp[32], sv[32];
-  int par[32];
+  float4 qp[32], qv[32];  // the warp's query points of this pass (FP32)
   int stk[kCritStack];
 };
 
@@ -497,27 +529,28 @@ __device__ __forceinline__ void fof6d_weights(const double* p, float w_lo[6], fl
 // velocities where those spread more, so the search prunes in velocity too): one warp per
 // 32 particles walks it with FP32 bounds of the comparator's sum and unites the accepted
 // pairs (the reference's comparator in FP64 for pairs within a few FP32 ulps of 1); the
-// components are then carried over to the physical tree's indices.
-__global__ void __launch_bounds__(32 * kWpb) k_crit6_warp(FofArgs a) {
+// components are then carried over to the physical tree's indices. Leaves are tested as in
+// k_link: their particles a lane each, two leaves at a time, one query after another.
+__global__ void __launch_bounds__(32 * kWpb, 8) k_crit6_warp(FofArgs a) {
   __shared__ CritSmem sm[kWpb];
   const unsigned FULL = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   CritSmem& w = sm[warp];
   const TreeView& tv = a.tv;
-  const int q = (blockIdx.x * kWpb + warp) * 32 + lane;
-  if ((blockIdx.x * kWpb + warp) * 32 >= tv.n) return;
-  const bool valid = q < tv.n;
+  const int q0 = (blockIdx.x * kWpb + warp) * a.qpw, q = q0 + lane;
+  if (q0 >= tv.n) return;
+  const bool valid = lane < a.qpw && q < tv.n;
   const int self = tv.pstart + (valid ? q : 0);
   const P4 me = tv.pos[self];
   const V4 mv = tv.vel[self];
   const double x0[3] = {me.x, me.y, me.z};
   float w_lo[6], w_hi[6];
   fof6d_weights(a.params, w_lo, w_hi);
-  const float thr_hi = 1.0f + 1.0f / 1048576.0f, thr_lo = 1.0f - 1.0f / 1048576.0f;
+  const float thr_hi = 1.0f + 1.0f / 1048576.0f;
   const NodeS* N = tv.nodes6 + tv.nbase;
   const NodeF6* F = tv.nodef6 + tv.nbase;
   int myroot = find_root(a.parent, self, a.err);
-  const int first = tv.pstart + (blockIdx.x * kWpb + warp) * 32;  // lane 0's particle
+  const int first = tv.pstart + q0;  // lane 0's particle
   const int npass = (tv.periodic && N[0].split_dim >= 0) ? 8 : 1;
   for (int pass = 0; pass < npass; pass++) {
     double xq[6] = {x0[0], x0[1], x0[2], mv.x, mv.y, mv.z};
@@ -549,7 +582,72 @@ __global__ void __launch_bounds__(32 * kWpb) k_crit6_warp(FofArgs a) {
     }
     if (lane == 0) w.stk[0] = 0;
     int sp = 1;
+    w.qp[lane] = make_float4(q32[0], q32[1], q32[2], 0.f);
+    w.qv[lane] = make_float4(q32[3], q32[4], q32[5], 0.f);
+    // |sqrt(s) - t| <= e + 2^-20 t for the round-to-nearest s of a pair whose comparator sum
+    // is t^2: every coordinate difference is off by at most its eps twice (the largest of the
+    // warp's, images included)
+    float e = 0.f;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      float d = e32[k];
+      for (int o = 16; o > 0; o >>= 1) d = fmaxf(d, __shfl_xor_sync(FULL, d, o));
+      d = __fadd_ru(d, tv.eps6[k]);
+      e = __fadd_ru(e, __fmul_ru(__fmul_ru(w_hi[k], d), d));
+    }
+    e = __fsqrt_ru(e);
+    const float lf = __fadd_ru(thr_hi, e), ln = __fsub_rd(1.0f - 1.0f / 1048576.0f, e);
+    const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 262144.0f);
+    const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 262144.0f) : 0.f;
     __syncwarp();
+    int st = 0, ct = 0, pend = 0;
+    unsigned mk = 0, m0 = 0, m1 = 0;
+    auto pairs = [&]() {
+      for (; __any_sync(FULL, ct > 0); st += 16, ct -= 16) {
+        const int ti = st + (lane & 15);
+        const bool ok = (lane & 15) < ct;
+        float4 cp = make_float4(0.f, 0.f, 0.f, 0.f), cv = cp;
+        int pj = 0;
+        if (ok) {
+          cp = tv.posf[ti];
+          cv = tv.velf[ti];
+          pj = ld_parent(a.parent, ti);
+        }
+#pragma unroll 1
+        for (unsigned qm = m0 | m1; qm; qm &= qm - 1) {
+          const int i = __ffs(qm) - 1, sq = first + i;
+          const int rq = __shfl_sync(FULL, myroot, i);
+          // direct pass: each pair once
+          bool in = ok && ((mk >> i) & 1u) && ti != sq && (pass != 0 || ti > sq) && pj != rq &&
+                    ti != rq;
+          if (!__any_sync(FULL, in)) continue;
+          const float4 a4 = w.qp[i], b4 = w.qv[i];
+          const float d[6] = {cp.x - a4.x, cp.y - a4.y, cp.z - a4.z,
+                              cv.x - b4.x, cv.y - b4.y, cv.z - b4.z};
+          float s = 0.f;
+#pragma unroll
+          for (int k = 0; k < 6; k++) s = fmaf(w_lo[k] * d[k], d[k], s);
+          in = in && !(s >= far2);  // (a NaN is left to FP64)
+          const bool band = in && !(s < near2);
+          if (__any_sync(FULL, band)) {
+            double xi[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) xi[k] = __shfl_sync(FULL, xq[k], i);
+            if (band) in = crit_cmp(2, a.params, xi, tv.vel[sq], tv.pos[ti], tv.vel[ti]);
+          }
+          if (!__any_sync(FULL, in)) continue;
+          if (in) {
+            pj = find_root(a.parent, pj, a.err);
+            if (pj != rq && pj != find_root(a.parent, rq, a.err)) unite(a.parent, sq, ti, a.err);
+          }
+          __syncwarp();
+          if (lane == i) myroot = find_root(a.parent, self, a.err);
+        }
+      }
+      pend = 0;
+      ct = 0;
+      mk = m0 = m1 = 0;
+    };
     // frontier-parallel: each step pops up to 32 nodes, lane i loads node i and drops it
     // when the warp's query box cannot reach it, so the dependent node loads overlap; the
     // surviving inner nodes are expanded at once, the surviving leaves tested against
@@ -595,39 +693,17 @@ __global__ void __launch_bounds__(32 * kWpb) k_crit6_warp(FofArgs a) {
         }
         const int nstart = __shfl_sync(FULL, nd.start, jn);
         const int ncount = __shfl_sync(FULL, nd.count, jn);
-        for (int c0 = 0; c0 < ncount; c0 += 32) {
-          const int mm = min(32, ncount - c0);
-          if (lane < mm) {
-            const int i = nstart + c0 + lane;
-            w.sp[lane] = tv.posf[i];
-            w.sv[lane] = tv.velf[i];
-            w.par[lane] = ld_parent(a.parent, i);
-          }
-          __syncwarp();
-          if (need) {
-            for (int jj = 0; jj < mm; jj++) {
-              const int ti = nstart + c0 + jj;
-              if (ti == self || (pass == 0 && ti < self)) continue;  // direct pass: each pair once
-              const int pj = w.par[jj];
-              if (pj == myroot || ti == myroot) continue;
-              const float4 cp = w.sp[jj], cv = w.sv[jj];
-              const float c[6] = {cp.x, cp.y, cp.z, cv.x, cv.y, cv.z};
-              if (pair_lb6f(q32, c, w_lo, e32) >= thr_hi) continue;
-              bool in = pair_ub6f(q32, c, w_hi, e32) < thr_lo;
-              if (!in) in = crit_cmp(2, a.params, xq, mv, tv.pos[ti], tv.vel[ti]);
-              if (in) {
-                int rt = find_root(a.parent, pj, a.err);
-                if (rt != myroot) myroot = find_root(a.parent, myroot, a.err);
-                if (rt != myroot) {
-                  unite(a.parent, self, ti, a.err);
-                  myroot = find_root(a.parent, self, a.err);
-                }
-              }
-            }
-          }
-          __syncwarp();
+        const unsigned nm = __ballot_sync(FULL, need);
+        if (pend == 0) m0 = nm;
+        else m1 = nm;
+        if ((lane >> 4) == pend) {
+          st = nstart;
+          ct = ncount;
+          mk = nm;
         }
+        if (++pend == 2) pairs();
       }
+      if (pend) pairs();
       // children of the expanded nodes: lane i pushes those of its own node
       const int ne = __popc(expand);
       if (sp + 2 * ne > kCritStack) {
@@ -922,6 +998,18 @@ __global__ void k_relabel(int* group, const int* newlbl, int n) {
 
 }  // namespace
 
+// Queries per warp of the link kernels (a lane each; the other lanes still take nodes and
+// candidates): as many as 32 where that leaves enough warps for every SM.
+constexpr int kQpwMax = 32, kQpwMin = 2;
+int queries_per_warp(int64_t n, int* qpw) {
+  int dev = 0, nsm = 0;
+  NBK_CUDA_TRY(cudaGetDevice(&dev));
+  NBK_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  *qpw = kQpwMax;
+  while (*qpw > kQpwMin && n / *qpw < 16 * nsm) *qpw /= 2;
+  return NBK_OK;
+}
+
 // FOF6d inside its search region on a physical tree (see k_crit6_warp): builds the
 // phase-space tree of the same particles, links on it, and unites the physical tree's
 // parent forest accordingly.
@@ -979,7 +1067,8 @@ static int link_fof6d_phase_tree(const FofArgs& a, DevAlloc& alloc, cudaStream_t
   k_iota<<<(n + 255) / 256, 256, 0, st>>>(parent6, n);
   note_launch();
   f.parent = parent6;
-  const int warps = (n + 31) / 32;
+  NBK_TRY(queries_per_warp(n, &f.qpw));
+  const int warps = (n + f.qpw - 1) / f.qpw;
   k_crit6_warp<<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(f);
   note_launch();
   // the phase-space tree's "input" order is the physical tree's order: perm6 maps to it
@@ -1021,14 +1110,15 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
     k_prelink<<<(n + 255) / 256, 256, 0, st>>>(f); note_launch();
     k_compress<<<(n + 255) / 256, 256, 0, st>>>(a.parent, n); note_launch();
   }
-  int warps = (n + 31) / 32;
+  NBK_TRY(queries_per_warp(n, &f.qpw));
+  const int warps = (n + f.qpw - 1) / f.qpw;
   if (a.crit == 2) {
     Phase ph("fof_nn_link", st);
     k_nn_link<<<(n + 255) / 256, 256, 0, st>>>(a); note_launch();
   } else if (a.crit && a.tv.nodes6 && a.crit_contained) {
     // FOF6d inside the search region on a phase-space tree: the warp search directly
     Phase ph("fof_criterion_link", st);
-    k_crit6_warp<<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(a); note_launch();
+    k_crit6_warp<<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(f); note_launch();
   } else if (a.crit && a.tv.nodes6) {
     Phase ph("fof_criterion_link", st);
     k_crit_link6<<<(n + 127) / 128, 128, 0, st>>>(a); note_launch();
@@ -1043,7 +1133,7 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
     k_crit_link<<<(n + 127) / 128, 128, 0, st>>>(a); note_launch();
   } else {
     Phase ph("fof_link", st);
-    k_link<false><<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(a); note_launch();
+    k_link<false><<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(f); note_launch();
   }
   Phase ph_label("fof_label", st);
   NBK_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * n, st));

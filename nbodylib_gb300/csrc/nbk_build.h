@@ -224,6 +224,7 @@ struct FofArgs {
   int crit_contained;  // crit 1: every pair the comparator accepts lies inside the search
                        //   region (FOF3d / FOF6d with params[6] <= the position search
                        //   distance^2), so reachability follows from the comparator
+  int qpw;             // queries per warp of the link kernels (set by run_fof)
 };
 int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tree,
             int* h_ngroup, DevAlloc& alloc, cudaStream_t st,
