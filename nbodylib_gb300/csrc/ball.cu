@@ -2,21 +2,30 @@
 // node recursions, src/KDTree/KDFindNearest.cxx:567-706, KDSplitNode.cxx:455-686,
 // 1341-1456, KDLeafNode.cxx:247-410).
 //
-// One warp serves 32 queries and walks the tree once for all of them, like the kNN
-// kernel. Results are returned as CSR: a counting pass, an exclusive scan, a filling
-// pass. Pair decisions are the reference's FP64 test d2 < fdist2 (strict); the whole-node
-// shortcut of the reference marks exactly the particles this test accepts (every member
-// of a node whose farthest corner is inside the radius passes it, because rounding is
-// monotone), so it changes only whether the target itself is reported, which
+// One warp serves up to 32 queries and walks the tree once for them. Results are returned as
+// CSR: a counting pass, an exclusive scan, a filling pass; a row lists its particles in tree
+// order, image by image. Pair decisions are the reference's FP64 test d2 < fdist2 (strict);
+// the whole-node shortcut of the reference marks exactly the particles this test accepts
+// (every member of a node whose farthest corner is inside the radius passes it, because
+// rounding is monotone), so it changes only whether the target itself is reported, which
 // nbk_ball_mark reproduces from the exact node boxes.
+//
+// What bounds it: instruction issue. A lane per query tested every particle of an opened leaf
+// for the whole warp, with two directed-rounding bounds, one node at a time (2.45 ms for 2^20
+// balls of 32 in a uniform box, half the lanes idle). Now up to 32 nodes are taken at once
+// (in tree order: the leaves ahead of the first inner node are tested, what follows is pushed
+// back), leaf particles are tested a lane each, two leaves at a time, one query after another
+// of those that want the leaf, and one round-to-nearest distance decides outside a band of
+// its own rounding error around the radius.
 #include "nbk_build.h"
 
 namespace nbk {
 
 namespace {
 
-constexpr int kStack = 64;
-constexpr int kWpb = 8;
+constexpr int kStack = 512;  // node stack of one warp
+constexpr int kBatch = kStack - 128;
+constexpr int kWpb = 4;
 
 struct BallArgs {
   TreeView tv;
@@ -24,6 +33,7 @@ struct BallArgs {
   const int* qidx;
   const double* qx;
   int nq;
+  int qpw;    // queries per warp
   double r2;
   int exclude_self;
   int* counts;
@@ -34,22 +44,22 @@ struct BallArgs {
 };
 
 struct BallSmem {
-  float4 sf[32];
-  P4 sp[32];
+  float4 q[32];  // the warp's query points of this pass (FP32)
   int stk[kStack];
 };
 
 template <bool FILL>
-__global__ void __launch_bounds__(32 * kWpb) k_ball(BallArgs a) {
+__global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
   __shared__ BallSmem sm[kWpb];
   const unsigned FULL = 0xffffffffu;
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int lane;  // read once
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  const int warp = threadIdx.x >> 5;
   BallSmem& w = sm[warp];
   const TreeView& tv = a.tv;
-  int gw = blockIdx.x * kWpb + warp;
-  if (gw * 32 >= a.nq) return;
-  int q = gw * 32 + lane;
-  bool valid = q < a.nq;
+  const int q0 = (blockIdx.x * kWpb + warp) * a.qpw, q = q0 + lane;
+  if (q0 >= a.nq) return;
+  const bool valid = lane < a.qpw && q < a.nq;
   int self = -1;
   double x0[3] = {0, 0, 0};
   if (valid) {
@@ -65,14 +75,22 @@ __global__ void __launch_bounds__(32 * kWpb) k_ball(BallArgs a) {
       x0[2] = a.qx[3 * (size_t)q + 2];
     }
   }
-  int64_t base = (FILL && valid) ? a.offsets[q] : 0;
+  const int64_t base = (FILL && valid) ? a.offsets[q] : 0;
+  const int room = (FILL && valid) ? (int)(a.offsets[q + 1] - base) : 0;
   int cnt = 0;
-  float thr = thresh_hi(a.r2), r2_lo = thresh_lo(a.r2);
-  long long r2k = a.r2 > 0.0 ? dkey(a.r2) : 0;  // nothing is inside r2 <= 0 or NaN
+  const float thr = thresh_hi(a.r2), r2_lo = thresh_lo(a.r2);
+  const long long r2k = a.r2 > 0.0 ? dkey(a.r2) : 0;  // nothing is inside r2 <= 0 or NaN
   // the query's own rounding bound, images included (it may lie outside the tree's box)
-  float eps = valid ? query_eps(tv, x0[0], x0[1], x0[2]) : tv.eps;
-  float two_eps = __fadd_ru(eps, tv.eps);
-  int npass = tv.periodic ? 8 : 1;
+  const float eps = valid ? query_eps(tv, x0[0], x0[1], x0[2]) : tv.eps;
+  // |sqrt(s) - d| <= e + 2^-21 d for the round-to-nearest s of a pair at distance d (the
+  // coordinate differences are off by eps + tv.eps each; the warp's largest)
+  float e = eps;
+  for (int o = 16; o > 0; o >>= 1) e = fmaxf(e, __shfl_xor_sync(FULL, e, o));
+  e = __fmul_ru(__fadd_ru(e, tv.eps), 1.7321f);
+  const float lf = __fadd_ru(__fsqrt_ru(thr), e), ln = __fsub_rd(__fsqrt_rd(r2_lo), e);
+  const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 524288.0f);
+  const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 524288.0f) : 0.f;
+  const int npass = tv.periodic ? 8 : 1;
   int near = 0;
   if (tv.periodic && valid)
     near = near_walls(make_float4(__double2float_rn(x0[0]), __double2float_rn(x0[1]),
@@ -82,87 +100,175 @@ __global__ void __launch_bounds__(32 * kWpb) k_ball(BallArgs a) {
     double xq[3] = {x0[0], x0[1], x0[2]};
     bool active = valid;
     if (pass > 0) {
-      bool may = (kImageMask[pass] & ~near) == 0;
-      if (!__any_sync(0xffffffffu, may)) continue;
-      double sval = reflect(x0, xq, tv.period, kImageMask[pass]);
-      active = active && may && (a.r2 > dmul(sval, sval));  // KDSplitNode.cxx:1356-1373
+      const bool may = valid && (kImageMask[pass] & ~near) == 0;
+      if (!__any_sync(FULL, may)) continue;
+      const double sval = reflect(x0, xq, tv.period, kImageMask[pass]);
+      active = may && (a.r2 > dmul(sval, sval));  // KDSplitNode.cxx:1356-1373
     }
     if (!__any_sync(FULL, active)) continue;
-    float qx = __double2float_rn(xq[0]), qy = __double2float_rn(xq[1]),
-          qz = __double2float_rn(xq[2]);
-    int sp = 1;
-    if (lane == 0) w.stk[0] = 0;
+    const float qx = __double2float_rn(xq[0]), qy = __double2float_rn(xq[1]),
+                qz = __double2float_rn(xq[2]);
+    // box around the active lanes' query points, widened by their rounding
+    float qlo[3], qhi[3];
+    {
+      const float v[3] = {qx, qy, qz};
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        float lo = active ? __fsub_rd(v[d], eps) : FLT_MAX;
+        float hi = active ? __fadd_ru(v[d], eps) : -FLT_MAX;
+        for (int o = 16; o > 0; o >>= 1) {
+          lo = fminf(lo, __shfl_xor_sync(FULL, lo, o));
+          hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, o));
+        }
+        qlo[d] = lo;
+        qhi[d] = hi;
+      }
+    }
     __syncwarp();
+    w.q[lane] = make_float4(qx, qy, qz, 0.f);
+    if (lane == 0) w.stk[0] = 0;
+    int sp = 1;
+    __syncwarp();
+#pragma unroll 1
     while (sp > 0) {
-      int h = w.stk[sp - 1];
-      sp--;
+      // the next nodes in tree order, the first on lane 0; above kBatch entries one at a time
+      // (a depth-first descent from there adds at most the tree depth). A node that has been
+      // tested is stored as its complement.
+      const int m = sp <= kBatch ? min(32, sp) : 1;
+      int h = -1;
+      NodeRec r{};
+      bool keep = false;
+      if (lane < m) {
+        h = w.stk[sp - 1 - lane];
+        keep = h < 0;
+        h = h < 0 ? ~h : h;
+        r = tv.node[tv.nbase + h];
+        if (!keep) {
+          const float gx = fmaxf(0.f, fmaxf(__fsub_rd(r.lo[0], qhi[0]), __fsub_rd(qlo[0], r.hi[0])));
+          const float gy = fmaxf(0.f, fmaxf(__fsub_rd(r.lo[1], qhi[1]), __fsub_rd(qlo[1], r.hi[1])));
+          const float gz = fmaxf(0.f, fmaxf(__fsub_rd(r.lo[2], qhi[2]), __fsub_rd(qlo[2], r.hi[2])));
+          keep = __fadd_rd(__fadd_rd(__fmul_rd(gx, gx), __fmul_rd(gy, gy)), __fmul_rd(gz, gz)) < thr;
+        }
+      }
       __syncwarp();
-      NodeRec r = tv.node[tv.nbase + h];
-      bool need = active && box_d2_lo(qx, qy, qz, eps, r) < thr;
-      if (!__any_sync(FULL, need)) continue;
-      if (r.count <= tv.b) {
-        for (int c0 = 0; c0 < r.count; c0 += 32) {
-          int m = min(32, r.count - c0);
-          if (lane < m) {
-            w.sf[lane] = tv.posf[r.start + c0 + lane];
-            w.sp[lane] = tv.pos[r.start + c0 + lane];
+      sp -= m;
+      const bool leaf = r.count <= tv.b;
+      const unsigned km = __ballot_sync(FULL, keep), im = __ballot_sync(FULL, keep && !leaf);
+      const unsigned ahead = im ? (im & (0u - im)) - 1u : 0xffffffffu;  // lanes before it
+      // what follows the first inner node goes back, its children in its place
+      const unsigned back = km & ~ahead, two = back & im;
+      const int up = 31 - lane;  // lanes after this one
+      const int slot = sp + (up ? __popc(back >> (lane + 1)) + __popc(two >> (lane + 1)) : 0);
+      const int total = __popc(back) + __popc(two);
+      if (sp + total > kStack) {
+        if (lane == 0) atomicExch(a.err, kErrCapacity);
+        return;
+      }
+      if ((back >> lane) & 1u) {
+        if (leaf) {
+          w.stk[slot] = ~h;
+        } else {
+          w.stk[slot] = 2 * h + 2;
+          w.stk[slot + 1] = 2 * h + 1;
+        }
+      }
+      sp += total;
+      // the leaves ahead, two at a time
+      unsigned lm = km & ahead;
+#pragma unroll 1
+      while (lm) {
+        int st = 0, ct = 0;
+        unsigned mk = 0, any = 0;
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+          if (!lm) break;
+          const int j = __ffs(lm) - 1;
+          NodeRec rj;
+#pragma unroll
+          for (int d = 0; d < 3; d++) {
+            rj.lo[d] = __shfl_sync(FULL, r.lo[d], j);
+            rj.hi[d] = __shfl_sync(FULL, r.hi[d], j);
           }
-          __syncwarp();
-          if (need) {
-            for (int j = 0; j < m; j++) {
-              int ti = r.start + c0 + j;
-              if (a.exclude_self && pass == 0 && ti == self) continue;
-              float4 cf = w.sf[j];
-              if (pair_d2_lo(qx, qy, qz, cf.x, cf.y, cf.z, two_eps) < thr) {
-                // FP32 upper bound inside the ball decides without FP64 unless the
-                // distance itself is wanted
-                double d2 = 0.0;
-                bool in = !(FILL && a.outd2) &&
-                          pair_d2_hi(qx, qy, qz, cf.x, cf.y, cf.z, two_eps) < r2_lo;
-                if (!in) {
-                  P4 c = w.sp[j];
-                  d2 = dist2_exact(xq[0], xq[1], xq[2], c.x, c.y, c.z);
-                  in = dkey(d2) < r2k;  // d2 < r2
-                }
-                if (in) {
-                  if (FILL) {
-                    if (base + cnt < a.offsets[q + 1]) {
-                      a.out[base + cnt] = ti;
-                      if (a.outd2) a.outd2[base + cnt] = d2;
-                    } else {
-                      atomicExch(a.err, kErrCapacity);  // fill disagrees with count
-                    }
-                  }
-                  cnt++;
+          const int cj = __shfl_sync(FULL, r.count, j), sj = __shfl_sync(FULL, r.start, j);
+          if (half == 1 && (cj > 16 || __any_sync(FULL, ct > 16))) break;  // a row stays in order
+          lm &= lm - 1;
+          const unsigned nm =
+              __ballot_sync(FULL, active && box_d2_lo(qx, qy, qz, eps, rj) < thr);
+          if ((lane >> 4) == half) {
+            st = sj;
+            ct = cj;
+            mk = nm;
+          }
+          any |= nm;
+        }
+        if (!any) continue;
+        const bool big = __any_sync(FULL, ct > 16);  // one leaf alone, 32 particles a step
+        if (big) {
+          st = __shfl_sync(FULL, st, 0);
+          ct = __shfl_sync(FULL, ct, 0);
+          mk = any;
+        }
+        const int step = big ? 32 : 16, off = big ? lane : (lane & 15);
+#pragma unroll 1
+        for (; __any_sync(FULL, ct > 0); st += step, ct -= step) {
+          const int ti = st + off;
+          const bool ok = off < ct;
+          float4 cf = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (ok) cf = tv.posf[ti];
+#pragma unroll 1
+          for (unsigned qm = any; qm; qm &= qm - 1) {
+            const int i = __ffs(qm) - 1;
+            const float4 qf = w.q[i];
+            const float dx = cf.x - qf.x, dy = cf.y - qf.y, dz = cf.z - qf.z;
+            const float s = dx * dx + dy * dy + dz * dz;
+            bool in = ok && ((mk >> i) & 1u) && !(s >= far2);
+            const int si = __shfl_sync(FULL, self, i);
+            if (a.exclude_self && pass == 0) in = in && ti != si;
+            const bool band = in && (!(s < near2) || (FILL && a.outd2));
+            double d2 = 0.0;
+            if (__any_sync(FULL, band)) {
+              double xi[3];
+#pragma unroll
+              for (int d = 0; d < 3; d++) xi[d] = __shfl_sync(FULL, xq[d], i);
+              if (band) {
+                const P4 c = tv.pos[ti];
+                d2 = dist2_exact(xi[0], xi[1], xi[2], c.x, c.y, c.z);
+                in = dkey(d2) < r2k;  // d2 < r2
+              }
+            }
+            const unsigned hit = __ballot_sync(FULL, in);
+            if (FILL && hit) {
+              const int64_t bi = __shfl_sync(FULL, base, i);
+              const int c = __shfl_sync(FULL, cnt, i) + __popc(hit & ((1u << lane) - 1u));
+              const int lim = __shfl_sync(FULL, room, i);
+              if (in) {
+                if (c < lim) {
+                  a.out[bi + c] = ti;
+                  if (a.outd2) a.outd2[bi + c] = d2;
+                } else {
+                  atomicExch(a.err, kErrCapacity);  // fill disagrees with count
                 }
               }
             }
+            if (lane == i) cnt += __popc(hit);
           }
-          __syncwarp();
         }
-      } else {
-        int hl = 2 * h + 1, hr = 2 * h + 2;
-        NodeRec rl = tv.node[tv.nbase + hl], rr = tv.node[tv.nbase + hr];
-        bool nl = need && box_d2_lo(qx, qy, qz, eps, rl) < thr;
-        bool nr = need && box_d2_lo(qx, qy, qz, eps, rr) < thr;
-        bool anyl = __any_sync(FULL, nl), anyr = __any_sync(FULL, nr);
-        if (sp + 2 > kStack) {
-          if (lane == 0) atomicExch(a.err, kErrCapacity);
-          return;
-        }
-        if (anyr) {
-          if (lane == 0) w.stk[sp] = hr;
-          sp++;
-        }
-        if (anyl) {
-          if (lane == 0) w.stk[sp] = hl;
-          sp++;
-        }
-        __syncwarp();
       }
+      __syncwarp();
     }
   }
   if (!FILL && valid) a.counts[q] = cnt;
+}
+
+// Queries per warp: 32 where that leaves enough warps for every SM (a lane each; the other
+// lanes still take nodes and particles).
+int ball_qpw(int64_t nq, int* qpw) {
+  int dev = 0, nsm = 0;
+  NBK_CUDA_TRY(cudaGetDevice(&dev));
+  NBK_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  *qpw = 32;
+  while (*qpw > 1 && nq / *qpw < 16 * nsm) *qpw /= 2;
+  return NBK_OK;
 }
 
 __global__ void k_scan64_blocks(const int* in, int64_t* out, int64_t* bsum, int n) {
@@ -287,8 +393,9 @@ int run_ball(const TreeView& tv, int qmode, const int* qidx, const double* qx, i
   a.exclude_self = exclude_self;
   a.counts = counts;
   a.err = err;
-  int warps = (nq + 31) / 32;
-  int blocks = (warps + kWpb - 1) / kWpb;
+  NBK_TRY(ball_qpw(nq, &a.qpw));
+  const int64_t warps = ((int64_t)nq + a.qpw - 1) / a.qpw;
+  const unsigned blocks = (unsigned)((warps + kWpb - 1) / kWpb);
   Phase ph("ball", st);
   k_ball<false><<<blocks, 32 * kWpb, 0, st>>>(a); note_launch();
   k_scan64_blocks<<<nb, 1024, 0, st>>>(counts, d_offsets, bsum, nq); note_launch();
@@ -335,6 +442,7 @@ int run_ball_mark(const TreeView& tv, int target, double fdist2, int imark, int*
   a.qmode = 0;
   a.qidx = d_t;
   a.nq = 1;
+  a.qpw = 1;
   a.r2 = fdist2;
   a.exclude_self = target_search;
   int* counts;
