@@ -12,15 +12,16 @@
 //   dL/dx_i += [sum_j c_ij dw/dh] (1/2) (x_i - x_K)/r_iK   (and the opposite on x_K).
 // The backward kernel recomputes every weight from the saved neighbour lists (4 B per
 // neighbour) instead of storing weights; one thread per particle, FP64 atomics for the
-// contributions that land on other particles. The quotients that do not depend on the
-// pair (g_i = w_i / rho_i, the table slopes (T[c+1]-T[c])/delta, 1/h, h^-3) are formed
-// once; a pair takes 1/r from an FP32 reciprocal square root and two FP64 Newton steps
-// (no division, no FP64 square root). Each pair's table cell is the forward pass's
-// (int)(r / h * 0.5 * (kernres - 1)): from the fast r / h, and from the correctly rounded
-// square root and division whenever the fast value lies within 1e-10 of a cell edge (its
-// own error is below 1e-12 there), so the frozen cells are exactly the forward's.
-// The forward (the warp-per-query kNN) writes each neighbour row ascending in distance,
-// so the row's last entry is the farthest neighbour, the one that set h_i.
+// contributions that land on other particles. What bounds it is the FP64 pipe: 30
+// instructions a pair (46 before the terms were rearranged: 3.45 ms at 2^20, k = 32). In the
+// table coordinate u = q (kernres - 1) / 2 the line of a cell is T = A + D u and q T' = D u,
+// factors of the particle alone (h^-3, h^-4, dL/drho_i) are taken out of the sums, the cell
+// comes from the bits of u, and r and 1/r from one FP32 reciprocal square root (corrected in
+// FP32 for r, by a cubic step for 1/r). Each pair's table cell is the forward pass's
+// (int)(r / h * 0.5 * (kernres - 1)): from the fast u, and from the correctly rounded square
+// root and division whenever u lies within 2^-30 of a cell edge (its own error is below
+// 2^-40 there), so the frozen cells are exactly the forward's.
+// Each saved row ends with the farthest neighbour, the one that set h_i.
 #include <algorithm>
 
 #include "nbk_build.h"
@@ -29,108 +30,115 @@ namespace nbk {
 
 namespace {
 
-// 1 / sqrt(x) to about 2e-16 relative: the FP32 reciprocal square root and two Newton
-// steps y (3/2 - x/2 y^2) in FP64; outside the FP32 normal range the FP64 path.
-__device__ __forceinline__ double rsqrt_newton(double x) {
-  const float xf = __double2float_rn(x);
-  if (!(xf > 1e-30f && xf < 1e30f)) return 1.0 / __dsqrt_rn(x);
-  double y = (double)rsqrtf(xf);
-  const double hx = 0.5 * x;
-  y = y * __fma_rn(-hx, y * y, 1.5);
-  y = y * __fma_rn(-hx, y * y, 1.5);
-  return y;
-}
-
-// g_i = w_i / rho_i in place of w_i (tree order), and the slope of every table cell
-// (0 for the last entry, whose cell the forward pass never interpolates).
-__global__ void k_adjoint_prep(double* wg, const double* __restrict__ rho, int64_t n,
-                               const double* __restrict__ T, int kr, double* slope) {
+// g_i = w_i / rho_i in place of w_i (tree order).
+__global__ void k_adjoint_prep(double* wg, const double* __restrict__ rho, int64_t n) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) wg[i] = wg[i] / rho[i];
-  if (i < kr) {
-    double delta = 2.0 / (double)(kr - 1);
-    slope[i] = i < kr - 1 ? (T[i + 1] - T[i]) / delta : 0.0;
+}
+
+// r = sqrt(x) and 1 / r, both to about an ulp (0 < x inside FP32's range; see sqrt_newton).
+__device__ __forceinline__ double root_pair(double x, double* inv) {
+  const double r = sqrt_newton(x);
+  const int hi = __double2hiint(x);
+  if ((unsigned)(hi - ((1023 - 70) << 20)) > (unsigned)(170 << 20)) {
+    *inv = 1.0 / r;
+    return r;
   }
+  float yf;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(yf) : "f"(f32_of_bits(hi, __double2loint(x))));
+  const double y = f64_of_f32(yf), e = __fma_rn(-r, y, 1.0);
+  *inv = __fma_rn(y, __fma_rn(e, e, e), y);
+  return r;
 }
 
 __global__ void __launch_bounds__(128) k_adjoint(TreeView tv, int K, const int* __restrict__ nn,
                                                  const double* __restrict__ g,
-                                                 const double* __restrict__ T,
-                                                 const double* __restrict__ slope, int kr,
+                                                 const double* __restrict__ T, int kr,
                                                  double* gpos, double* gmass) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= tv.n) return;
   int ti = tv.pstart + i;
   const int* row = nn + (size_t)i * K;
   P4 xi = tv.pos[ti];
-  double gi = g[ti];
+  const double gi = g[ti], mi = xi.m;
   // farthest neighbour: the one that set h_i in the forward pass (the row's last entry)
   const int kf = row[K - 1];
   P4 xk = tv.pos[kf];
   const double best = dist2_exact(xi.x, xi.y, xi.z, xk.x, xk.y, xk.z);
-  const double hh = 0.5 * __dsqrt_rn(best);  // the forward's h_i, for the cell edge cases
-  const double irk = rsqrt_newton(best);      // 1 / r_iK
+  double irk;                                // 1 / r_iK
+  const double hh = 0.5 * root_pair(best, &irk);  // the forward's h_i
   const double ih = 2.0 * irk;                // 1 / h_i
   const double norm = ih * ih * ih;
-  const double delta = 2.0 / (double)(kr - 1);
-  const double hk = 0.5 * (double)(kr - 1);
+  const double hk = 0.5 * (double)(kr - 1), c1 = ih * hk;
   const double nh = -0.5 * norm * ih;  // dw/dh = nh (3 T + q T'), dw/dr = -nh T'
-  double A = 0.0, gmi = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+  const double pr = -nh * hk;          // dw/dr = pr D
+  const double gn = 0.5 * gi * norm;
+  const double* A = T + kr;
+  const double* D = T + 3 * (size_t)kr;
+  double acc = 0.0, gmi = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
   for (int s = 0; s < K; s++) {
-    int j = row[s];
-    P4 xj = tv.pos[j];
-    double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    double d2 = dist2_exact(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z);
-    double ir = rsqrt_newton(d2);  // 1 / r_ij (the target search excluded r = 0)
-    double q = d2 * ir * ih;
-    double u = q * hk;
-    int c = (int)u;
-    double fr = u - (double)c;
-    if (fr < 1e-10 || fr > 1.0 - 1e-10) c = (int)(__dsqrt_rn(d2) / hh * 0.5 * (double)(kr - 1));
-    double Tp = slope[c < kr - 1 ? c : kr - 1];
-    double Tq = c < kr - 1 ? __fma_rn(Tp, q - delta * (double)c, T[c]) : T[kr - 1];
-    double w = 0.5 * Tq * norm;
-    double gj = g[j];
-    double cij = gi * xj.m + gj * xi.m;
-    atomicAdd(&gmass[j], gi * w);
-    gmi += gj * w;
-    double dwdr = -nh * Tp;
-    double dwdh = nh * (3.0 * Tq + q * Tp);
-    A += cij * dwdh;
-    double coef = cij * dwdr * ir;
-    gx += coef * dx;
-    gy += coef * dy;
-    gz += coef * dz;
-    atomicAdd(&gpos[3 * (size_t)j + 0], -coef * dx);
-    atomicAdd(&gpos[3 * (size_t)j + 1], -coef * dy);
-    atomicAdd(&gpos[3 * (size_t)j + 2], -coef * dz);
+    const int j = row[s];
+    const P4 xj = tv.pos[j];
+    const double dx = dsub(xi.x, xj.x), dy = dsub(xi.y, xj.y), dz = dsub(xi.z, xj.z);
+    const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dmul(dx, dx)));
+    double ir;  // 1 / r_ij (the target search excluded r = 0)
+    const double u = dmul(root_pair(d2, &ir), c1);
+    // the cell (int)u and the fraction of u in units of 2^-32, from its bits; the farthest
+    // neighbour (the row's last) is at u = kernres - 1 exactly
+    const int e = (__double2hiint(u) >> 20) - 1023;
+    const unsigned long long m =
+        ((unsigned long long)__double_as_longlong(u) << 11) | 0x8000000000000000ull;
+    int c = e < 0 ? 0 : (int)(m >> (63 - min(e, 31)));
+    const unsigned fr =
+        (unsigned)((e < 0 ? m >> min(-1 - e, 63) : m << min(e + 1, 63)) >> 32);
+    if (s == K - 1) {
+      c = kr - 1;
+    } else if (fr + 4u < 8u) {
+      const double de = dist2_exact(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z);
+      c = (int)(dsqrt_call(de) / hh * 0.5 * (double)(kr - 1));
+    }
+    c = c < kr - 1 ? c : kr - 1;
+    const double Dc = D[c];                    // 0 for the last entry
+    const double t = dmul(Dc, u);              // q T'
+    const double Tq = c < kr - 1 ? dadd(A[c], t) : T[kr - 1];
+    const double gj = g[j];
+    const double cij = __fma_rn(gj, mi, dmul(gi, xj.m));
+    atomicAdd(&gmass[j], dmul(gn, Tq));
+    gmi = __fma_rn(gj, Tq, gmi);
+    acc = __fma_rn(cij, __fma_rn(3.0, Tq, t), acc);
+    const double c0 = dmul(dmul(cij, ir), Dc);
+    gx = __fma_rn(c0, dx, gx);
+    gy = __fma_rn(c0, dy, gy);
+    gz = __fma_rn(c0, dz, gz);
+    const double cs = -dmul(c0, pr);
+    atomicAdd(&gpos[3 * (size_t)j + 0], dmul(cs, dx));
+    atomicAdd(&gpos[3 * (size_t)j + 1], dmul(cs, dy));
+    atomicAdd(&gpos[3 * (size_t)j + 2], dmul(cs, dz));
   }
-  double ch = A * 0.5 * irk;
+  const double ch = acc * nh * 0.5 * irk;
   double kx = ch * (xi.x - xk.x), ky = ch * (xi.y - xk.y), kz = ch * (xi.z - xk.z);
   atomicAdd(&gpos[3 * (size_t)kf + 0], -kx);
   atomicAdd(&gpos[3 * (size_t)kf + 1], -ky);
   atomicAdd(&gpos[3 * (size_t)kf + 2], -kz);
-  atomicAdd(&gpos[3 * (size_t)ti + 0], gx + kx);
-  atomicAdd(&gpos[3 * (size_t)ti + 1], gy + ky);
-  atomicAdd(&gpos[3 * (size_t)ti + 2], gz + kz);
-  atomicAdd(&gmass[ti], gmi);
+  atomicAdd(&gpos[3 * (size_t)ti + 0], __fma_rn(pr, gx, kx));
+  atomicAdd(&gpos[3 * (size_t)ti + 1], __fma_rn(pr, gy, ky));
+  atomicAdd(&gpos[3 * (size_t)ti + 2], __fma_rn(pr, gz, kz));
+  atomicAdd(&gmass[ti], gmi * 0.5 * norm);
 }
 
 }  // namespace
 
 int run_density_adjoint(const TreeView& tv, int k, const int* d_nn, double* d_w_tree,
                         const double* d_rho_tree, const double* kernel, int kernres,
-                        double* d_slope, double* d_gpos_tree, double* d_gmass_tree,
-                        cudaStream_t st) {
+                        double* d_gpos_tree, double* d_gmass_tree, cudaStream_t st) {
   if (tv.n == 0) return NBK_OK;
   NBK_CUDA_TRY(cudaMemsetAsync(d_gpos_tree, 0, sizeof(double) * 3 * tv.n, st));
   NBK_CUDA_TRY(cudaMemsetAsync(d_gmass_tree, 0, sizeof(double) * tv.n, st));
   Phase ph("adjoint_backward", st);
-  int64_t m = std::max<int64_t>(tv.n, kernres);
-  k_adjoint_prep<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(d_w_tree, d_rho_tree, tv.n, kernel,
-                                                               kernres, d_slope);
+  k_adjoint_prep<<<(unsigned)(((int64_t)tv.n + 255) / 256), 256, 0, st>>>(d_w_tree, d_rho_tree,
+                                                                          tv.n);
   note_launch();
-  k_adjoint<<<(tv.n + 127) / 128, 128, 0, st>>>(tv, k, d_nn, d_w_tree, kernel, d_slope, kernres,
+  k_adjoint<<<(tv.n + 127) / 128, 128, 0, st>>>(tv, k, d_nn, d_w_tree, kernel, kernres,
                                                 d_gpos_tree, d_gmass_tree);
   note_launch();
   NBK_CUDA_TRY(cudaGetLastError());
