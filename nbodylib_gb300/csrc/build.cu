@@ -150,6 +150,7 @@ __device__ __forceinline__ T sel(const T* a, int dim) {
 template <int ND>
 __global__ void k_init_soa(const double* __restrict__ pos_in, const double* __restrict__ vel_in,
                            double* C, int64_t cs, int* ID, int64_t n, int* err) {
+  chain_wait();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   bool bad = false;
@@ -181,6 +182,7 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 template <int ND>
 __global__ void __launch_bounds__(kThreads) k_bbox(const Chunk* __restrict__ chunks,
                                                    GNodeT<ND>* g, const double* C, int64_t cs) {
+  chain_wait();
   Chunk c = chunks[blockIdx.x];
   unsigned long long mn[ND], mx[ND];
 #pragma unroll
@@ -268,6 +270,7 @@ __global__ void __launch_bounds__(kThreads) k_radix(const Chunk* __restrict__ ch
   unsigned* h = reinterpret_cast<unsigned*>(sk);
   __shared__ unsigned wsum[32], tot;
   __shared__ int s_last;
+  chain_wait();
   Chunk c = chunks[blockIdx.x];
   const GNodeT<ND> s = g[c.g];
   if (s.mask == ~0ull) return;  // the median key of this node is already known
@@ -560,6 +563,7 @@ __global__ void __launch_bounds__(kThreads) k_count_scan(const Chunk* __restrict
                                                          unsigned* cnt_eq, unsigned* base_less,
                                                          unsigned* base_eq, NodeOut<ND> out) {
   __shared__ int s_last;
+  chain_wait();
   count_body<ND>((int)blockIdx.x, chunks, g, Cb, cs, cnt_less, cnt_eq);
   const int node = chunks[blockIdx.x].g;
   __threadfence();
@@ -592,6 +596,7 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const Chunk* __restrict__ 
   constexpr int kWarps = kThreads / 32, kPerWarp = kChunk / kWarps;
   __shared__ unsigned wl[kWarps], we[kWarps], wv[kWarps];
   __shared__ unsigned long long bb[kWarps][4 * ND];
+  chain_wait();
   Chunk c = chunks[blockIdx.x];
   const GNodeT<ND>& s = g[c.g];
   const unsigned long long piv = s.prefix;
@@ -798,6 +803,7 @@ __global__ void __launch_bounds__(kMidThreads) k_mid_build(
   MNode<ND>* nxt = cur + kMidNodes;
   __shared__ unsigned wsum[kMidGroups][32], tot[kMidGroups];
   __shared__ int n_cur, n_next, s_k[kMidGroups], s_ncand[kMidGroups];
+  chain_wait();
   __shared__ unsigned s_fill[kMidGroups];
   __shared__ unsigned long long s_prefix[kMidGroups];
   // per group: left min, left max, right min, right max
@@ -1187,6 +1193,7 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_build(
   constexpr int K = L::K;
   constexpr int NL = L::kLists;
 
+  chain_wait();
   const LRoot R = roots[blockIdx.x];
   const int S = R.size;
   const double* C = R.buf ? Cb : Ca;
@@ -1787,33 +1794,28 @@ static int build_forest_t(const std::vector<TreeSpec>& trees, int b, const doubl
     int* I2 = L.buf ? IDa : IDb;
     // boxes of the first level's nodes; every later level gets them from the scatter above
     if (li == 0) {
-      k_bbox<ND><<<nc, kThreads, 0, st>>>(d_c, d_g, C, cs); note_launch();
+      NBK_CUDA_TRY(launch_chain(k_bbox<ND>, nc, kThreads, 0, st, d_c, d_g, C, cs));
     }
     for (int pass = 0; pass < kPasses; pass++) {
-      k_radix<ND><<<nc, kThreads, 0, st>>>(d_c, d_g, C, cs, d_hist, d_cand, pass, nout, (int)p0,
-                                           d_err); note_launch();
+      NBK_CUDA_TRY(launch_chain(k_radix<ND>, nc, kThreads, 0, st, d_c, d_g, C, cs, d_hist, d_cand,
+                                pass, nout, (int)p0, d_err));
     }
-    k_count_scan<ND><<<nc, kThreads, 0, st>>>(d_c, d_g, C, cs, cl, ce, bl, be, nout);
-    note_launch();
-    k_scatter<ND><<<nc, kThreads, 0, st>>>(d_c, d_g, C, I, C2, I2, cs, bl, be, d_err, d_gnext);
-    note_launch();
-    NBK_CUDA_TRY(cudaGetLastError());
+    NBK_CUDA_TRY(launch_chain(k_count_scan<ND>, nc, kThreads, 0, st, d_c, d_g, C, cs, cl, ce, bl,
+                              be, nout));
+    NBK_CUDA_TRY(launch_chain(k_scatter<ND>, nc, kThreads, 0, st, d_c, d_g, C, I, C2, I2, cs, bl,
+                              be, d_err, d_gnext));
   }
   if (nmroots > 0) {
     size_t sm = MidLayout<ND>::total;
     NBK_TRY(ensure_dyn_smem((const void*)k_mid_build<ND>, (int)sm));
-    k_mid_build<ND><<<(unsigned)nmroots, kMidThreads, sm, st>>>(d_m, Ca, IDa, Cb, IDb, cs, nout,
-                                                                d_err, (int)p0);
-    note_launch();
-    NBK_CUDA_TRY(cudaGetLastError());
+    NBK_CUDA_TRY(launch_chain(k_mid_build<ND>, (unsigned)nmroots, kMidThreads, sm, st, d_m, Ca, IDa,
+                              Cb, IDb, cs, nout, d_err, (int)p0));
   }
   if (nroots > 0) {
     size_t sm = LocalLayout<ND>::total;
     NBK_TRY(ensure_dyn_smem((const void*)k_local_build<ND>, (int)sm));
-    k_local_build<ND><<<(unsigned)nroots, kLocalThreads, sm, st>>>(
-        d_r, Ca, IDa, Cb, IDb, cs, d_mass_in, d_vel_in, b, nout, pout, d_err, (int)p0);
-    note_launch();
-    NBK_CUDA_TRY(cudaGetLastError());
+    NBK_CUDA_TRY(launch_chain(k_local_build<ND>, (unsigned)nroots, kLocalThreads, sm, st, d_r, Ca,
+                              IDa, Cb, IDb, cs, d_mass_in, d_vel_in, b, nout, pout, d_err, (int)p0));
   }
   if (root_out && root_src)
     NBK_CUDA_TRY(cudaMemcpyAsync(root_out, root_src, root_bytes, cudaMemcpyDeviceToHost, st));

@@ -145,6 +145,7 @@ __global__ void k_gather_d(const double* in, const int* perm, double* out, int64
   out[i] = in[perm[i]];
 }
 __global__ void k_scatter_i(const int* tv, const int* perm, int* out, int64_t n) {
+  chain_wait();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   out[perm[i]] = tv[i];
@@ -1698,8 +1699,8 @@ int nbk_fof(nbk_tree* t, double fdist, int32_t minnum, int order, int32_t* group
   NBK_TRY(run_fof(a, (int)t->nslots, minnum, order, gtree, ps ? &ps->i[0] : &ng, S.alloc, t->st,
                   ps != nullptr));
   if (t->n > 0) {
-    k_scatter_i<<<(unsigned)((t->n + 255) / 256), 256, 0, t->st>>>(gtree, t->arr.perm, dg, t->n); note_launch();
-    NBK_CUDA_TRY(cudaGetLastError());
+    NBK_CUDA_TRY(launch_chain(k_scatter_i, (unsigned)((t->n + 255) / 256), 256, 0, t->st, gtree,
+                              t->arr.perm, dg, t->n));
   }
   NBK_TRY(S.finish());
   if (ps) {

@@ -77,13 +77,18 @@ __device__ __forceinline__ bool node_compact(const NodeRec& r, float ll2_lo) {
   return d < ll2_lo;
 }
 
-__global__ void k_iota(int* p, int n) {
+// Every particle its own root; the members counted later start at zero.
+__global__ void k_start(int* p, int* cnt, int n) {
+  chain_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = i;
+  if (i >= n) return;
+  p[i] = i;
+  if (cnt) cnt[i] = 0;
 }
 
 // 1. unite each particle with the first particle of its highest compact ancestor
 __global__ void k_prelink(FofArgs a) {
+  chain_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   const TreeView& tv = a.tv;
   if (t >= tv.n) return;
@@ -166,6 +171,7 @@ __device__ __forceinline__ bool crit_cmp(int cmp, const double* p, const double 
 template <bool CRIT3D>
 __global__ void __launch_bounds__(32 * kWpb, 10) k_link(FofArgs a) {
   __shared__ FofSmem sm[kWpb];
+  chain_wait();
   const unsigned FULL = 0xffffffffu;
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   FofSmem& w = sm[warp];
@@ -533,6 +539,7 @@ __device__ __forceinline__ void fof6d_weights(const double* p, float w_lo[6], fl
 // k_link: their particles a lane each, two leaves at a time, one query after another.
 __global__ void __launch_bounds__(32 * kWpb, 8) k_crit6_warp(FofArgs a) {
   __shared__ CritSmem sm[kWpb];
+  chain_wait();
   const unsigned FULL = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   CritSmem& w = sm[warp];
@@ -869,6 +876,7 @@ __global__ void __launch_bounds__(128) k_crit_link6(FofArgs a) {
 
 // Point every particle straight at its root (between phases: no unions in flight).
 __global__ void k_compress(int* parent, int n) {
+  chain_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int x = i;
@@ -881,6 +889,7 @@ __global__ void k_compress(int* parent, int n) {
 }
 
 __global__ void k_flatten_count(int* parent, int n, int* cnt, int* err) {
+  chain_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool valid = i < n;
   int x = valid ? i : -1;
@@ -899,47 +908,52 @@ __global__ void k_flatten_count(int* parent, int n, int* cnt, int* err) {
   if (valid && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&cnt[x], __popc(peers));
 }
 
-__global__ void k_valid(const int* parent, const int* cnt, int n, int minnum, int* flag) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  flag[i] = (parent[i] == i && cnt[i] >= minnum) ? 1 : 0;
-}
-
-// exclusive scan (three-phase, 1024 per block)
-__global__ void k_scan_blocks(const int* in, int* out, int* bsum, int n) {
-  __shared__ int s[1024];
-  int i = blockIdx.x * 1024 + threadIdx.x;
-  int v = i < n ? in[i] : 0;
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    int t = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
-    __syncthreads();
-    s[threadIdx.x] += t;
-    __syncthreads();
+// Exclusive scan over a block of 1024 threads (wsum: 32 words): the thread's prefix; *tot the
+// block's sum.
+__device__ __forceinline__ int scan1024(int v, int* wsum, int* tot) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int x = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += t;
   }
-  if (i < n) out[i] = s[threadIdx.x] - v;
-  if (threadIdx.x == 1023) bsum[blockIdx.x] = s[1023];
-}
-__global__ void k_scan_sums(int* bsum, int nb, int* total) {
-  __shared__ int run;
-  if (threadIdx.x == 0) run = 0;
+  if (lane == 31) wsum[w] = x;
   __syncthreads();
-  for (int c0 = 0; c0 < nb; c0 += 1024) {
-    __shared__ int s[1024];
-    int i = c0 + threadIdx.x;
-    int v = i < nb ? bsum[i] : 0;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      int t = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
-      __syncthreads();
-      s[threadIdx.x] += t;
-      __syncthreads();
+  if (w == 0) {
+    const int y = wsum[lane];
+    int z = y;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, z, o);
+      if (lane >= o) z += t;
     }
-    if (i < nb) bsum[i] = run + s[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == 1023) run += s[1023];
+    wsum[lane] = z - y;
+    if (lane == 31) *tot = z;
+  }
+  __syncthreads();
+  return x - v + wsum[w];
+}
+// The roots of components with at least minnum members, numbered in increasing order: their
+// exclusive scan in two steps, per 1024 particles (lbl, bsum) and over the blocks' sums.
+__global__ void __launch_bounds__(1024) k_number(const int* parent, const int* cnt, int n,
+                                                 int minnum, int* flag, int* lbl, int* bsum) {
+  __shared__ int wsum[32], tot;
+  chain_wait();
+  const int i = blockIdx.x * 1024 + threadIdx.x;
+  const int v = i < n && parent[i] == i && cnt[i] >= minnum ? 1 : 0;
+  if (flag && i < n) flag[i] = v;
+  const int x = scan1024(v, wsum, &tot);
+  if (i < n) lbl[i] = x;
+  if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
+}
+__global__ void __launch_bounds__(1024) k_scan_sums(int* bsum, int nb, int* total) {
+  __shared__ int wsum[32], tot;
+  chain_wait();
+  int run = 0;
+  for (int c0 = 0; c0 < nb; c0 += 1024) {
+    const int i = c0 + threadIdx.x;
+    const int x = scan1024(i < nb ? bsum[i] : 0, wsum, &tot);
+    if (i < nb) bsum[i] = run + x;
+    run += tot;
     __syncthreads();
   }
   if (threadIdx.x == 0) *total = run;
@@ -949,11 +963,13 @@ __global__ void k_scan_add(int* out, const int* bsum, int n) {
   if (i < n) out[i] += bsum[blockIdx.x];
 }
 
-__global__ void k_label(const int* parent, const int* flag, const int* lbl, int n, int* group) {
+__global__ void k_label(const int* parent, const int* cnt, const int* lbl, const int* bsum, int n,
+                        int minnum, int* group) {
+  chain_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int r = parent[i];
-  group[i] = flag[r] ? lbl[r] + 1 : 0;
+  group[i] = cnt[r] >= minnum ? lbl[r] + bsum[r >> 10] + 1 : 0;
 }
 
 // order = 1: sort keys (size descending, then label) with a bitonic network in global
@@ -1064,13 +1080,11 @@ static int link_fof6d_phase_tree(const FofArgs& a, DevAlloc& alloc, cudaStream_t
   v.eps = a.tv.eps;
   int* parent6;
   NBK_TRY(alloc.get((void**)&parent6, sizeof(int) * (size_t)n));
-  k_iota<<<(n + 255) / 256, 256, 0, st>>>(parent6, n);
-  note_launch();
+  NBK_CUDA_TRY(launch_chain(k_start, (n + 255) / 256, 256, 0, st, parent6, nullptr, n));
   f.parent = parent6;
   NBK_TRY(queries_per_warp(n, &f.qpw));
   const int warps = (n + f.qpw - 1) / f.qpw;
-  k_crit6_warp<<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(f);
-  note_launch();
+  NBK_CUDA_TRY(launch_chain(k_crit6_warp, (warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st, f));
   // the phase-space tree's "input" order is the physical tree's order: perm6 maps to it
   k_carry_roots<<<(n + 255) / 256, 256, 0, st>>>(parent6, A6.perm, a.parent + a.tv.pstart, n,
                                                  a.err);
@@ -1099,7 +1113,7 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
                                    {(void**)&bsum, sizeof(int) * (nb + 1)},
                                    {(void**)&d_total, sizeof(int)}},
                                st, alloc));
-  k_iota<<<(n + 255) / 256, 256, 0, st>>>(a.parent, n); note_launch();
+  NBK_CUDA_TRY(launch_chain(k_start, (n + 255) / 256, 256, 0, st, a.parent, cnt, n));
   // FOFCriterion with FOF3d inside its search region links exactly the pairs with
   // sum dx^2 / params[6] < 1: the FOF kernels with ll^2 = params[6]
   const bool fof3d = a.crit == 1 && a.crit_contained && a.cmp == 0 && !a.tv.nodes6;
@@ -1107,8 +1121,8 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
   if (fof3d) f.ll2 = a.params[6];
   if (!a.crit || fof3d) {
     Phase ph("fof_prelink", st);
-    k_prelink<<<(n + 255) / 256, 256, 0, st>>>(f); note_launch();
-    k_compress<<<(n + 255) / 256, 256, 0, st>>>(a.parent, n); note_launch();
+    NBK_CUDA_TRY(launch_chain(k_prelink, (n + 255) / 256, 256, 0, st, f));
+    NBK_CUDA_TRY(launch_chain(k_compress, (n + 255) / 256, 256, 0, st, a.parent, n));
   }
   NBK_TRY(queries_per_warp(n, &f.qpw));
   const int warps = (n + f.qpw - 1) / f.qpw;
@@ -1118,13 +1132,13 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
   } else if (a.crit && a.tv.nodes6 && a.crit_contained) {
     // FOF6d inside the search region on a phase-space tree: the warp search directly
     Phase ph("fof_criterion_link", st);
-    k_crit6_warp<<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(f); note_launch();
+    NBK_CUDA_TRY(launch_chain(k_crit6_warp, (warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st, f));
   } else if (a.crit && a.tv.nodes6) {
     Phase ph("fof_criterion_link", st);
     k_crit_link6<<<(n + 127) / 128, 128, 0, st>>>(a); note_launch();
   } else if (fof3d) {
     Phase ph("fof_criterion_link", st);
-    k_link<true><<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(f); note_launch();
+    NBK_CUDA_TRY(launch_chain(k_link<true>, (warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st, f));
   } else if (a.crit && a.crit_contained && a.cmp == 2) {
     Phase ph("fof_criterion_link", st);
     NBK_TRY(link_fof6d_phase_tree(a, alloc, st));
@@ -1133,16 +1147,15 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
     k_crit_link<<<(n + 127) / 128, 128, 0, st>>>(a); note_launch();
   } else {
     Phase ph("fof_link", st);
-    k_link<false><<<(warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st>>>(f); note_launch();
+    NBK_CUDA_TRY(launch_chain(k_link<false>, (warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st, f));
   }
   Phase ph_label("fof_label", st);
-  NBK_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * n, st));
-  k_flatten_count<<<(n + 255) / 256, 256, 0, st>>>(a.parent, n, cnt, a.err); note_launch();
-  k_valid<<<(n + 255) / 256, 256, 0, st>>>(a.parent, cnt, n, minnum, flag); note_launch();
-  k_scan_blocks<<<nb, 1024, 0, st>>>(flag, lbl, bsum, n); note_launch();
-  k_scan_sums<<<1, 1024, 0, st>>>(bsum, nb, d_total); note_launch();
-  k_scan_add<<<nb, 1024, 0, st>>>(lbl, bsum, n); note_launch();
-  k_label<<<(n + 255) / 256, 256, 0, st>>>(a.parent, flag, lbl, n, d_group_tree); note_launch();
+  NBK_CUDA_TRY(launch_chain(k_flatten_count, (n + 255) / 256, 256, 0, st, a.parent, n, cnt, a.err));
+  NBK_CUDA_TRY(launch_chain(k_number, nb, 1024, 0, st, a.parent, cnt, n, minnum,
+                            order ? flag : nullptr, lbl, bsum));
+  NBK_CUDA_TRY(launch_chain(k_scan_sums, 1, 1024, 0, st, bsum, nb, d_total));
+  NBK_CUDA_TRY(launch_chain(k_label, (n + 255) / 256, 256, 0, st, a.parent, cnt, lbl, bsum, n,
+                            minnum, d_group_tree));
   NBK_CUDA_TRY(cudaGetLastError());
   if (defer_count && !order) {
     // the caller's page-locked h_ngroup is read after the caller's own synchronisation
@@ -1161,6 +1174,7 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
     int* newlbl;
     NBK_TRY(alloc.get((void**)&keys, sizeof(unsigned long long) * P));
     NBK_TRY(alloc.get((void**)&newlbl, sizeof(int) * total));
+    k_scan_add<<<nb, 1024, 0, st>>>(lbl, bsum, n); note_launch();
     k_order_keys<<<(n + 255) / 256, 256, 0, st>>>(a.parent, flag, lbl, cnt, n, keys); note_launch();
     if (P > total) k_pad<<<(P - total + 255) / 256, 256, 0, st>>>(keys, total, P); note_launch();
     for (int kk = 2; kk <= P; kk <<= 1)

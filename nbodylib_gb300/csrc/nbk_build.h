@@ -16,6 +16,24 @@
 
 namespace nbk {
 
+// Launch of a kernel that begins with chain_wait (nbk_internal.cuh).
+template <typename... P, typename... A>
+cudaError_t launch_chain(void (*k)(P...), unsigned grid, unsigned block, size_t smem,
+                         cudaStream_t st, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  note_launch();
+  return cudaLaunchKernelEx(&c, k, P(args)...);
+}
+
 constexpr int kLocalMax = 1024;  // subtrees up to this size finish in one CTA
 
 // One tree of a forest: particles [pstart, pstart+n) in both input and tree order, nodes
