@@ -24,7 +24,7 @@
 // A query that this cannot answer exactly -- fewer than K particles within the radius, a
 // candidate not provably at a non-zero distance (the target search skips zero distances,
 // KDLeafNode.cxx:19-21), more candidates than the buffer holds within the rounding of the
-// K-th, distances outside the FP32 range, a periodic query whose image gates could open --
+// K-th, distances outside the FP32 range, a periodic query too close to an image gate --
 // and every query of a group whose box meets too many particles is appended to a list that
 // a second launch serves with the warp-per-query search.
 //
@@ -180,10 +180,10 @@ __device__ __forceinline__ bool grp_near(const GrpGeom& ge, float lx, float ly, 
 }
 
 // Append the particle ti (one per lane, valid lanes only) to the staged candidates when it
-// is within reach of the group's box.
+// is within reach of the group's box. Its index carries the image pass (tag) it was found in.
 template <int S>
 __device__ __forceinline__ void grp_stage(GrpSmem<S>& w, const TreeView& tv, const GrpGeom& ge,
-                                          int lane, bool valid, int ti, int& chn) {
+                                          int lane, bool valid, int ti, int tag, int& chn) {
   float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
   bool in = false;
   if (valid) {
@@ -195,7 +195,7 @@ __device__ __forceinline__ void grp_stage(GrpSmem<S>& w, const TreeView& tv, con
     const float4 r = tv.posr[ti];
     w.ch[chn + __popc(pm & ((1u << lane) - 1u))] =
         make_float4((c.x - ge.ch.x) + (r.x - ge.cl.x), (c.y - ge.ch.y) + (r.y - ge.cl.y),
-                    (c.z - ge.ch.z) + (r.z - ge.cl.z), __int_as_float(ti));
+                    (c.z - ge.ch.z) + (r.z - ge.cl.z), __int_as_float(ti | tag));
   }
   chn += __popc(pm);
 }
@@ -260,7 +260,7 @@ __device__ __forceinline__ float grp_radius(float ex, float ey, float ez, int n,
 // nodes a step. Returns false when the queries have to take the second launch.
 template <int S>
 __device__ bool grp_walk(GrpSmem<S>& w, const TreeView& tv, GrpGeom& ge, GrpLane& L, int lane,
-                         int gs, int hh, int lev, int K, float two_e) {
+                         int gs, int hh, int lev, int tag, int K, float two_e) {
   const unsigned FULL = 0xffffffffu;
   const unsigned act = __ballot_sync(FULL, L.act);
   int chn = 0, nst = 0, sp = 0, m = lev + 1, h = hh;
@@ -299,7 +299,7 @@ __device__ bool grp_walk(GrpSmem<S>& w, const TreeView& tv, GrpGeom& ge, GrpLane
         ct = __shfl_sync(FULL, r.count, src & 31);
         if (src < 0) ct = 0;
       }
-      grp_stage<S>(w, tv, ge, lane, (lane & 15) < ct, st + (lane & 15), chn);
+      grp_stage<S>(w, tv, ge, lane, (lane & 15) < ct, st + (lane & 15), tag, chn);
       st += 16;
       ct -= 16;
       continue;
@@ -333,6 +333,29 @@ __device__ bool grp_walk(GrpSmem<S>& w, const TreeView& tv, GrpGeom& ge, GrpLane
     __syncwarp();
   }
   return false;
+}
+
+// The box around the active lanes' points, widened by e2.
+template <int S>
+__device__ __forceinline__ void grp_box(GrpGeom& ge, bool act, float4 p, float e2) {
+  const unsigned FULL = 0xffffffffu;
+  float lo[3], hi[3];
+  lo[0] = act ? __fsub_rd(p.x, e2) : FLT_MAX;
+  lo[1] = act ? __fsub_rd(p.y, e2) : FLT_MAX;
+  lo[2] = act ? __fsub_rd(p.z, e2) : FLT_MAX;
+  hi[0] = act ? __fadd_ru(p.x, e2) : -FLT_MAX;
+  hi[1] = act ? __fadd_ru(p.y, e2) : -FLT_MAX;
+  hi[2] = act ? __fadd_ru(p.z, e2) : -FLT_MAX;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+#pragma unroll
+    for (int o = GrpCfg<S>::G / 2; o > 0; o >>= 1) {
+      lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
+      hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
+    }
+    ge.qlo[d] = __shfl_sync(FULL, lo[d], 0);
+    ge.qhi[d] = __shfl_sync(FULL, hi[d], 0);
+  }
 }
 
 // One group: on return lane q < gn holds the state of query gs + q and its buffer holds
@@ -396,26 +419,7 @@ __device__ void grp_search(GrpSmem<S>& w, const TreeView& tv, int lane, int g, i
     L.act = lane < gn && L.cnt < K;
     if (!__any_sync(FULL, L.act)) break;
     const float r = kGrpRadius[pass] * rad;
-    float lo[3], hi[3];
-    lo[0] = L.act ? __fsub_rd(mine.x, e2) : FLT_MAX;
-    lo[1] = L.act ? __fsub_rd(mine.y, e2) : FLT_MAX;
-    lo[2] = L.act ? __fsub_rd(mine.z, e2) : FLT_MAX;
-    hi[0] = L.act ? __fadd_ru(mine.x, e2) : -FLT_MAX;
-    hi[1] = L.act ? __fadd_ru(mine.y, e2) : -FLT_MAX;
-    hi[2] = L.act ? __fadd_ru(mine.z, e2) : -FLT_MAX;
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
-        hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      ge.qlo[d] = __shfl_sync(FULL, lo[d], 0);
-      ge.qhi[d] = __shfl_sync(FULL, hi[d], 0);
-    }
+    grp_box<S>(ge, L.act, mine, e2);
     ge.reach = grp_thresh(r * r, two_e);
     if (L.act) {
       L.cnt = 0;
@@ -423,7 +427,7 @@ __device__ void grp_search(GrpSmem<S>& w, const TreeView& tv, int lane, int g, i
       w.qs[lane] = make_float4(L.x, L.y, L.z, L.thr);
     }
     __syncwarp();
-    if (!grp_walk<S>(w, tv, ge, L, lane, gs, hh, lev, K, two_e)) {
+    if (!grp_walk<S>(w, tv, ge, L, lane, gs, hh, lev, 0, K, two_e)) {
       if (L.act) L.thr = -1.f;
       break;
     }
@@ -671,9 +675,178 @@ __global__ void __launch_bounds__(32 * kWqWpb, 4) k_knn_wq_list(KnnArgs a) {
   }
 }
 
-// K: neighbours other than the query itself. A periodic search (FindNearest) takes the
-// image passes in the second launch for the queries whose gates could open; for the rest
-// its k + 1 list is the query itself at zero distance, then the K = k nearest others.
+// Queries of `mask` left to the second launch.
+__device__ __forceinline__ void grp_leave(int* fb, int lane, int gs, unsigned mask) {
+  if (!mask) return;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(&fb[0], __popc(mask));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if ((mask >> lane) & 1u) fb[1 + base + __popc(mask & ((1u << lane) - 1u))] = gs + lane;
+}
+
+constexpr int kGrpImage = 28;  // an index's bits from here on: the image pass it was found in
+
+// FindNearest on a periodic tree: the direct pass's K nearest, then the image passes in the
+// reference's order with its gates (KDSplitNode.cxx:1126-1147), each for the queries of the
+// group whose gate it opens. A gate compares the exact K-th distance with a wall distance; the
+// bounds of the selection decide unless they straddle it (that query takes the second launch).
+// The images of the queries are searched with offsets from one of them as the centre.
+template <int S>
+__device__ void grp_periodic(const KnnArgs& a, GrpSmem<S>& w, int lane, int g, int depth, int K) {
+  const unsigned FULL = 0xffffffffu;
+  const TreeView& tv = a.tv;
+  GrpLane L;
+  int gs, gn;
+  float two_e;
+  grp_search<S>(w, tv, lane, g, depth, K, L, gs, gn, two_e);
+  // cut every buffer to the K nearest; `okm`: the queries answered here
+  unsigned okm = 0u;
+  auto cut = [&](unsigned which, bool direct) {
+#pragma unroll 1
+    for (unsigned left = which; left; left &= left - 1) {
+      const int q = __ffs(left) - 1;
+      const float thr = __shfl_sync(FULL, L.thr, q);
+      const int cnt = __shfl_sync(FULL, L.cnt, q);
+      okm &= ~(1u << q);
+      if (thr < 0.f || cnt < K) continue;
+      const GrpCut f = grp_tighten<S>(w.bs[q], w.bi[q], lane, cnt, K, 0, two_e);
+      const float zero2 = __fmul_ru(__fmul_ru(two_e, two_e), 1.01f);
+      if (f.thr < 0.f || f.cnt > 32 * S + 32 || (direct && (f.thr > thr || f.smin <= zero2)))
+        continue;
+      okm |= 1u << q;
+      if (lane == q) {
+        L.cnt = f.cnt;
+        L.thr = fminf(thr, f.thr);
+      }
+    }
+  };
+  cut((1u << gn) - 1u, true);
+  const bool mine = (okm >> lane) & 1u;
+  double x0[3] = {0, 0, 0};
+  int near_sq = 0, near_lin = 0;
+  if (mine) {
+    const P4 p = tv.pos[gs + lane];
+    x0[0] = p.x;
+    x0[1] = p.y;
+    x0[2] = p.z;
+    const float4 qf = tv.posf[gs + lane];
+    const float qeps = __fmul_ru(2.f, tv.eps);
+    near_sq = near_walls(qf, tv.period, qeps, L.thr);
+    near_lin = near_walls_lin(qf, tv.period, qeps, L.thr);
+  }
+#pragma unroll 1
+  for (int pass = 1; pass < 8; pass++) {
+    const int mk = kImageMask[pass];
+    const bool lin = !(pass <= 3 || a.min_image);
+    bool open = ((okm >> lane) & 1u) && (mk & ~(lin ? near_lin : near_sq)) == 0;
+    if (!__any_sync(FULL, open)) continue;
+    double xp[3];
+    const float sv = __double2float_rn(reflect(x0, xp, tv.period, mk));
+    // the K-th distance is between lo and hi
+    const float hi = __fsqrt_ru(L.thr);
+    const float lo = fmaxf(0.f, hi * (1.0f - 1.0f / 65536.0f) - 2.f * two_e);
+    const float t1 = lin ? lo * lo : lo, t2 = lin ? L.thr : hi;
+    const float m = fabsf(sv) * 1e-6f;
+    const bool surely = t1 > sv + m, never = t2 < sv - m;
+    okm &= ~__ballot_sync(FULL, open && !surely && !never);  // too close to call
+    open = open && surely;
+    const unsigned om = __ballot_sync(FULL, open);
+    if (!om) continue;
+    GrpGeom ge;
+    double c[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) c[d] = __shfl_sync(FULL, xp[d], __ffs(om) - 1);
+    ge.ch = make_float4(__double2float_rn(c[0]), __double2float_rn(c[1]), __double2float_rn(c[2]), 0.f);
+    ge.cl = make_float4(__double2float_rn(dsub(c[0], (double)ge.ch.x)),
+                        __double2float_rn(dsub(c[1], (double)ge.ch.y)),
+                        __double2float_rn(dsub(c[2], (double)ge.ch.z)), 0.f);
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+    L.act = open;
+    if (open) {
+      p = make_float4(__double2float_rn(xp[0]), __double2float_rn(xp[1]), __double2float_rn(xp[2]), 0.f);
+      L.x = __double2float_rn(dsub(xp[0], c[0]));
+      L.y = __double2float_rn(dsub(xp[1], c[1]));
+      L.z = __double2float_rn(dsub(xp[2], c[2]));
+      w.qs[lane] = make_float4(L.x, L.y, L.z, L.thr);
+    }
+    const float far = __uint_as_float(__reduce_max_sync(
+        FULL, open ? __float_as_uint(fmaxf(fabsf(L.x), fmaxf(fabsf(L.y), fabsf(L.z)))) : 0u));
+    two_e = fmaxf(two_e, __fmul_ru(4.f, __fadd_ru(__fmul_ru(far, 1.f / 4194304.f),
+                                                     __fmul_ru(tv.eps, 1.f / 524288.f))));
+    grp_box<S>(ge, open, p, __fmul_ru(2.f, tv.eps));
+    const float wide = __uint_as_float(__reduce_max_sync(FULL, open ? __float_as_uint(L.thr) : 0u));
+    ge.reach = grp_thresh(wide, two_e);
+    __syncwarp();
+    if (!grp_walk<S>(w, tv, ge, L, lane, gs, 0, 0, pass << kGrpImage, K, two_e)) {
+      okm &= ~om;
+      continue;
+    }
+    cut(om, false);
+  }
+  // the exact distances, from the image each neighbour was found in; rows as kEpiNN's
+  const int off = 1 - (a.kheap - (a.drop_largest ? 1 : 0) - a.kout);
+#pragma unroll 1
+  for (unsigned left = okm; left; left &= left - 1) {
+    const int q = __ffs(left) - 1, cnt = __shfl_sync(FULL, L.cnt, q);
+    double x[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) x[d] = __shfl_sync(FULL, x0[d], q);
+    long long key[S + 1];
+    int idx[S + 1];
+    auto exact = [&](int id) {
+      const int mk = kImageMask[id >> kGrpImage];
+      double xp[3] = {x[0], x[1], x[2]};
+      if (mk) reflect(x, xp, tv.period, mk);
+      const P4 y = tv.pos[id & ((1 << kGrpImage) - 1)];
+      return dkey(dist2_exact(xp[0], xp[1], xp[2], y.x, y.y, y.z));
+    };
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s <= S; s++) {
+      const int p = s * 32 + lane;
+      key[s] = 0;
+      idx[s] = -1;
+      if (p < cnt) {
+        idx[s] = w.bi[q][p];
+        key[s] = exact(idx[s]);
+      }
+    }
+    if (cnt > K) {
+      grp_keep<S>(key, idx, w.bi[q], lane, cnt, K);
+#pragma unroll
+      for (int s = 0; s < S; s++)
+        if (s * 32 + lane < K) {
+          idx[s] = w.bi[q][s * 32 + lane];
+          key[s] = exact(idx[s]);
+        }
+    }
+    long long kk[S];
+    int jj[S];
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const bool in = s * 32 + lane < K;
+      kk[s] = in ? key[s] : kWqSent;
+      jj[s] = in ? idx[s] & ((1 << kGrpImage) - 1) : -1;
+    }
+    grp_sort<S>(kk, jj, lane);
+    const size_t row = (size_t)(gs + q - a.q0) * a.kout;
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const int i = s * 32 + lane + off;
+      if (s * 32 + lane < K && i >= 0 && i < a.kout) {
+        a.nn[row + i] = jj[s];
+        a.d2[row + i] = __longlong_as_double(kk[s]);
+      }
+    }
+    if (off > 0 && lane == 0) {
+      a.nn[row] = gs + q;
+      a.d2[row] = 0.0;
+    }
+  }
+  grp_leave(a.fb, lane, gs, ((1u << gn) - 1u) & ~okm);
+}
+
+// A group without images: its searches, then what EPI makes of the neighbours.
 template <int S, int EPI>
 __device__ __forceinline__ void grp_serve(const KnnArgs& a, const TreeView& tv, GrpSmem<S>& w,
                                           int lane, int g, int depth, int K) {
@@ -688,15 +861,7 @@ __device__ __forceinline__ void grp_serve(const KnnArgs& a, const TreeView& tv, 
     float thr = __shfl_sync(FULL, L.thr, q);
     const int cnt = __shfl_sync(FULL, L.cnt, q), self = gs + q;
     const int how = grp_select<S>(w, tv, lane, q, self, cnt, K, two_e, thr);
-    bool ok = how != 0;
-    if (EPI == kEpiNN && ok && a.periodic) {
-      const float4 qf = tv.posf[self];
-      const float qeps = __fmul_ru(2.f, tv.eps);
-      const int near_sq = near_walls(qf, tv.period, qeps, thr);
-      const int near_lin = near_walls_lin(qf, tv.period, qeps, thr);
-      ok = near_sq == 0 && (a.min_image || __popc(near_lin) < 2);
-    }
-    if (!ok) continue;
+    if (how == 0) continue;
     okm |= 1u << q;
     if (EPI == kEpiSave) grp_save<S>(a, tv, w, lane, q, self, how, K, two_e);
     if (EPI == kEpiNN) {
@@ -714,9 +879,9 @@ __device__ __forceinline__ void grp_serve(const KnnArgs& a, const TreeView& tv, 
         }
       }
       grp_sort<S>(key, idx, lane);
-      // a periodic list starts with the query itself, then the others; the row leaves out
-      // the nearest (FindNearest) or the largest (FindNearestPos) where one more was asked
-      const int off = (a.periodic ? 1 : 0) - (a.kheap - (a.drop_largest ? 1 : 0) - a.kout);
+      // the row leaves out the nearest (FindNearest) or the largest (FindNearestPos) where one
+      // more was asked
+      const int off = -(a.kheap - (a.drop_largest ? 1 : 0) - a.kout);
       const size_t row = (size_t)(self - a.q0) * a.kout;
 #pragma unroll
       for (int s = 0; s < S; s++) {
@@ -726,23 +891,23 @@ __device__ __forceinline__ void grp_serve(const KnnArgs& a, const TreeView& tv, 
           a.d2[row + i] = __longlong_as_double(key[s]);
         }
       }
-      if (off > 0 && lane == 0) {
-        a.nn[row] = self;
-        a.d2[row] = 0.0;
-      }
     }
   }
   __syncwarp();
   if (EPI == kEpiDensity || EPI == kEpiDensVel || EPI == kEpiDensSave)
     grp_density<S, EPI == kEpiDensSave>(a, tv, w, lane, gs, okm, K);
   if (EPI == kEpiDensVel || EPI == kEpiVel) grp_veldensity<S>(a, tv, w, lane, gs, okm, K);
-  const unsigned am = ~okm & (gn >= 32 ? FULL : (1u << gn) - 1u);
-  if (am) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&a.fb[0], __popc(am));
-    base = __shfl_sync(FULL, base, 0);
-    if ((am >> lane) & 1u) a.fb[1 + base + __popc(am & ((1u << lane) - 1u))] = gs + lane;
-  }
+  grp_leave(a.fb, lane, gs, ((1u << gn) - 1u) & ~okm);
+}
+
+// K: neighbours other than the query itself; a periodic search's k + 1 list is the query
+// itself at zero distance, then the K = k nearest others (images included).
+template <int S>
+__global__ void __launch_bounds__(32 * kGrpWpb, 6) k_knn_group_periodic(KnnArgs a, int depth, int K) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GrpSmem<S>& w = reinterpret_cast<GrpSmem<S>*>(smem_raw)[threadIdx.x >> 5];
+  const int g = blockIdx.x * kGrpWpb + (threadIdx.x >> 5);
+  if (g < (1 << depth)) grp_periodic<S>(a, w, lane_id(), g, depth, K);
 }
 
 template <int S, int EPI>
@@ -843,7 +1008,12 @@ int launch_group(const KnnArgs& a, int K, cudaStream_t st) {
   NBK_CUDA_TRY(cudaMemsetAsync(a.fb, 0, sizeof(int), st));
   Phase ph(kNames[EPI], st);
   const unsigned blocks = ((1u << (depth - a.slices)) + kGrpWpb - 1) / kGrpWpb;
-  k_knn_group<S, EPI><<<blocks, 32 * kGrpWpb, sm, st>>>(a, depth, K); note_launch();
+  if (EPI == kEpiNN && a.periodic) {
+    NBK_TRY(ensure_dyn_smem((const void*)k_knn_group_periodic<S>, (int)sm));
+    k_knn_group_periodic<S><<<blocks, 32 * kGrpWpb, sm, st>>>(a, depth, K); note_launch();
+  } else {
+    k_knn_group<S, EPI><<<blocks, 32 * kGrpWpb, sm, st>>>(a, depth, K); note_launch();
+  }
   const unsigned lb = (unsigned)std::min<int64_t>(4 * nsm, ((int64_t)a.nq + kWqWpb - 1) / kWqWpb);
   if (a.kheap <= 32) k_knn_wq_list<1, EPI><<<lb, 32 * kWqWpb, 0, st>>>(a);
   else if (a.kheap <= 64) k_knn_wq_list<2, EPI><<<lb, 32 * kWqWpb, 0, st>>>(a);
@@ -880,7 +1050,8 @@ int launch_knn_group_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st
 bool group_search_serves(const KnnArgs& a) {
   const int K = a.periodic ? a.kheap - 1 : a.kheap;
   return a.qmode == 0 && a.fb && (a.nq == a.tv.n || a.slices > 0) && a.kheap <= 128 && K >= 1 &&
-         a.tv.n >= 4 * (K + 1) && a.tv.eps < 1e11f && (a.exclude_self || a.periodic);
+         a.tv.n >= 4 * (K + 1) && a.tv.eps < 1e11f &&
+         (a.periodic ? a.tv.n <= (1 << kGrpImage) : a.exclude_self != 0);
 }
 
 int launch_knn_group(const KnnArgs& a, int epi, cudaStream_t st) {

@@ -5,9 +5,10 @@ import numpy as np
 import pytest
 
 import oracle
-from nbodylib_gb300 import KDTree
+from nbodylib_gb300 import PERIODIC_MIN_IMAGE, PERIODIC_REF, KDTree
 from nbodylib_gb300 import synthetic as syn
-from tests.helpers import assert_density_close, assert_knn_equal, rows_by_id, to_ids
+from tests.helpers import (assert_density_close, assert_knn_equal, brute_min_image_knn, rows_by_id,
+                           to_ids)
 
 pytestmark = pytest.mark.gpu
 
@@ -72,6 +73,25 @@ def test_periodic_rows(gpu, port_built, method, n, b, k):
     oi, od = o.knn(k, method)
     assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), oi, od,
                      f"method {method}")
+
+
+@pytest.mark.parametrize("mode", [PERIODIC_REF, PERIODIC_MIN_IMAGE])
+@pytest.mark.parametrize("per", [[1.0, 1.0, 1.0], [1.0, 0.25, 2.0], [1.0, 1.0, 0.01]])
+def test_periodic_images(gpu, port_built, mode, per):
+    """Short sides (a particle's own images among its neighbours, lists across several walls)
+    in both image modes: the squared distances of the reference's search, or of brute force."""
+    n, k = 4097, 32
+    rng = np.random.default_rng(17)
+    pos = rng.random((n, 3)) * per
+    o = oracle.OracleTree(pos, None, np.ones(n), 16, 0, 0, 1000, per, backend="port", nthreads=8)
+    t = KDTree(pos, None, np.ones(n), 16, kerntype=0, period=per)
+    nn, d2 = t.FindNearest(k, periodic_mode=mode)
+    perm = t.GetPerm()
+    got = rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm)
+    if mode == PERIODIC_REF:
+        assert_knn_equal(*got, *o.knn(k, 0), f"images, period {per}")
+    elif min(per) > 0.1:  # every neighbour once: below half the shortest side
+        assert_knn_equal(*got, *brute_min_image_knn(pos, per, k), f"minimum image, period {per}")
 
 
 @pytest.mark.parametrize("n,b,k", [(40, 16, 8), (3001, 1000, 32), (5003, 16, 33), (5003, 1, 64),
