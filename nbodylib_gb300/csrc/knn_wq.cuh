@@ -40,7 +40,7 @@ namespace nbk {
 namespace {
 
 constexpr int kWqStack = 192;      // frontier stack (node indices) per warp
-constexpr int kWqBatchLimit = 64;  // above this many entries the stack pops one at a time
+constexpr int kWqBatchLimit = 96;  // above this many entries the stack pops one at a time
 constexpr long long kWqSent = 0x7fffffffffffffffll;  // key beyond position k - 1
 
 struct WqSmem {
@@ -244,7 +244,7 @@ __device__ __forceinline__ void wq_set_point(WqQuery<S>& Q, const TreeView& tv, 
 // Exact FP64 test of the first `cnt` queued candidates (one per lane) and insertion of
 // those below the k-th distance.
 template <int S>
-__device__ void wq_flush(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int lane, int cnt) {
+__device__ __forceinline__ void wq_flush(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int lane, int cnt) {
   const unsigned FULL = 0xffffffffu;
   bool have = lane < cnt;
   int ti = have ? w.queue[lane] : 0;
@@ -280,118 +280,103 @@ __device__ void wq_flush(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int lane,
   Q.thr = fminf(Q.thr, thresh_hi_bits(Q.topk));
 }
 
-// FP32 screen of one candidate per lane (valid lanes only); survivors join the queue,
-// which is flushed 32 at a time.
-template <int S>
-__device__ __forceinline__ void wq_consider(WqQuery<S>& Q, WqSmem& w, const TreeView& tv,
-                                            int lane, bool valid, int ti) {
-  const unsigned FULL = 0xffffffffu;
-  bool pass = false;
-  if (valid) {
-    float4 cf = tv.posf[ti];
-    pass = pair_d2_lo(Q.qx, Q.qy, Q.qz, cf.x, cf.y, cf.z, Q.two_eps) < Q.thr;
-  }
-  unsigned pm = __ballot_sync(FULL, pass);
-  if (!pm) return;
-  if (pass) w.queue[Q.qn + __popc(pm & ((1u << lane) - 1u))] = ti;
-  Q.qn += __popc(pm);
-  __syncwarp();
-  if (Q.qn >= 32) {
-    wq_flush<S>(Q, w, tv, lane, 32);
-    __syncwarp();
-    int rest = Q.qn - 32;
-    int moved = lane < rest ? w.queue[32 + lane] : 0;
-    __syncwarp();
-    if (lane < rest) w.queue[lane] = moved;
-    Q.qn = rest;
-    __syncwarp();
-  }
-}
-
-template <int S>
-__device__ __forceinline__ void wq_drain(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int lane) {
-  if (Q.qn > 0) {
-    wq_flush<S>(Q, w, tv, lane, Q.qn);
-    Q.qn = 0;
-    __syncwarp();
-  }
-}
-
-// Every particle of the node range [start, start + count) through the screen.
-template <int S>
-__device__ __forceinline__ void wq_range(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int lane,
-                                         int start, int count) {
-  for (int c0 = 0; c0 < count; c0 += 32)
-    wq_consider<S>(Q, w, tv, lane, c0 + lane < count, start + c0 + lane);
-}
-
-// Frontier-parallel traversal of every node whose FP32 box bound is below the k-th
-// distance: the whole tree when `home` is -1, else the whole tree but the subtree at heap
-// index `home` (already searched), which is the union of the subtrees of the siblings of
-// home and of each of its ancestors: those are pushed at once, so the first step tests
-// them all together instead of descending from the root one level per step. Returns
+// One pass over the tree: the particles [r0, r1) of the subtree at heap index `home` (those
+// around the query), then the subtrees of the siblings of home and of each of its ancestors,
+// which are tested together, one per lane, instead of descending from the root one level per
+// step; or the whole tree when `home` is -1. Frontier-parallel: up to 32 nodes per step are
+// tested against the k-th distance. Candidates (32 particles of the range, or the particles of
+// two leaves, 16 each, per step) that pass the FP32 screen join the queue, which is flushed 32
+// at a time. There is one place each for screening, flushing and testing nodes: inlined
+// several times over, the kernels waited for instructions (five of ten issue slots). Returns
 // false when the stack would overflow (the caller sets the error word).
 template <int S>
-__device__ bool wq_traverse(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int lane, int home) {
+__device__ __forceinline__ bool wq_pass(WqQuery<S>& Q, WqSmem& w, const TreeView& tv, int lane,
+                                        int home, int r0, int r1) {
   const unsigned FULL = 0xffffffffu;
-  int sp = 0;
-  if (home < 0) {
-    if (lane == 0) w.stk[0] = 0;
-    sp = 1;
-  } else {
-    // at most 31 levels (n < 2^31), well inside the stack
-    for (int h = home; h > 0; h = (h - 1) >> 1) {
-      if (lane == 0) w.stk[sp] = (h & 1) ? h + 1 : h - 1;
-      sp++;
+  int sp = 0, m = 1, h = 0;
+  if (home >= 0) {
+    m = 31 - __clz(home + 1);  // home's level (at most 31, n < 2^31)
+    if (lane < m) {
+      const int a = ((home + 1) >> lane) - 1;
+      h = (a & 1) ? a + 1 : a - 1;
     }
   }
-  __syncwarp();
-  for (int guard = 0; sp > 0 && guard < (1 << 24); guard++) {
-    int m = sp <= kWqBatchLimit ? min(32, sp) : 1;
-    int h = 0;
-    NodeRec r{};
+  unsigned lm = 0;     // leaves of the last step not screened yet (a bit per lane)
+  NodeRec r{};
+  int st = 0, ct = 0;  // the leaf this half warp screens, and how much of it is left
+#pragma unroll 1
+  for (int guard = 0; guard < (1 << 26); guard++) {
+    const bool part = __any_sync(FULL, ct > 0);
+    const bool have = r0 < r1 || part || lm;
+    const bool done = !have && m == 0;
+    if (have) {
+      int ti;
+      bool pass;
+      if (r0 < r1) {
+        ti = r0 + lane;
+        pass = ti < r1;
+        r0 += 32;
+      } else {
+        if (!part) {
+          const int l0 = __ffs(lm) - 1;
+          lm &= lm - 1;
+          const int l1 = lm ? __ffs(lm) - 1 : -1;
+          lm &= lm - 1;
+          const int src = lane < 16 ? l0 : l1;
+          st = __shfl_sync(FULL, r.start, src & 31);
+          ct = __shfl_sync(FULL, r.count, src & 31);
+          if (src < 0) ct = 0;
+        }
+        ti = st + (lane & 15);
+        pass = (lane & 15) < ct;
+        st += 16;
+        ct -= 16;
+      }
+      if (pass) {
+        const float4 cf = tv.posf[ti];
+        pass = pair_d2_lo(Q.qx, Q.qy, Q.qz, cf.x, cf.y, cf.z, Q.two_eps) < Q.thr;
+      }
+      const unsigned pm = __ballot_sync(FULL, pass);
+      if (pass) w.queue[Q.qn + __popc(pm & ((1u << lane) - 1u))] = ti;
+      Q.qn += __popc(pm);
+    }
+    if (Q.qn >= 32 || (done && Q.qn > 0)) {
+      __syncwarp();
+      const int cnt = min(32, Q.qn), rest = Q.qn - cnt;
+      wq_flush<S>(Q, w, tv, lane, cnt);
+      __syncwarp();
+      const int moved = lane < rest ? w.queue[32 + lane] : 0;
+      __syncwarp();
+      if (lane < rest) w.queue[lane] = moved;
+      Q.qn = rest;
+    }
+    if (done) return true;
+    if (have) continue;
+    // the next nodes
     bool need = false;
     if (lane < m) {
-      h = w.stk[sp - 1 - lane];
       r = tv.node[tv.nbase + h];
-      float blo = box_d2_lo(Q.qx, Q.qy, Q.qz, Q.eps, r);
-      need = blo < Q.thr;
+      need = box_d2_lo(Q.qx, Q.qy, Q.qz, Q.eps, r) < Q.thr;
     }
-    __syncwarp();
-    sp -= m;
-    bool leaf = need && r.count <= tv.b;
-    unsigned inner = __ballot_sync(FULL, need && !leaf);
-    int ne = __popc(inner);
+    const bool leaf = need && r.count <= tv.b;
+    const unsigned inner = __ballot_sync(FULL, need && !leaf);
+    lm = __ballot_sync(FULL, leaf);
+    const int ne = __popc(inner);
     if (sp + 2 * ne > kWqStack) return false;
-    if ((inner >> lane) & 1u) {
-      int slot = sp + 2 * __popc(inner & ((1u << lane) - 1u));
+    if ((inner >> lane) & 1u) {  // the children of the lowest lane's node end on top
+      const int slot = sp + 2 * __popc((inner >> lane) >> 1);
       w.stk[slot] = 2 * h + 2;
       w.stk[slot + 1] = 2 * h + 1;
     }
     sp += 2 * ne;
-    // leaves: packed into the 32 lanes (several small leaves per screening step)
-    unsigned lm = __ballot_sync(FULL, leaf);
-    int fill = 0, my = 0;
-    while (lm) {
-      int l = __ffs(lm) - 1;
-      int st = __shfl_sync(FULL, r.start, l), ct = __shfl_sync(FULL, r.count, l);
-      if (fill > 0 && fill + ct > 32) {
-        wq_consider<S>(Q, w, tv, lane, lane < fill, my);
-        fill = 0;
-      }
-      lm &= lm - 1;
-      if (ct > 32) {
-        for (int c0 = 0; c0 < ct; c0 += 32)
-          wq_consider<S>(Q, w, tv, lane, c0 + lane < ct, st + c0 + lane);
-        continue;
-      }
-      if (lane >= fill && lane < fill + ct) my = st + lane - fill;
-      fill += ct;
-    }
-    if (fill > 0) wq_consider<S>(Q, w, tv, lane, lane < fill, my);
+    __syncwarp();
+    m = sp <= kWqBatchLimit ? min(32, sp) : 1;
+    m = min(m, sp);
+    if (lane < m) h = w.stk[sp - 1 - lane];
+    sp -= m;
     __syncwarp();
   }
-  return sp == 0;
+  return false;
 }
 
 // Heap index, first particle and size of the smallest node on the path of tree index
@@ -502,39 +487,42 @@ __device__ void wq_search(WqQuery<S>& Q, WqSmem& w, const KnnArgs& a, const Tree
   Q.qn = 0;
   Q.self = exclude_self ? self : -1;
   wq_set_point<S>(Q, tv, x0);
-  int hh, hs, hn;
-  if (self >= 0) wq_home(tv, self, K + 1, hh, hs, hn);
-  else wq_home_point(tv, x0, K + 1, hh, hs, hn);
+  int home, r0, rn;
+  if (self >= 0) wq_home(tv, self, K + 1, home, r0, rn);
+  else wq_home_point(tv, x0, K + 1, home, r0, rn);
   // the bound lets the rest of the tree be pruned at once
-  Q.thr = fminf(Q.thr, wq_home_bound<S>(Q, tv, lane, self, hs, hn, K, exclude_self));
-  wq_range<S>(Q, w, tv, lane, hs, hn);
-  bool ok = hh == 0 || wq_traverse<S>(Q, w, tv, lane, hh);
-  wq_drain<S>(Q, w, tv, lane);
-  if (ok && a.periodic) {
-    Q.self = -1;
-    // image passes in the reference's order; the k-th distance only shrinks, so walls
-    // ruled out after the direct pass stay ruled out
-    float4 qf = make_float4(__double2float_rn(x0[0]), __double2float_rn(x0[1]),
-                            __double2float_rn(x0[2]), 0.f);
-    float top_hi = thresh_hi_bits(Q.topk);
-    float qeps = query_eps(tv, x0[0], x0[1], x0[2]);
-    int near_sq = near_walls(qf, tv.period, qeps, top_hi);
-    int near_lin = near_walls_lin(qf, tv.period, qeps, top_hi);
-    for (int pass = 1; pass < 8 && ok; pass++) {
-      int mk = kImageMask[pass];
-      bool lin = !(pass <= 3 || a.min_image);
+  Q.thr = fminf(Q.thr, wq_home_bound<S>(Q, tv, lane, self, r0, rn, K, exclude_self));
+  int near_sq = 0, near_lin = 0;
+  bool ok = true;
+#pragma unroll 1
+  for (int pass = 0; pass < 8 && ok; pass++) {
+    // pass 0 searches around the query; the image passes follow in the reference's order
+    if (pass > 0) {
+      if (!a.periodic) break;
+      const int mk = kImageMask[pass];
+      const bool lin = !(pass <= 3 || a.min_image);
+      if (pass == 1) {
+        // the k-th distance only shrinks, so walls ruled out after the direct pass stay ruled out
+        Q.self = -1;
+        const float4 qf = make_float4(__double2float_rn(x0[0]), __double2float_rn(x0[1]),
+                                      __double2float_rn(x0[2]), 0.f);
+        const float top_hi = thresh_hi_bits(Q.topk);
+        const float qeps = query_eps(tv, x0[0], x0[1], x0[2]);
+        near_sq = near_walls(qf, tv.period, qeps, top_hi);
+        near_lin = near_walls_lin(qf, tv.period, qeps, top_hi);
+      }
       if ((mk & ~(lin ? near_lin : near_sq)) != 0) continue;
       double xq[3];
-      double sval = reflect(x0, xq, tv.period, mk);
-      double top = __longlong_as_double(Q.topk);
+      const double sval = reflect(x0, xq, tv.period, mk);
+      const double top = __longlong_as_double(Q.topk);
       // KDSplitNode.cxx:1129 gates 1-D images with sqrt(top) > sval, :1134-1146 the 2-D
       // and 3-D images with top > sval
-      bool g = lin ? (top > sval) : (__dsqrt_rn(top) > sval);
-      if (!g) continue;
+      if (!(lin ? (top > sval) : (dsqrt_call(top) > sval))) continue;
       wq_set_point<S>(Q, tv, xq);
-      ok = wq_traverse<S>(Q, w, tv, lane, -1);
-      wq_drain<S>(Q, w, tv, lane);
+      home = -1;
+      r0 = rn = 0;
     }
+    ok = wq_pass<S>(Q, w, tv, lane, home, r0, r0 + rn);
   }
   if (!ok && lane == 0) atomicExch(a.err, kErrCapacity);
 }
