@@ -14,10 +14,11 @@
 // order (not the terms) differs from the reference's. A row costs 4 B per neighbour each way;
 // trees of more than kSliceMax particles go slice by slice, so that the rows stay small.
 //
-// What bounds it: the FP64 pipe, 19 instructions a pair for CalcSmoothVel and 37 for
-// CalcSmoothVelDisp (its nine sums are six, the matrix being symmetric). As epilogues of a
-// lane-per-query search with all divisions per pair the two took 8.2 ms each at 2^20
-// clustered particles, Nsmooth = 32.
+// What bounds it: the search, and in k_smooth_rows the FP64 pipe (85% busy), 18 instructions a
+// pair for CalcSmoothVel and 36 for CalcSmoothVelDisp (its nine sums are six, the matrix being
+// symmetric). As epilogues of a lane-per-query search with all divisions per pair the two took
+// 8.2 ms each at 2^20 clustered particles, Nsmooth = 32; now the searches take 2.65 ms
+// each and everything after them 3.8 ms for the two.
 #include <algorithm>
 
 #include "knn_wq.cuh"
@@ -128,9 +129,12 @@ __global__ void __launch_bounds__(128) k_smooth_rows(SmoothArgs s, SmoothPrep P,
     const double dx = dsub(x, c.x), dy = dsub(y, c.y), dz = dsub(z, c.z);
     const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dmul(dx, dx)));
     // the farthest neighbour sits at q = 2 exactly: the table's last entry
-    const double w = d2 == top ? T[kr - 1] : w_at_u(dmul(sqrt_newton(d2), c1), kr, T);
-    const double ta = dmul(dmul(w, wnorm), P.mr[j]);  // W_ij m_j / rho_j, into the query
-    const double tb = dmul(w, wi);                    // W_ij m_i / rho_i, into neighbour j
+    // (compared by their bits: FP64 compares take the FP64 pipe)
+    const double w = dkey(d2) == dkey(top) ? T[kr - 1] : w_at_u(dmul(sqrt_newton(d2), c1), kr, T);
+    // W_ij m_j / rho_j into the query (times wnorm: at the end, but for the kurtosis, whose
+    // terms are shifted), W_ij m_i / rho_i into neighbour j
+    const double ta = dmul(SM == kSmVelKurt ? dmul(w, wnorm) : w, P.mr[j]);
+    const double tb = dmul(w, wi);
     if (SM == kSmMeanOne) {
       acc[0] = __fma_rn(ta, P.wt[j], acc[0]);
     } else if (SM == kSmDispOne) {
@@ -192,6 +196,9 @@ __global__ void __launch_bounds__(128) k_smooth_rows(SmoothArgs s, SmoothPrep P,
       }
     }
   }
+  if (SM != kSmVelKurt)
+#pragma unroll
+    for (int k = 0; k < 6; k++) acc[k] = dmul(acc[k], wnorm);
   constexpr int kAcc = SM == kSmVelDisp || SM == kSmVelDispOne ? 6
                        : SM == kSmMeanOne || SM == kSmDispOne  ? 1
                                                                : 3;
