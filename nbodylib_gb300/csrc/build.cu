@@ -1167,7 +1167,8 @@ struct PartOut {
   V4* vel;
   int* perm;
   float4* velf;  // ND = 6 only
-  float4* posr;  // ND = 3 only
+  float4* posr;  // FP32 residuals (null: not kept)
+  float4* velr;  // ND = 6 only
 };
 
 template <int ND>
@@ -1464,15 +1465,21 @@ __global__ void __launch_bounds__(kLocalThreads) k_local_build(
     const float4 f = make_float4(__double2float_rn(p.x), __double2float_rn(p.y),
                                  __double2float_rn(p.z), 0.f);
     po.posf[t] = f;
-    if (ND == 3)
+    if (ND == 3 || po.posr)
       po.posr[t] = make_float4(__double2float_rn(dsub(p.x, (double)f.x)),
                                __double2float_rn(dsub(p.y, (double)f.y)),
                                __double2float_rn(dsub(p.z, (double)f.z)), 0.f);
     po.perm[t] = ii;
     if (ND == 6) {
       po.vel[t] = make_v4(cc[3 * K + q], cc[4 * K + q], cc[5 * K + q], 0.0);
-      po.velf[t] = make_float4(__double2float_rn(cc[3 * K + q]), __double2float_rn(cc[4 * K + q]),
-                               __double2float_rn(cc[5 * K + q]), 0.f);
+      const double vx = cc[3 * K + q], vy = cc[4 * K + q], vz = cc[5 * K + q];
+      const float4 g = make_float4(__double2float_rn(vx), __double2float_rn(vy),
+                                   __double2float_rn(vz), 0.f);
+      po.velf[t] = g;
+      if (po.velr)
+        po.velr[t] = make_float4(__double2float_rn(dsub(vx, (double)g.x)),
+                                 __double2float_rn(dsub(vy, (double)g.y)),
+                                 __double2float_rn(dsub(vz, (double)g.z)), 0.f);
     } else if (po.vel && vel_in) {
       po.vel[t] = make_v4(vel_in[3 * ii], vel_in[3 * ii + 1], vel_in[3 * ii + 2], 0.0);
     }
@@ -1838,7 +1845,7 @@ int build_forest(const std::vector<TreeSpec>& trees, int b, const double* d_pos_
                  const double* d_mass_in, const double* d_vel_in, BuiltArrays& out,
                  DevAlloc& alloc, cudaStream_t st, NodeX* root_out) {
   NodeOut<3> no{out.node, out.nodex};
-  PartOut<3> po{out.pos, out.posf, out.vel, out.perm, nullptr, out.posr};
+  PartOut<3> po{out.pos, out.posf, out.vel, out.perm, nullptr, out.posr, nullptr};
   const void* src = trees.empty() ? nullptr : (const void*)(out.nodex + trees[0].nbase);
   return build_forest_t<3>(trees, b, d_pos_in, d_mass_in, d_vel_in, no, po, alloc, st, root_out,
                            sizeof(NodeX), src);
@@ -1852,7 +1859,7 @@ int build_forest_phase(const std::vector<TreeSpec>& trees, int b, const double* 
     return NBK_ERR_INVALID;
   }
   NodeOut<6> no{out.nodes6, out.nodeb6, out.nodef6};
-  PartOut<6> po{out.pos, out.posf, out.vel, out.perm, out.velf, nullptr};
+  PartOut<6> po{out.pos, out.posf, out.vel, out.perm, out.velf, out.posr, out.velr};
   const void* src = trees.empty() ? nullptr : (const void*)(out.nodeb6 + trees[0].nbase);
   return build_forest_t<6>(trees, b, d_pos_in, d_mass_in, d_vel_in, no, po, alloc, st, root_out,
                            sizeof(NodeB6), src);

@@ -379,6 +379,7 @@ struct nbk_tree {
     v.pos = arr.pos;
     v.posf = arr.posf;
     v.posr = arr.posr;
+    v.velr = arr.velr;
     v.vel = arr.vel;
     v.perm = arr.perm;
     v.node = arr.node;
@@ -765,12 +766,13 @@ int nbk_create(const double* pos, const double* vel, const double* mass, int64_t
     size_t zeroed = block_bytes(parts);
     parts.push_back({(void**)&A.pos, sizeof(P4) * n});
     parts.push_back({(void**)&A.posf, sizeof(float4) * n});
-    if (!phs) parts.push_back({(void**)&A.posr, sizeof(float4) * n});
+    parts.push_back({(void**)&A.posr, sizeof(float4) * n});
     parts.push_back({(void**)&A.perm, sizeof(int) * n});
     if (vel) parts.push_back({(void**)&A.vel, sizeof(V4) * n});
     if (phs) {
       parts.push_back({(void**)&A.nodef6, sizeof(NodeF6) * t->nslots});
       parts.push_back({(void**)&A.velf, sizeof(float4) * n});
+      parts.push_back({(void**)&A.velr, sizeof(float4) * n});
     }
     NBK_TRY(dev_malloc(&t->block, block_bytes(parts), st));
     carve_block(t->block, parts);

@@ -46,7 +46,8 @@ struct TreeSpec {
 struct BuiltArrays {
   P4* pos = nullptr;
   float4* posf = nullptr;
-  float4* posr = nullptr;     // physical / velocity trees
+  float4* posr = nullptr;     // FP32 residuals (null: not kept)
+  float4* velr = nullptr;     // phase-space trees
   V4* vel = nullptr;
   int* perm = nullptr;
   NodeRec* node = nullptr;    // physical / velocity trees

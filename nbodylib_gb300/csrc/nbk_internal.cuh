@@ -3,7 +3,7 @@
 // HBM layout of a built tree (all arrays in tree order unless noted):
 //   P4      pos[n]    x, y, z, mass as FP64 (32 B, two 16-B vector loads)
 //   float4  posf[n]   x, y, z rounded to nearest FP32 (candidate filter)
-//   float4  posr[n]   x - posf.x, ... rounded to FP32 (local offsets of the group search)
+//   float4  posr[n]   x - posf.x, ... rounded to FP32 (local offsets of the group searches)
 //   V4 vel[n]    vx, vy, vz, 0 (only when velocities were given)
 //   int32   perm[n]   tree index -> input index
 //   NodeRec node[]    heap-indexed (root 0, children 2h+1 / 2h+2): FP32 bounding box
@@ -71,7 +71,8 @@ struct __align__(16) NodeF6 {  // the same box in FP32, rounded outward
 struct TreeView {
   const P4* pos;
   const float4* posf;
-  const float4* posr;    // physical / velocity trees
+  const float4* posr;    // FP32 residuals
+  const float4* velr;    // phase-space trees
   const V4* vel;
   const int* perm;
   const NodeRec* node;
@@ -262,18 +263,10 @@ __device__ __forceinline__ int near_walls_lin(float4 q, const double p[3], float
 // (KDSplitNode.cxx:1126-1147).
 __device__ __constant__ static const int kImageMask[8] = {0, 1, 2, 4, 3, 5, 6, 7};
 
-// Wsm (KDCalcSmoothQuantities.cxx:12-15) on the host-built table.
-__device__ __forceinline__ double wsm(double r, int i, int size, double delta, const double* x) {
-  if (i < size - 1) {
-    double xi = x[i], xj = x[i + 1];
-    return dadd(xi, __ddiv_rn(dmul(dsub(xj, xi), dsub(r, dmul(delta, (double)i))), delta));
-  }
-  return x[i];
-}
-// The same interpolation from the table's device image [T | A | B]: on cell i the line
-// through T[i] and T[i+1] is A[i] + B[i] q, one FMA. The cell index is the reference's
-// (int)(q * 0.5 * (size - 1)); the result differs from wsm() by a few units in the last
-// place (the interpolant is continuous across cells, so a neighbouring cell gives the
+// Wsm (KDCalcSmoothQuantities.cxx:12-15) from the device image [T | A | B | D] of the
+// host-built table: on cell i the line through T[i] and T[i+1] is A[i] + B[i] q, one FMA. The
+// cell index is the reference's (int)(q * 0.5 * (size - 1)); the result differs from the
+// reference's interpolation by a few units in the last place (the interpolant is continuous across cells, so a neighbouring cell gives the
 // same value up to rounding).
 __device__ __forceinline__ double wsm_line(double q, int size, double inv_delta,
                                            const double* img) {
@@ -403,16 +396,6 @@ __device__ __forceinline__ double sqrt_newton(double x) {
       (int)((((u & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20)) | (u & 0x80000000u)), (int)(u << 29));
   const double q = dadd(f64_of_f32(q0), d1);
   return __fma_rn(__fma_rn(-q, q, x), f64_of_f32(hy), q);
-}
-
-// W(q) at q = sqrt(d2) / h with h = sqrt(top) / 2 (ih = 1/h): the farthest neighbour
-// (d2 == top) is at q = 2 exactly in the reference's arithmetic, the table's last entry
-// (0 for the compact kernels); the product with 1/h could land an ulp below, in the
-// previous cell.
-__device__ __forceinline__ double w_at_d2(double d2, long long topk, double ih, int size,
-                                          double inv_delta, const double* img) {
-  if (dkey(d2) == topk) return img[size - 1];
-  return wsm_line(dmul(__dsqrt_rn(d2), ih), size, inv_delta, img);
 }
 
 // Kernels that follow one another in a chain are launched as programmatic dependents of the

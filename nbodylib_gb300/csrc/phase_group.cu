@@ -28,9 +28,15 @@
 // visiting it took up to 90 ms. Queries without a metric spacing take the lane-per-query
 // kernel.
 //
-// Coordinates are screened as FP32 offsets from the group's middle particle, formed in FP64,
-// so that their rounding is relative to the group's extent: with s the FP32 sum and d the
-// distance, |sqrt(s) - d| <= E + 2^-20 sqrt(s), E = sqrt(sum w (2^-23 extent)^2).
+// Measured (2^18 clustered particles, local metric, CalcDensity(32); it depends on the seed):
+// 6.3-14.7 ms, a lane per query 31-50 ms; the FP64 pipe and instruction issue are each half
+// busy at 20 warps per SM (28 warps: 12.6 against 11.5 ms, spills). Offsets formed in FP64
+// from the exact coordinates cost 11.5 ms where the FP32 copies and residuals cost 9.5.
+//
+// Coordinates are screened as FP32 offsets from the group's middle particle, formed from the
+// FP32 copies and their residuals, so that their rounding is relative to the group's extent:
+// with s the FP32 sum and d the distance, |sqrt(s) - d| <= E + 2^-20 sqrt(s),
+// E = sqrt(sum w (2^-22 extent + 2^-19 eps)^2), eps the FP32 rounding of a coordinate.
 #include <algorithm>
 
 #include "knn_select.cuh"
@@ -41,8 +47,11 @@ namespace {
 
 constexpr int kPgWpb = 4;     // warps (groups) per block
 constexpr int kPgStack = 192;
-constexpr int kPgPop = 16;    // nodes tested per step
-constexpr int kPgSeed = 1;    // home holds at least this many times K particles
+// nodes tested per step (2^18 clustered particles, k = 32: 32 at once 29 ms, 16 13 ms: the
+// frontier grows before the K-th distances have shrunk)
+constexpr int kPgPop = 16;
+// home holds at least this many times K particles (2 and 4 times were no faster)
+constexpr int kPgSeed = 1;
 
 // One query's row in shared memory.
 struct __align__(16) PgQuery {
@@ -65,20 +74,22 @@ struct PgSmem {
 // buffer count and E.
 struct PgPass {
   int gs, gn;      // first particle (tree index), particles
-  double c[6];     // centre
+  float4 ph, pl, vh, vl;  // centre: FP32 copies and residuals
   int cnt;
   float two_e;
   unsigned act;
   bool skip_self;
 };
 
-// FP32 value of any double, rounded to nearest, on the integer pipe; below FP32's normal
-// range it is zero.
-__device__ __forceinline__ float f32_signed(double x) {
-  const int hi = __double2hiint(x);
-  const float m = f32_of_bits(hi & 0x7fffffff, __double2loint(x));
-  const float v = (hi & 0x7fffffff) < ((1023 - 126) << 20) ? 0.f : m;
-  return __uint_as_float(__float_as_uint(v) | ((unsigned)hi & 0x80000000u));
+// Offsets of particle ti from the group's centre.
+__device__ __forceinline__ void pg_offsets(const TreeView& tv, const PgPass& P, int ti, float c[6]) {
+  const float4 p = tv.posf[ti], pr = tv.posr[ti], v = tv.velf[ti], vr = tv.velr[ti];
+  c[0] = (p.x - P.ph.x) + (pr.x - P.pl.x);
+  c[1] = (p.y - P.ph.y) + (pr.y - P.pl.y);
+  c[2] = (p.z - P.ph.z) + (pr.z - P.pl.z);
+  c[3] = (v.x - P.vh.x) + (vr.x - P.vl.x);
+  c[4] = (v.y - P.vh.y) + (vr.y - P.vl.y);
+  c[5] = (v.z - P.vh.z) + (vr.z - P.vl.z);
 }
 
 // Screen one candidate per lane (mask: the queries that want it) for every query of `any`.
@@ -88,16 +99,7 @@ __device__ __forceinline__ void pg_screen(PgSmem<S>& w, const TreeView& tv, PgPa
   const unsigned FULL = 0xffffffffu;
   constexpr int cap = GrpCfg<S>::cap;
   float c[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (mask) {
-    const P4 p = tv.pos[ti];
-    const V4 v = tv.vel[ti];
-    c[0] = f32_signed(dsub(p.x, P.c[0]));
-    c[1] = f32_signed(dsub(p.y, P.c[1]));
-    c[2] = f32_signed(dsub(p.z, P.c[2]));
-    c[3] = f32_signed(dsub(v.x, P.c[3]));
-    c[4] = f32_signed(dsub(v.y, P.c[4]));
-    c[5] = f32_signed(dsub(v.z, P.c[5]));
-  }
+  if (mask) pg_offsets(tv, P, ti, c);
 #pragma unroll 1
   for (unsigned any = __reduce_or_sync(FULL, mask) & P.act; any; any &= any - 1) {
     const int i = __ffs(any) - 1;
@@ -386,28 +388,24 @@ __global__ void __launch_bounds__(32 * kPgWpb, 5) k_phase_group(PhaseArgs pa, Pg
   P.gs = tv.pstart + s0;
   P.gn = sz;
   {
-    const P4 p = tv.pos[P.gs + (sz >> 1)];
-    const V4 v = tv.vel[P.gs + (sz >> 1)];
-    P.c[0] = p.x;
-    P.c[1] = p.y;
-    P.c[2] = p.z;
-    P.c[3] = v.x;
-    P.c[4] = v.y;
-    P.c[5] = v.z;
+    const int mid = P.gs + (sz >> 1);
+    P.ph = tv.posf[mid];
+    P.pl = tv.posr[mid];
+    P.vh = tv.velf[mid];
+    P.vl = tv.velr[mid];
   }
   float far[6];
   {
     float o[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (lane < sz) {
-      const P4 p = tv.pos[P.gs + lane];
-      const V4 v = tv.vel[P.gs + lane];
-      const double y[6] = {p.x, p.y, p.z, v.x, v.y, v.z};
+      const float4 p = tv.posf[P.gs + lane], v = tv.velf[P.gs + lane];
+      const float y[6] = {p.x, p.y, p.z, v.x, v.y, v.z};
       PgQuery& Q = w.q[lane];
+      pg_offsets(tv, P, P.gs + lane, o);
 #pragma unroll
       for (int k = 0; k < 6; k++) {
-        o[k] = f32_signed(dsub(y[k], P.c[k]));
         Q.q[k] = o[k];
-        Q.a[k] = __double2float_rn(y[k]);
+        Q.a[k] = y[k];
         Q.w[k] = 1.f;
       }
     }
@@ -417,13 +415,15 @@ __global__ void __launch_bounds__(32 * kPgWpb, 5) k_phase_group(PhaseArgs pa, Pg
   }
   __syncwarp();
   const unsigned all = (1u << sz) - 1u;
-  // 2E of weights u: each offset carries 2^-24 of it (both ends); the parts proportional to
-  // the distance are in the relative margin of grp_thresh
+  // 2E of weights u: each offset carries 2^-23 of it (both ends) and its residual's rounding
+  // (far below 2^-19 eps); the parts proportional to the distance are in the relative margin
+  // of grp_thresh
   auto two_e_of = [&](const float u[6]) {
     float s = 0.f;
 #pragma unroll
     for (int k = 0; k < 6; k++) {
-      const float e = __fadd_ru(__fmul_ru(far[k], 1.f / 4194304.f), 1e-37f);
+      const float e = __fadd_ru(__fmul_ru(far[k], 1.f / 4194304.f),
+                                __fmul_ru(tv.eps6[k], 1.f / 524288.f));
       s = __fadd_ru(s, __fmul_ru(__fmul_ru(__fmul_ru(u[k], 1.0001f), e), e));
     }
     return __fmul_ru(__fsqrt_ru(s), 2.02f);
@@ -983,7 +983,8 @@ int launch_pg_e(const PhaseArgs& pa, DevAlloc& alloc, cudaStream_t st) {
 
 }  // namespace
 
-// Every particle of a tree, no images; the screened squares must stay inside FP32.
+// Every particle of a tree, no images; the screened squares must stay inside FP32. Queries in
+// no order, part of a tree or with images take a lane each (phase.cu).
 bool phase_group_serves(const PhaseArgs& pa) {
   const KnnArgs& a = pa.k;
   if (pa.epi == kPhDensPart || a.qmode != 0 || a.q0 != 0 || a.nq != a.tv.n || a.periodic ||
