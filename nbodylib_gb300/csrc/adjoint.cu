@@ -13,7 +13,7 @@
 // The backward kernel recomputes every weight from the saved neighbour lists (4 B per
 // neighbour) instead of storing weights; one thread per particle, FP64 atomics for the
 // contributions that land on other particles. What bounds it is the FP64 pipe: 30
-// instructions a pair (46 before the terms were rearranged: 3.45 ms at 2^20, k = 32). In the
+// instructions a pair, 2.08 ms at 2^20, k = 32 (46 before the terms were rearranged, 3.45 ms). In the
 // table coordinate u = q (kernres - 1) / 2 the line of a cell is T = A + D u and q T' = D u,
 // factors of the particle alone (h^-3, h^-4, dL/drho_i) are taken out of the sums, the cell
 // comes from the bits of u, and r and 1/r from one FP32 reciprocal square root (corrected in
