@@ -27,6 +27,12 @@ namespace {
 constexpr int kStack = 512;  // node stack of one warp
 constexpr int kBatch = kStack - 128;
 constexpr int kWpb = 4;
+// Volume in cubed radii of the box around a warp's balls above which inner nodes are tested
+// query by query: 32 balls apart from one another fill 134. (2^17 targets in random order of
+// 2^20 particles, 32 per ball: 98 ms never tested, 1.82 with this line; 2^20 in tree order:
+// 1.55 either way, 1.86 always tested; 20,001 with 64 per ball: 0.66 with the line at 512,
+// 0.29 at 128, 1.32 never.)
+constexpr float kBallVolume = 128.f;
 
 struct BallArgs {
   TreeView tv;
@@ -91,6 +97,7 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
   const float lf = __fadd_ru(__fsqrt_ru(thr), e), ln = __fsub_rd(__fsqrt_rd(r2_lo), e);
   const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 524288.0f);
   const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 524288.0f) : 0.f;
+  const float rinv = rsqrtf(thr);  // 0 or NaN: strict, or no ball
   const int npass = tv.periodic ? 8 : 1;
   int near = 0;
   if (tv.periodic && valid)
@@ -109,8 +116,10 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
     if (!__any_sync(FULL, active)) continue;
     const float qx = __double2float_rn(xq[0]), qy = __double2float_rn(xq[1]),
                 qz = __double2float_rn(xq[2]);
-    // box around the active lanes' query points, widened by their rounding
-    float qlo[3], qhi[3];
+    // box around the active lanes' query points, widened by their rounding; where it is much
+    // larger than their balls together (points in no order, or on both sides of a high split)
+    // inner nodes are opened only if a ball reaches them
+    float qlo[3], qhi[3], vol = 1.f;
     {
       const float v[3] = {qx, qy, qz};
 #pragma unroll
@@ -123,8 +132,10 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
         }
         qlo[d] = lo;
         qhi[d] = hi;
+        vol *= (hi - lo) * rinv + 2.f;
       }
     }
+    const bool strict = !(vol <= kBallVolume);
     __syncwarp();
     w.q[lane] = make_float4(qx, qy, qz, 0.f);
     if (lane == 0) w.stk[0] = 0;
@@ -154,6 +165,20 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
       __syncwarp();
       sp -= m;
       const bool leaf = r.count <= tv.b;
+      if (strict) {
+#pragma unroll 1
+        for (unsigned left = __ballot_sync(FULL, keep && !leaf); left; left &= left - 1) {
+          const int j = __ffs(left) - 1;
+          NodeRec rj;
+#pragma unroll
+          for (int d = 0; d < 3; d++) {
+            rj.lo[d] = __shfl_sync(FULL, r.lo[d], j);
+            rj.hi[d] = __shfl_sync(FULL, r.hi[d], j);
+          }
+          const bool reach = __any_sync(FULL, active && box_d2_lo(qx, qy, qz, eps, rj) < thr);
+          if (lane == j) keep = reach;
+        }
+      }
       const unsigned km = __ballot_sync(FULL, keep), im = __ballot_sync(FULL, keep && !leaf);
       const unsigned ahead = im ? (im & (0u - im)) - 1u : 0xffffffffu;  // lanes before it
       // what follows the first inner node goes back, its children in its place
@@ -262,7 +287,8 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
 }
 
 // Queries per warp: 32 where that leaves enough warps for every SM (a lane each; the other
-// lanes still take nodes and particles).
+// lanes still take nodes and particles). 16,385 balls of 32: 0.28 ms with 32 a warp, 0.22 with
+// the 4 of this rule; 55,839 of 39: 0.41 and 0.36 with 16.
 int ball_qpw(int64_t nq, int* qpw) {
   int dev = 0, nsm = 0;
   NBK_CUDA_TRY(cudaGetDevice(&dev));

@@ -11,6 +11,21 @@ from tests.helpers import d2_ref, reflect_images
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("n", [129, 5003, 40001])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_order_of_targets(gpu, n, periodic):
+    """A target's row does not depend on the targets beside it: a few in random order (balls all
+    over the box), all of them in tree order."""
+    pos, mass = syn.clustered_box(n, 1.0, seed=4, nspheres=6)
+    t = KDTree(pos, None, mass, 16, kerntype=0, period=[1.0, 1.0, 1.0] if periodic else None)
+    some = np.random.default_rng(1).permutation(n)[:3000].astype(np.int32)
+    for r in (1e-3, 0.02):
+        off, idx = t.SearchBallPosTagged(np.arange(n, dtype=np.int32), r * r)
+        off2, idx2 = t.SearchBallPosTagged(some, r * r)
+        for i, j in enumerate(some):
+            assert np.array_equal(idx2[off2[i]:off2[i + 1]], idx[off[j]:off[j + 1]]), (r, j)
+
+
 @pytest.mark.parametrize("n,b,nq", [(40, 16, 1), (2049, 16, 3), (3001, 5, 700), (3001, 17, 33),
                                     (3001, 100, 64), (5003, 16, 5003)])
 @pytest.mark.parametrize("periodic", [False, True])
