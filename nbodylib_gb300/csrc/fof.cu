@@ -1017,7 +1017,9 @@ __global__ void k_relabel(int* group, const int* newlbl, int n) {
 }  // namespace
 
 // Queries per warp of the link kernels (a lane each; the other lanes still take nodes and
-// candidates): as many as 32 where that leaves enough warps for every SM.
+// candidates): as many as 32 where that leaves enough warps for every SM (linking 5,003
+// particles: 0.24 ms with 32 a warp, 0.16 with the 2 of this rule; 2^20: 1.23 ms with 32,
+// 1.30 with 16, 1.66 with 8, before the blocks of 4 warps).
 constexpr int kQpwMax = 32, kQpwMin = 2;
 int queries_per_warp(int64_t n, int* qpw) {
   int dev = 0, nsm = 0;
