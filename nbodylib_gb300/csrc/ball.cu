@@ -16,8 +16,8 @@
 // (in tree order: the leaves ahead of the first inner node are tested, what follows is pushed
 // back), leaf particles are tested a lane each, two leaves at a time, one query after another
 // of those that want the leaf, and one round-to-nearest distance decides outside a band of
-// its own rounding error around the radius: 1.24 ms (both passes; 40 warps per SM, 1.31 ms
-// with 32).
+// its own rounding error around the radius: 1.50 ms (both passes; 32 warps per SM, 1.53 ms
+// with 40, which spills).
 #include "nbk_build.h"
 
 namespace nbk {
@@ -27,11 +27,11 @@ namespace {
 constexpr int kStack = 512;  // node stack of one warp
 constexpr int kBatch = kStack - 128;
 constexpr int kWpb = 4;
-// Volume in cubed radii of the box around a warp's balls above which inner nodes are tested
-// query by query: 32 balls apart from one another fill 134. (2^17 targets in random order of
-// 2^20 particles, 32 per ball: 98 ms never tested, 1.82 with this line; 2^20 in tree order:
-// 1.55 either way, 1.86 always tested; 20,001 with 64 per ball: 0.66 with the line at 512,
-// 0.29 at 128, 1.32 never.)
+// Volume in cubed radii of the box around a warp's balls above which nodes are tested query by
+// query: 32 balls apart from one another fill 134. (2^17 targets in random order of 2^20
+// particles, 32 per ball: 98 ms never tested, 1.28 with this line; 20,001 targets with 64 per
+// ball: 1.32 never, 0.66 with the line at 512, 0.24 at 128; 2^20 in tree order 1.55 either way,
+// 1.86 always tested.)
 constexpr float kBallVolume = 128.f;
 
 struct BallArgs {
@@ -56,7 +56,7 @@ struct BallSmem {
 };
 
 template <bool FILL>
-__global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
+__global__ void __launch_bounds__(32 * kWpb, 8) k_ball(BallArgs a) {
   __shared__ BallSmem sm[kWpb];
   const unsigned FULL = 0xffffffffu;
   int lane;  // read once
@@ -97,7 +97,6 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
   const float lf = __fadd_ru(__fsqrt_ru(thr), e), ln = __fsub_rd(__fsqrt_rd(r2_lo), e);
   const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 524288.0f);
   const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 524288.0f) : 0.f;
-  const float rinv = rsqrtf(thr);  // 0 or NaN: strict, or no ball
   const int npass = tv.periodic ? 8 : 1;
   int near = 0;
   if (tv.periodic && valid)
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
                 qz = __double2float_rn(xq[2]);
     // box around the active lanes' query points, widened by their rounding; where it is much
     // larger than their balls together (points in no order, or on both sides of a high split)
-    // inner nodes are opened only if a ball reaches them
+    // nodes are taken only if a ball reaches them
     float qlo[3], qhi[3], vol = 1.f;
     {
       const float v[3] = {qx, qy, qz};
@@ -132,10 +131,10 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
         }
         qlo[d] = lo;
         qhi[d] = hi;
-        vol *= (hi - lo) * rinv + 2.f;
+        vol *= (hi - lo) * rsqrtf(thr) + 2.f;
       }
     }
-    const bool strict = !(vol <= kBallVolume);
+    const bool strict = !(vol <= kBallVolume);  // infinite or NaN: an empty ball
     __syncwarp();
     w.q[lane] = make_float4(qx, qy, qz, 0.f);
     if (lane == 0) w.stk[0] = 0;
@@ -166,18 +165,17 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_ball(BallArgs a) {
       sp -= m;
       const bool leaf = r.count <= tv.b;
       if (strict) {
+        // a lane per node, as far as a hit of any query can be (see far2)
+        bool reach = false;
 #pragma unroll 1
-        for (unsigned left = __ballot_sync(FULL, keep && !leaf); left; left &= left - 1) {
-          const int j = __ffs(left) - 1;
-          NodeRec rj;
-#pragma unroll
-          for (int d = 0; d < 3; d++) {
-            rj.lo[d] = __shfl_sync(FULL, r.lo[d], j);
-            rj.hi[d] = __shfl_sync(FULL, r.hi[d], j);
-          }
-          const bool reach = __any_sync(FULL, active && box_d2_lo(qx, qy, qz, eps, rj) < thr);
-          if (lane == j) keep = reach;
+        for (unsigned qm = __ballot_sync(FULL, active); qm; qm &= qm - 1) {
+          const float4 qf = w.q[__ffs(qm) - 1];
+          const float gx = fmaxf(0.f, fmaxf(r.lo[0] - qf.x, qf.x - r.hi[0]));
+          const float gy = fmaxf(0.f, fmaxf(r.lo[1] - qf.y, qf.y - r.hi[1]));
+          const float gz = fmaxf(0.f, fmaxf(r.lo[2] - qf.z, qf.z - r.hi[2]));
+          reach = reach || !(gx * gx + gy * gy + gz * gz >= far2);
         }
+        keep = keep && reach;
       }
       const unsigned km = __ballot_sync(FULL, keep), im = __ballot_sync(FULL, keep && !leaf);
       const unsigned ahead = im ? (im & (0u - im)) - 1u : 0xffffffffu;  // lanes before it
