@@ -1050,15 +1050,17 @@ int launch_knn_group_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st
 }
 
 // Every particle of a tree (or a slice of it), none of them given zero-distance or image
-// answers that FP32 offsets cannot tell apart, k within the buffers, squares inside FP32, and
-// four times as many particles as neighbours: in a smaller tree home is most of the tree and
-// the radius guessed from it means nothing. Everything else takes a warp per query
-// (clustered particles, k = 32, density: 2^20 3.0 ms here, 5.4 there; 1001 0.089 and 0.10;
-// 129 the same).
+// answers that FP32 offsets cannot tell apart, k within the buffers, squares inside FP32.
+// Below kGrpMin particles there are too few groups to fill the SMs with the warps that a group
+// needs one after another, and a warp per query ends sooner. (Density of clustered particles,
+// group and warp per query: 5,459 with k = 21 69 and 46 us; 20,001 with k = 32 179 and 149;
+// 32,769 with k = 8 128 and 145, k = 32 198 and 192, k = 64 273 and 278, uniform 98 and 178;
+// 65,537 with k = 32 302 and 346; 2^20 3.0 and 5.4 ms.)
+constexpr int kGrpMin = 32768;
 bool group_search_serves(const KnnArgs& a) {
   const int K = a.periodic ? a.kheap - 1 : a.kheap;
   return a.qmode == 0 && a.fb && (a.nq == a.tv.n || a.slices > 0) && a.kheap <= 128 && K >= 1 &&
-         a.tv.n >= 4 * (K + 1) && a.tv.eps < 1e11f &&
+         a.tv.n >= kGrpMin && a.tv.eps < 1e11f &&
          (a.periodic ? a.tv.n <= (1 << kGrpImage) : a.exclude_self != 0);
 }
 

@@ -59,6 +59,30 @@ def test_every_particle(gpu, port_built, kind, n, b, k):
     assert_density_close(t.CalcVelDensity(ns, k), o.veldensity(ns, k), f"veldensity {kind}")
 
 
+# from this many particles on every particle's search goes by groups
+LARGE = [("clustered", 32767, 16, 32), ("clustered", 32768, 5, 32), ("uniform", 32771, 1000, 40),
+         ("clustered", 40009, 16, 65), ("clustered", 32769, 8, 127), ("plane", 32771, 16, 32),
+         ("pairs", 32769, 16, 16), ("offset", 40009, 16, 64)]
+
+
+@pytest.mark.parametrize("kind,n,b,k", LARGE)
+def test_every_particle_large(gpu, port_built, kind, n, b, k):
+    test_every_particle(gpu, port_built, kind, n, b, k)
+
+
+@pytest.mark.parametrize("method,per,k", [(0, [1.0, 1.0, 1.0], 31), (1, [1.0, 1.0, 1.0], 64),
+                                          (0, [1.0, 0.25, 2.0], 32)])
+def test_periodic_rows_large(gpu, port_built, method, per, k):
+    n = 32771
+    pos = np.random.default_rng(17).random((n, 3)) * per
+    o = oracle.OracleTree(pos, None, np.ones(n), 16, 0, 0, 1000, per, backend="port", nthreads=8)
+    t = KDTree(pos, None, np.ones(n), 16, kerntype=0, period=per)
+    nn, d2 = (t.FindNearest if method == 0 else t.FindNearestPos)(k)
+    perm = t.GetPerm()
+    assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), *o.knn(k, method),
+                     f"method {method}, period {per}")
+
+
 @pytest.mark.parametrize("method", [0, 1])
 @pytest.mark.parametrize("n,b,k", [(500, 600, 32), (4097, 16, 31), (4097, 16, 32), (9001, 16, 64)])
 def test_periodic_rows(gpu, port_built, method, n, b, k):
