@@ -430,9 +430,9 @@ int nbk_batch_density_pertree_search(nbk_batch* batch, int k, double* rho);
    tune_json (NUL-terminated, up to cap bytes). (No reference counterpart.) */
 int nbk_batch_get_params(const nbk_batch* batch, int32_t* bucket_size, int32_t* query_bucket,
                          char* tune_json, int64_t cap);
-/* How the batched search maps queries to warps: 1 (the default) a warp serves one query
-   at a time (its k-list spread over the lanes' registers), 0 a lane serves one query and
-   a warp 32 queries of a bucket. The autotuner chooses it with the leaf and bucket sizes.
+/* How the batched search maps queries to warps: 1 (the default) a warp serves a group of
+   up to 8 neighbouring queries, one after another over one walk of the tree, 0 a lane
+   serves one query and a warp 32 queries of a bucket. The autotuner chooses it with the leaf and bucket sizes.
    (No reference counterpart.) */
 int nbk_batch_set_query_mapping(nbk_batch* batch, int warp_per_query);
 int nbk_batch_get_query_mapping(const nbk_batch* batch, int32_t* warp_per_query);

@@ -540,7 +540,7 @@ class BatchedDensity:
         return b.value, q.value, buf.value.decode()
 
     def query_mapping(self):
-        """1: a warp serves one query at a time; 0: a lane per query (32 per warp)."""
+        """1: a warp serves a group of neighbouring queries; 0: a lane per query (32 per warp)."""
         w = ctypes.c_int32()
         _capi.check(self._lib.nbk_batch_get_query_mapping(self._h, ctypes.byref(w)))
         return w.value
