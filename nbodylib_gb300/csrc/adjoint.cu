@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(128) k_adjoint(TreeView tv, int K, const int* 
   const double gi = g[ti], mi = xi.m;
   // farthest neighbour: the one that set h_i in the forward pass (the row's last entry)
   const int kf = row[K - 1];
+  if (kf < 0) return;  // too few neighbours, no row: reported by the search
   P4 xk = tv.pos[kf];
   const double best = dist2_exact(xi.x, xi.y, xi.z, xk.x, xk.y, xk.z);
   double irk;                                // 1 / r_iK

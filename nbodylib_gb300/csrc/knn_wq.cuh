@@ -609,7 +609,9 @@ __device__ __forceinline__ void wq_epilogue(const KnnArgs& a, const TreeView& tv
   for (int s = 0; s < S; s++) missing |= (s * 32 + lane < K) && L.idx[s] < 0;
   if (__any_sync(FULL, missing)) {
     if (lane == 0) atomicExch(a.err, kErrTooFew);
-    if (EPI == kEpiSave && lane == 0) a.nn[(size_t)qi * K + K - 1] = -1;  // no row
+    // no row: what reads the saved rows skips it
+    if (EPI == kEpiSave && lane == 0) a.nn[(size_t)qi * K + K - 1] = -1;
+    if (EPI == kEpiDensSave && lane == 0) a.nn[(size_t)(self - tv.pstart) * K + K - 1] = -1;
     return;
   }
   if (EPI == kEpiSave) {
