@@ -188,10 +188,8 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_link(FofArgs a) {
   float eps = tv.eps;
   // |sqrt(s) - d| <= e + 2^-21 d for the round-to-nearest s of a pair at distance d: each
   // coordinate difference is off by at most 2 eps, sqrt(3) of it in the distance
-  const float e = __fmul_ru(tv.eps, 3.4642f);
-  const float lf = __fadd_ru(__fsqrt_ru(thr), e), ln = __fsub_rd(__fsqrt_rd(ll2_lo), e);
-  const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 524288.0f);
-  const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 524288.0f) : 0.f;
+  const Band band = fp32_band(thr, ll2_lo, __fmul_ru(tv.eps, 3.4642f), 1.0f / 524288.0f);
+  const float far2 = band.far2, near2 = band.near2;
   int myroot = find_root(a.parent, self, a.err);  // cached; refreshed when it goes stale
   int npass = tv.periodic ? 8 : 1;
   int near = tv.periodic && valid ? near_walls(tv.posf[self], tv.period, eps, thr) : 0;
@@ -255,12 +253,12 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_link(FofArgs a) {
           const float dx = cf.x - qf.x, dy = cf.y - qf.y, dz = cf.z - qf.z;
           const float s = dx * dx + dy * dy + dz * dz;
           in = in && !(s >= far2);  // (a NaN is left to FP64)
-          const bool band = in && !(s < near2);
-          if (__any_sync(FULL, band)) {
+          const bool open = in && !(s < near2);
+          if (__any_sync(FULL, open)) {
             double xi[3];
 #pragma unroll
             for (int d = 0; d < 3; d++) xi[d] = __shfl_sync(FULL, xq[d], i);
-            if (band) {
+            if (open) {
               const P4 c = tv.pos[ti];
               if (CRIT3D) in = crit_cmp(0, a.params, xi, make_v4(0, 0, 0, 0), c, make_v4(0, 0, 0, 0));
               else in = dkey(dist2_exact(xi[0], xi[1], xi[2], c.x, c.y, c.z)) < ll2k;

@@ -1,0 +1,32 @@
+"""Links and balls at scales whose squares leave FP32's range (positions in centimetres or
+metres, or very small ones), where FP64 has to decide: the same answers as the restatement's
+or brute force, and the same as at scale one."""
+import numpy as np
+import pytest
+
+import oracle
+from nbodylib_gb300 import KDTree
+from nbodylib_gb300 import synthetic as syn
+from nbodylib_gb300.kdtree import FOF3D
+from tests.helpers import assert_same_partition
+
+pytestmark = pytest.mark.gpu
+
+SCALES = [1.0, 1e22, 1e18, 3e-16, 1e-20, 1e-22]
+
+
+@pytest.mark.parametrize("scale", SCALES)
+@pytest.mark.parametrize("periodic", [False, True])
+def test_fof(gpu, port_built, scale, periodic):
+    n, box = 3001, 20.0 * scale
+    pos, mass = syn.clustered_box(n, 20.0, seed=3, nspheres=20)
+    pos = pos * scale
+    per = [box] * 3 if periodic else None
+    ll = syn.linking_length(n, box)
+    o = oracle.OracleTree(pos, None, mass, 16, 0, 0, 1000, per, backend="port", nthreads=8)
+    t = KDTree(pos, None, mass, 16, kerntype=0, period=per)
+    for got, want in ((t.FOF(ll, 5), o.fof(ll, 5)),
+                      (t.FOFCriterion(FOF3D, [0, ll * ll, 0, 0, 0, 0, ll * ll, 0], 5),
+                       o.fof_criterion(0, [0, ll * ll, 0, 0, 0, 0, ll * ll, 0], 5))):
+        assert got[1] == want[1] > 0
+        assert_same_partition(got[0], want[0], f"scale {scale}")
