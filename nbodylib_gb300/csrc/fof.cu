@@ -603,9 +603,14 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_crit6_warp(FofArgs a) {
       e = __fadd_ru(e, __fmul_ru(__fmul_ru(w_hi[k], d), d));
     }
     e = __fsqrt_ru(e);
-    const float lf = __fadd_ru(thr_hi, e), ln = __fsub_rd(1.0f - 1.0f / 1048576.0f, e);
-    const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 262144.0f);
-    const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 262144.0f) : 0.f;
+    Band band = fp32_band(thr_hi, 1.0f - 1.0f / 1048576.0f, e, 1.0f / 262144.0f);
+    // s takes the weights rounded down: only where both ends of them are ordinary numbers is
+    // that a relative error too
+    if (!(fminf(w_lo[0], w_lo[3]) > 1e-30f && fmaxf(w_hi[0], w_hi[3]) < 1e30f)) {
+      band.far2 = __int_as_float(0x7fffffff);  // NaN
+      band.near2 = 0.f;
+    }
+    const float far2 = band.far2, near2 = band.near2;
     __syncwarp();
     int st = 0, ct = 0, pend = 0;
     unsigned mk = 0, m0 = 0, m1 = 0;
@@ -635,12 +640,12 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_crit6_warp(FofArgs a) {
 #pragma unroll
           for (int k = 0; k < 6; k++) s = fmaf(w_lo[k] * d[k], d[k], s);
           in = in && !(s >= far2);  // (a NaN is left to FP64)
-          const bool band = in && !(s < near2);
-          if (__any_sync(FULL, band)) {
+          const bool open = in && !(s < near2);
+          if (__any_sync(FULL, open)) {
             double xi[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) xi[k] = __shfl_sync(FULL, xq[k], i);
-            if (band) in = crit_cmp(2, a.params, xi, tv.vel[sq], tv.pos[ti], tv.vel[ti]);
+            if (open) in = crit_cmp(2, a.params, xi, tv.vel[sq], tv.pos[ti], tv.vel[ti]);
           }
           if (!__any_sync(FULL, in)) continue;
           if (in) {

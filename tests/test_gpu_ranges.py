@@ -7,7 +7,7 @@ import pytest
 import oracle
 from nbodylib_gb300 import KDTree
 from nbodylib_gb300 import synthetic as syn
-from nbodylib_gb300.kdtree import FOF3D
+from nbodylib_gb300.kdtree import FOF3D, FOF6D
 from tests.helpers import assert_same_partition
 
 pytestmark = pytest.mark.gpu
@@ -30,3 +30,21 @@ def test_fof(gpu, port_built, scale, periodic):
                        o.fof_criterion(0, [0, ll * ll, 0, 0, 0, 0, ll * ll, 0], 5))):
         assert got[1] == want[1] > 0
         assert_same_partition(got[0], want[0], f"scale {scale}")
+
+
+@pytest.mark.parametrize("length,speed", [(1.0, 1.0), (1e22, 1.0), (1e22, 1e7), (1.0, 1e22),
+                                          (1e-20, 1.0), (1.0, 1e-20), (1e-20, 1e20)])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_fof6d(gpu, port_built, length, speed, periodic):
+    n = 2001
+    pos, mass, vel = syn.clustered_box(n, 20.0, seed=3, nspheres=20, velocities=True)
+    pos, vel, box = pos * length, vel * speed, 20.0 * length
+    per = [box] * 3 if periodic else None
+    ll = syn.linking_length(n, box)
+    p = [0, ll * ll, 0, 0, 0, 0, ll * ll, 0.04 * speed * speed]
+    o = oracle.OracleTree(pos, vel, mass, 16, 0, 0, 1000, per, backend="port", nthreads=8)
+    t = KDTree(pos, vel, mass, 16, kerntype=0, period=per)
+    g, ng = t.FOFCriterion(FOF6D, p, 5)
+    go, ngo = o.fof_criterion(2, p, 5)
+    assert ng == ngo > 0
+    assert_same_partition(g, go, f"length {length}, speed {speed}")
