@@ -93,10 +93,9 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_ball(BallArgs a) {
   // coordinate differences are off by eps + tv.eps each; the warp's largest)
   float e = eps;
   for (int o = 16; o > 0; o >>= 1) e = fmaxf(e, __shfl_xor_sync(FULL, e, o));
-  e = __fmul_ru(__fadd_ru(e, tv.eps), 1.7321f);
-  const float lf = __fadd_ru(__fsqrt_ru(thr), e), ln = __fsub_rd(__fsqrt_rd(r2_lo), e);
-  const float far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + 1.0f / 524288.0f);
-  const float near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - 1.0f / 524288.0f) : 0.f;
+  const Band band = fp32_band(thr, r2_lo, __fmul_ru(__fadd_ru(e, tv.eps), 1.7321f),
+                              1.0f / 524288.0f);
+  const float far2 = band.far2, near2 = band.near2;
   const int npass = tv.periodic ? 8 : 1;
   int near = 0;
   if (tv.periodic && valid)
@@ -165,15 +164,19 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_ball(BallArgs a) {
       sp -= m;
       const bool leaf = r.count <= tv.b;
       if (strict) {
-        // a lane per node, as far as a hit of any query can be (see far2)
+        // a lane per node: whether any query's ball reaches its box (widened by the largest
+        // rounding of the warp's queries)
+        const float lx = __fsub_rd(r.lo[0], e), hx = __fadd_ru(r.hi[0], e);
+        const float ly = __fsub_rd(r.lo[1], e), hy = __fadd_ru(r.hi[1], e);
+        const float lz = __fsub_rd(r.lo[2], e), hz = __fadd_ru(r.hi[2], e);
         bool reach = false;
 #pragma unroll 1
         for (unsigned qm = __ballot_sync(FULL, active); qm; qm &= qm - 1) {
           const float4 qf = w.q[__ffs(qm) - 1];
-          const float gx = fmaxf(0.f, fmaxf(r.lo[0] - qf.x, qf.x - r.hi[0]));
-          const float gy = fmaxf(0.f, fmaxf(r.lo[1] - qf.y, qf.y - r.hi[1]));
-          const float gz = fmaxf(0.f, fmaxf(r.lo[2] - qf.z, qf.z - r.hi[2]));
-          reach = reach || !(gx * gx + gy * gy + gz * gz >= far2);
+          const float gx = fmaxf(0.f, fmaxf(__fsub_rd(lx, qf.x), __fsub_rd(qf.x, hx)));
+          const float gy = fmaxf(0.f, fmaxf(__fsub_rd(ly, qf.y), __fsub_rd(qf.y, hy)));
+          const float gz = fmaxf(0.f, fmaxf(__fsub_rd(lz, qf.z), __fsub_rd(qf.z, hz)));
+          reach = reach || __fmaf_rd(gz, gz, __fmaf_rd(gy, gy, __fmul_rd(gx, gx))) < thr;
         }
         keep = keep && reach;
       }
@@ -248,13 +251,13 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_ball(BallArgs a) {
             bool in = ok && ((mk >> i) & 1u) && !(s >= far2);
             const int si = __shfl_sync(FULL, self, i);
             if (a.exclude_self && pass == 0) in = in && ti != si;
-            const bool band = in && (!(s < near2) || (FILL && a.outd2));
+            const bool open = in && (!(s < near2) || (FILL && a.outd2));
             double d2 = 0.0;
-            if (__any_sync(FULL, band)) {
+            if (__any_sync(FULL, open)) {
               double xi[3];
 #pragma unroll
               for (int d = 0; d < 3; d++) xi[d] = __shfl_sync(FULL, xq[d], i);
-              if (band) {
+              if (open) {
                 const P4 c = tv.pos[ti];
                 d2 = dist2_exact(xi[0], xi[1], xi[2], c.x, c.y, c.z);
                 in = dkey(d2) < r2k;  // d2 < r2

@@ -8,7 +8,7 @@ import oracle
 from nbodylib_gb300 import KDTree
 from nbodylib_gb300 import synthetic as syn
 from nbodylib_gb300.kdtree import FOF3D, FOF6D
-from tests.helpers import assert_same_partition
+from tests.helpers import assert_same_partition, d2_ref, reflect_images
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +48,31 @@ def test_fof6d(gpu, port_built, length, speed, periodic):
     go, ngo = o.fof_criterion(2, p, 5)
     assert ng == ngo > 0
     assert_same_partition(g, go, f"length {length}, speed {speed}")
+
+
+@pytest.mark.parametrize("scale", SCALES)
+@pytest.mark.parametrize("periodic", [False, True])
+def test_ball(gpu, scale, periodic):
+    """Rows of a few targets, and of all of them in random order (balls all over the box)."""
+    n = 5003
+    pos, mass = syn.clustered_box(n, 1.0, seed=9, nspheres=6)
+    pos = pos * scale
+    per = [scale] * 3 if periodic else None
+    t = KDTree(pos, None, mass, 16, kerntype=0, period=per)
+    tree = pos[t.GetPerm()]
+    order = np.random.default_rng(1).permutation(n).astype(np.int32)
+    for r in (0.01 * scale, 0.06 * scale):
+        off, idx = t.SearchBallPosTagged(order, r * r)
+        few, fidx = t.SearchBallPosTagged(order[:3], r * r)
+        assert np.array_equal(few, off[:4]) and np.array_equal(fidx, idx[:few[3]])
+        for i in range(0, n, 7):
+            x = tree[order[i]]
+            want = []
+            for p, y in enumerate(reflect_images(x[None], per)[:, 0] if periodic else x[None]):
+                if p:  # an image is searched when its wall distance is inside the radius
+                    s = np.where(x < 0.5 * scale, x, scale - x)[y != x]
+                    if not (r * r > (np.abs(s[0]) if s.size == 1 else np.sqrt((s * s).sum())) ** 2):
+                        continue
+                hit = np.nonzero(d2_ref(y, tree) < r * r)[0]
+                want += [j for j in hit if periodic or j != order[i]]
+            assert idx[off[i]:off[i + 1]].tolist() == want, (r, i)
