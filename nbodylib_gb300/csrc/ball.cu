@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_ball(BallArgs a) {
   // coordinate differences are off by eps + tv.eps each; the warp's largest)
   float e = eps;
   for (int o = 16; o > 0; o >>= 1) e = fmaxf(e, __shfl_xor_sync(FULL, e, o));
-  const Band band = fp32_band(thr, r2_lo, __fmul_ru(__fadd_ru(e, tv.eps), 1.7321f),
-                              1.0f / 524288.0f);
+  const Band band = fp32_band(__fsqrt_ru(thr), __fsqrt_rd(r2_lo),
+                              __fmul_ru(__fadd_ru(e, tv.eps), 1.7321f), 1.0f / 524288.0f);
   const float far2 = band.far2, near2 = band.near2;
   const int npass = tv.periodic ? 8 : 1;
   int near = 0;
@@ -164,19 +164,16 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_ball(BallArgs a) {
       sp -= m;
       const bool leaf = r.count <= tv.b;
       if (strict) {
-        // a lane per node: whether any query's ball reaches its box (widened by the largest
-        // rounding of the warp's queries)
-        const float lx = __fsub_rd(r.lo[0], e), hx = __fadd_ru(r.hi[0], e);
-        const float ly = __fsub_rd(r.lo[1], e), hy = __fadd_ru(r.hi[1], e);
-        const float lz = __fsub_rd(r.lo[2], e), hz = __fadd_ru(r.hi[2], e);
+        // a lane per node, as far as a hit of any query can be (see far2; outside
+        // FP32's range every node)
         bool reach = false;
 #pragma unroll 1
         for (unsigned qm = __ballot_sync(FULL, active); qm; qm &= qm - 1) {
           const float4 qf = w.q[__ffs(qm) - 1];
-          const float gx = fmaxf(0.f, fmaxf(__fsub_rd(lx, qf.x), __fsub_rd(qf.x, hx)));
-          const float gy = fmaxf(0.f, fmaxf(__fsub_rd(ly, qf.y), __fsub_rd(qf.y, hy)));
-          const float gz = fmaxf(0.f, fmaxf(__fsub_rd(lz, qf.z), __fsub_rd(qf.z, hz)));
-          reach = reach || __fmaf_rd(gz, gz, __fmaf_rd(gy, gy, __fmul_rd(gx, gx))) < thr;
+          const float gx = fmaxf(0.f, fmaxf(r.lo[0] - qf.x, qf.x - r.hi[0]));
+          const float gy = fmaxf(0.f, fmaxf(r.lo[1] - qf.y, qf.y - r.hi[1]));
+          const float gz = fmaxf(0.f, fmaxf(r.lo[2] - qf.z, qf.z - r.hi[2]));
+          reach = reach || !(gx * gx + gy * gy + gz * gz >= far2);
         }
         keep = keep && reach;
       }

@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(32 * kWpb, 10) k_link(FofArgs a) {
   float eps = tv.eps;
   // |sqrt(s) - d| <= e + 2^-21 d for the round-to-nearest s of a pair at distance d: each
   // coordinate difference is off by at most 2 eps, sqrt(3) of it in the distance
-  const Band band = fp32_band(thr, ll2_lo, __fmul_ru(tv.eps, 3.4642f), 1.0f / 524288.0f);
+  const Band band = fp32_band(__fsqrt_ru(thr), __fsqrt_rd(ll2_lo), __fmul_ru(tv.eps, 3.4642f),
+                              1.0f / 524288.0f);
   const float far2 = band.far2, near2 = band.near2;
   int myroot = find_root(a.parent, self, a.err);  // cached; refreshed when it goes stale
   int npass = tv.periodic ? 8 : 1;
@@ -602,14 +603,9 @@ __global__ void __launch_bounds__(32 * kWpb, 8) k_crit6_warp(FofArgs a) {
       d = __fadd_ru(d, tv.eps6[k]);
       e = __fadd_ru(e, __fmul_ru(__fmul_ru(w_hi[k], d), d));
     }
-    e = __fsqrt_ru(e);
-    Band band = fp32_band(thr_hi, 1.0f - 1.0f / 1048576.0f, e, 1.0f / 262144.0f);
-    // s takes the weights rounded down: only where both ends of them are ordinary numbers is
-    // that a relative error too
-    if (!(fminf(w_lo[0], w_lo[3]) > 1e-30f && fmaxf(w_hi[0], w_hi[3]) < 1e30f)) {
-      band.far2 = __int_as_float(0x7fffffff);  // NaN
-      band.near2 = 0.f;
-    }
+    // (s takes the weights rounded down, a relative error only where they are normal floats)
+    e = a.fp32_weights ? __fsqrt_ru(e) : FLT_MAX;
+    const Band band = fp32_band(thr_hi, 1.0f - 1.0f / 1048576.0f, e, 1.0f / 262144.0f);
     const float far2 = band.far2, near2 = band.near2;
     __syncwarp();
     int st = 0, ct = 0, pend = 0;
@@ -1033,6 +1029,11 @@ int queries_per_warp(int64_t n, int* qpw) {
   return NBK_OK;
 }
 
+// Whether the FOF6d weights 1 / params[6] and 1 / params[7] are far inside FP32's range.
+static int fof6d_weights_in_fp32(const double* p) {
+  return p[6] > 1e-30 && p[6] < 1e30 && p[7] > 1e-30 && p[7] < 1e30;
+}
+
 // FOF6d inside its search region on a physical tree (see k_crit6_warp): builds the
 // phase-space tree of the same particles, links on it, and unites the physical tree's
 // parent forest accordingly.
@@ -1133,6 +1134,7 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
   }
   NBK_TRY(queries_per_warp(n, &f.qpw));
   const int warps = (n + f.qpw - 1) / f.qpw;
+  f.fp32_weights = fof6d_weights_in_fp32(a.params);
   if (a.crit == 2) {
     Phase ph("fof_nn_link", st);
     k_nn_link<<<(n + 255) / 256, 256, 0, st>>>(a); note_launch();
@@ -1148,7 +1150,7 @@ int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tr
     NBK_CUDA_TRY(launch_chain(k_link<true>, (warps + kWpb - 1) / kWpb, 32 * kWpb, 0, st, f));
   } else if (a.crit && a.crit_contained && a.cmp == 2) {
     Phase ph("fof_criterion_link", st);
-    NBK_TRY(link_fof6d_phase_tree(a, alloc, st));
+    NBK_TRY(link_fof6d_phase_tree(f, alloc, st));
   } else if (a.crit) {
     Phase ph("fof_criterion_link", st);
     k_crit_link<<<(n + 127) / 128, 128, 0, st>>>(a); note_launch();

@@ -244,6 +244,7 @@ struct FofArgs {
                        //   region (FOF3d / FOF6d with params[6] <= the position search
                        //   distance^2), so reachability follows from the comparator
   int qpw;             // queries per warp of the link kernels (set by run_fof)
+  int fp32_weights;    // FOF6d: the weights are normal FP32 numbers (set by run_fof)
 };
 int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tree,
             int* h_ngroup, DevAlloc& alloc, cudaStream_t st,

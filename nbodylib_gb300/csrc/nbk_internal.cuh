@@ -208,25 +208,22 @@ __device__ __forceinline__ float thresh_lo(double t) {
 }
 
 // Decisions on a round-to-nearest FP32 square s of a length or scaled sum t: with
-// |sqrt(s) - t| <= e + m t / 2, s >= far2 proves t^2 at or above the threshold (hi is an FP32
+// |sqrt(s) - t| <= e + m t / 2, s >= far2 proves t at or above the threshold (hi is an FP32
 // value at or above it), s < near2 proves it below (lo is one at or below it), and what lies
 // between is left to FP64. That bound is relative, so it holds only where no square leaves
 // FP32's range: a threshold outside it (positions in metres or centimetres, or very small
-// ones) gives a far2 that nothing reaches and a near2 of zero, and FP64 decides every pair.
-// (Directed rounding needed no such case: its overflows and underflows stay bounds.)
+// ones) or an e beyond it gives a far2 of NaN, which nothing reaches, and a near2 of zero, and
+// FP64 decides every pair. (Directed rounding needed no such case: its overflows and
+// underflows stay bounds.)
 struct Band {
   float near2, far2;
 };
 __device__ __forceinline__ Band fp32_band(float hi, float lo, float e, float m) {
-  const float lf = __fadd_ru(__fsqrt_ru(hi), e), ln = __fsub_rd(__fsqrt_rd(lo), e);
+  if (!(lo > 1e-15f && hi < 1e14f && e < 1e14f)) e = __int_as_float(0x7fffffff);  // NaN
+  const float lf = __fadd_ru(hi, e), ln = __fsub_rd(lo, e);
   Band b;
   b.far2 = __fmul_ru(__fmul_ru(lf, lf), 1.0f + m);
-  b.near2 = ln > 0.f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - m) : 0.f;
-  if (!(lo > 1e-30f && b.far2 < 1e30f)) {
-    b.far2 = __int_as_float(0x7fffffff);  // NaN
-    b.near2 = 0.f;
-  }
-  if (b.near2 < 1e-30f) b.near2 = 0.f;
+  b.near2 = ln > 1e-15f ? __fmul_rd(__fmul_rd(ln, ln), 1.0f - m) : 0.f;
   return b;
 }
 
