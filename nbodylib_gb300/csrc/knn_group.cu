@@ -423,7 +423,7 @@ __device__ void grp_search(GrpSmem<S>& w, const TreeView& tv, int lane, int g, i
     ge.reach = grp_thresh(r * r, two_e);
     if (L.act) {
       L.cnt = 0;
-      L.thr = r * r;
+      L.thr = fminf(r * r, FLT_MAX);
       w.qs[lane] = make_float4(L.x, L.y, L.z, L.thr);
     }
     __syncwarp();

@@ -89,7 +89,9 @@ __device__ __noinline__ GrpCut grp_tighten(unsigned* bs, int* bi, int lane, int 
     } else {
       lo = mid + 1;
     }
-    pv = 0.5f * (__uint_as_float(lo) + __uint_as_float(hi));
+    // halved before the sum: between squares near FP32's end the pivot would be infinite and
+    // each step one unit in the last place
+    pv = 0.5f * __uint_as_float(lo) + 0.5f * __uint_as_float(hi);
   }
   unsigned kth = 0u;
 #pragma unroll
@@ -100,7 +102,8 @@ __device__ __noinline__ GrpCut grp_tighten(unsigned* bs, int* bi, int lane, int 
     out.thr = -1.f;
     return out;
   }
-  out.thr = grp_thresh(__uint_as_float(kth), two_e);
+  // finite: an infinite square among the entries would do the same
+  out.thr = fminf(grp_thresh(__uint_as_float(kth), two_e), FLT_MAX);
   if (cnt == K) return out;
   const unsigned tb = __float_as_uint(out.thr);
   int id[R], n = 0;

@@ -1,0 +1,36 @@
+"""Phase-space searches whose metric takes squares to the ends of FP32's range."""
+import numpy as np
+import pytest
+
+import oracle
+from nbodylib_gb300 import KDTree
+from nbodylib_gb300.kdtree import KSPH, TPHS
+from tests.helpers import assert_knn_equal, rows_by_id, to_ids
+
+pytestmark = pytest.mark.gpu
+
+
+def assert_rows_equal(pos, vel, b, k, aniso):
+    n = len(pos)
+    o = oracle.OracleTree(pos, vel, np.ones(n), b, TPHS, 0, 1000, None, backend="port",
+                          nthreads=8, aniso=aniso)
+    t = KDTree(pos, vel, np.ones(n), b, treetype=TPHS, kerntype=KSPH, aniso=aniso)
+    perm = t.GetPerm()
+    nn, d2 = t.FindNearest(k)
+    t.close()
+    oi, od = o.knn(k, 0)
+    assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), oi, od)
+    return d2
+
+
+@pytest.mark.parametrize("k", [8, 32, 40])
+def test_squares_near_the_largest_float(gpu, port_built, k):
+    """Two particles 2e-15 apart in one coordinate weigh it with 2.5e29: the others, at
+    2.8e4 to 3.6e4 in it, are at squared distances of 2e38 to 3.3e38 from them."""
+    rng = np.random.default_rng(7)
+    pos, vel = rng.random((2001, 3)) * 10.0, rng.random((2001, 3)) * 10.0
+    pos[:, 0] = rng.uniform(2.8e4, 3.6e4, 2001)
+    pos[0, 0], pos[1, 0] = 0.0, 2e-15
+    pos[1, 1:], vel[1] = pos[0, 1:] + 0.1, vel[0] + 0.1
+    d2 = assert_rows_equal(pos, vel, 16, k, 0)
+    assert (d2 == 1e32).sum() >= 2 * (k - 1)  # farther than the searches go
