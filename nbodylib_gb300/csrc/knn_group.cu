@@ -24,9 +24,10 @@
 // A query that this cannot answer exactly -- fewer than K particles within the radius, a
 // candidate not provably at a non-zero distance (the target search skips zero distances,
 // KDLeafNode.cxx:19-21), more candidates than the buffer holds within the rounding of the
-// K-th, distances outside the FP32 range, a periodic query too close to an image gate --
-// and every query of a group whose box meets too many particles is appended to a list that
-// a second launch serves with the warp-per-query search.
+// K-th, distances outside the FP32 range or not surely below the reference's MAXVALUE, a
+// periodic query too close to an image gate -- and every query of a group whose box meets too
+// many particles is appended to a list that a second launch serves with the warp-per-query
+// search.
 //
 // The FP64 pipe (two operations per SM clock: 16 cycles a warp instruction) is the bound of
 // the density sums. Per neighbour 13 FP64 instructions are left: 6 for the distance (fused;

@@ -7,6 +7,9 @@ namespace nbk {
 namespace {
 
 constexpr int kGrpSlack = 3;  // entries beyond the K-th a buffer cut may leave
+// The reference's lists start with squared distances of kMaxValue and take nothing at or
+// beyond it: a query whose K-th bound is not surely below is left to a search with such a list.
+constexpr float kGrpFarthest = 0.99999e32f;
 
 // S slots of 32 neighbours: K <= 32 S. Groups shrink as the buffers grow, so that a warp's
 // shared memory stays near 6 KB.
@@ -44,7 +47,7 @@ __device__ __forceinline__ float grp_thresh(float s, float two_e) {
 }
 
 struct GrpCut {
-  float thr;   // bound of the cut (-1: the FP32 range does not resolve the distances)
+  float thr;   // bound of the cut (-1: FP32 does not resolve the distances, or kGrpFarthest)
   float smin;  // the smallest squared distance
   int cnt;     // entries left
 };
@@ -98,12 +101,11 @@ __device__ __noinline__ GrpCut grp_tighten(unsigned* bs, int* bi, int lane, int 
   for (int t = 0; t < R; t++)
     if (r[t] <= hi) kth = max(kth, r[t]);
   kth = __reduce_max_sync(FULL, kth);
-  if (kth < 0x0da24260u || kth >= 0x7e000000u) {  // below 1e-30, near overflow
+  out.thr = grp_thresh(__uint_as_float(kth), two_e);
+  if (kth < 0x0da24260u || !(out.thr <= kGrpFarthest)) {  // below 1e-30, beyond kMaxValue
     out.thr = -1.f;
     return out;
   }
-  // finite: an infinite square among the entries would do the same
-  out.thr = fminf(grp_thresh(__uint_as_float(kth), two_e), FLT_MAX);
   if (cnt == K) return out;
   const unsigned tb = __float_as_uint(out.thr);
   int id[R], n = 0;

@@ -34,3 +34,11 @@ def test_squares_near_the_largest_float(gpu, port_built, k):
     pos[1, 1:], vel[1] = pos[0, 1:] + 0.1, vel[0] + 0.1
     d2 = assert_rows_equal(pos, vel, 16, k, 0)
     assert (d2 == 1e32).sum() >= 2 * (k - 1)  # farther than the searches go
+
+
+@pytest.mark.parametrize("box", [1e15, 2.5e17])
+def test_particles_farther_than_the_search_goes(gpu, port_built, box):
+    """Lists start at squared distances of 1e32 and take nothing there or beyond."""
+    rng = np.random.default_rng(9)
+    d2 = assert_rows_equal(rng.random((3001, 3)) * box, rng.random((3001, 3)), 16, 32, -1)
+    assert (d2 == 1e32).any() == (box > 1e17)
