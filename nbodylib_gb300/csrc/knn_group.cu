@@ -245,15 +245,17 @@ __device__ __forceinline__ bool grp_wanted(GrpSmem<S>& w, const GrpGeom& ge, Grp
 
 // Distance within which a box of extents e (sorted or not) with n particles is expected to
 // hold K of them, taken as the largest of the line, square and cube estimates (the cube's
-// unless the box is flat or thin).
+// unless the box is flat or thin). From logarithms: products of extents leave FP32's range
+// where the extents are far inside it.
 __device__ __forceinline__ float grp_radius(float ex, float ey, float ez, int n, int K) {
   const float a = fmaxf(ex, fmaxf(ey, ez)), c = fminf(ex, fminf(ey, ez));
   const float b = fmaxf(fminf(ex, ey), fminf(fmaxf(ex, ey), ez));
-  const float f = __fdividef((float)K, (float)n);
-  const float r1 = 0.5f * f * a;
-  const float r2 = sqrtf(f * a * b * 0.31831f);
-  const float r3 = exp2f(log2f(f * a * b * c * 0.23873f) * (1.0f / 3.0f));
-  return fmaxf(r1, fmaxf(r2, r3));
+  const float f = log2f(__fdividef((float)K, (float)n));
+  const float la = log2f(a), lb = log2f(b), lc = log2f(c);  // -inf where flat
+  const float r1 = f + la - 1.f;
+  const float r2 = (f + la + lb - 1.6515f) * 0.5f;                    // 1 / pi
+  const float r3 = (f + la + lb + lc - 2.0665f) * (1.0f / 3.0f);     // 3 / (4 pi)
+  return exp2f(fmaxf(r1, fmaxf(r2, r3)));
 }
 
 // One walk of the tree for the active queries: first home itself and the siblings of home
