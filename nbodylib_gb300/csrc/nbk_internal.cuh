@@ -296,11 +296,13 @@ __device__ __forceinline__ double wsm_line(double q, int size, double inv_delta,
 }
 
 // W at the table coordinate u = q (size - 1) / 2 from the image's sections A and D: on cell
-// i = (int)u the line is A[i] + D[i] u. The cell comes from the bits of u (u < 2^20).
+// i = (int)u the line is A[i] + D[i] u. The cell comes from the top 32 bits of u's
+// significand (any u below 2^31, so any table; an infinite or NaN u is past the last cell).
 __device__ __forceinline__ double w_at_u(double u, int size, const double* img) {
   const int hi = __double2hiint(u), e = (hi >> 20) - 1023;
-  const int i = e < 0 ? 0 : ((hi & 0xfffff) | 0x100000) >> max(20 - e, 0);
-  if (i < size - 1) return __fma_rn(img[3 * size + i], u, img[size + i]);
+  const unsigned m = __funnelshift_l((unsigned)__double2loint(u), (unsigned)hi, 11) | 0x80000000u;
+  const unsigned i = e < 0 ? 0u : m >> max(31 - e, 0);
+  if (i < (unsigned)(size - 1)) return __fma_rn(img[3 * (size_t)size + i], u, img[(size_t)size + i]);
   return img[size - 1];
 }
 
