@@ -250,8 +250,8 @@ __device__ __forceinline__ bool grp_wanted(GrpSmem<S>& w, const GrpGeom& ge, Grp
 __device__ __forceinline__ float grp_radius(float ex, float ey, float ez, int n, int K) {
   const float a = fmaxf(ex, fmaxf(ey, ez)), c = fminf(ex, fminf(ey, ez));
   const float b = fmaxf(fminf(ex, ey), fminf(fmaxf(ex, ey), ez));
-  const float f = log2f(__fdividef((float)K, (float)n));
-  const float la = log2f(a), lb = log2f(b), lc = log2f(c);  // -inf where flat
+  const float f = __log2f(__fdividef((float)K, (float)n));
+  const float la = __log2f(a), lb = __log2f(b), lc = __log2f(c);  // -inf where flat
   const float r1 = f + la - 1.f;
   const float r2 = (f + la + lb - 1.6515f) * 0.5f;                    // 1 / pi
   const float r3 = (f + la + lb + lc - 2.0665f) * (1.0f / 3.0f);     // 3 / (4 pi)
