@@ -725,6 +725,7 @@ __device__ void grp_periodic(const KnnArgs& a, GrpSmem<S>& w, int lane, int g, i
   };
   cut((1u << gn) - 1u, true);
   const bool mine = (okm >> lane) & 1u;
+  float slack = 2.f * two_e;  // a bound's root is at most this and 2^-16 above the K-th distance
   double x0[3] = {0, 0, 0};
   int near_sq = 0, near_lin = 0;
   if (mine) {
@@ -747,7 +748,7 @@ __device__ void grp_periodic(const KnnArgs& a, GrpSmem<S>& w, int lane, int g, i
     const float sv = __double2float_rn(reflect(x0, xp, tv.period, mk));
     // the K-th distance is between lo and hi
     const float hi = __fsqrt_ru(L.thr);
-    const float lo = fmaxf(0.f, hi * (1.0f - 1.0f / 65536.0f) - 2.f * two_e);
+    const float lo = fmaxf(0.f, hi * (1.0f - 1.0f / 65536.0f) - slack);
     const float t1 = lin ? lo * lo : lo, t2 = lin ? L.thr : hi;
     const float m = fabsf(sv) * 1e-6f;
     const bool surely = t1 > sv + m, never = t2 < sv - m;
@@ -774,8 +775,16 @@ __device__ void grp_periodic(const KnnArgs& a, GrpSmem<S>& w, int lane, int g, i
     }
     const float far = __uint_as_float(__reduce_max_sync(
         FULL, open ? __float_as_uint(fmaxf(fabsf(L.x), fmaxf(fabsf(L.y), fabsf(L.z)))) : 0u));
-    two_e = fmaxf(two_e, __fmul_ru(4.f, __fadd_ru(__fmul_ru(far, 1.f / 4194304.f),
-                                                     __fmul_ru(tv.eps, 1.f / 524288.f))));
+    const float here = __fmul_ru(4.f, __fadd_ru(__fmul_ru(far, 1.f / 4194304.f),
+                                                __fmul_ru(tv.eps, 1.f / 524288.f)));
+    if (here > two_e) {
+      // these offsets are rounded more than those the bounds were formed with: the bounds
+      // widen by as much, and so does what lies between them and the K-th distances
+      two_e = here;
+      slack = __fadd_ru(slack, 2.f * two_e);
+      L.thr = grp_thresh(L.thr, two_e);
+      if (open) w.qs[lane].w = L.thr;
+    }
     grp_box<S>(ge, open, p, __fmul_ru(2.f, tv.eps));
     const float wide = __uint_as_float(__reduce_max_sync(FULL, open ? __float_as_uint(L.thr) : 0u));
     ge.reach = grp_thresh(wide, two_e);
