@@ -41,7 +41,7 @@ struct nbk_batch {
   double* d_mass_in = nullptr;
   bool own_inputs = false;
   TreeInfo* d_trees = nullptr;
-  WorkItem* d_items = nullptr;  // lane-per-query form only: made at its first use
+  WorkItem* d_items = nullptr;  // lane-per-query form only: made when that is chosen
   int nitems = 0;
   int* d_goff = nullptr;    // first search group of each tree for groups of 8, 4, 2; pstart
   int ntrees = 0;           // non-empty trees (the entries of d_trees)
@@ -160,7 +160,7 @@ int make_items(nbk_batch* B) {
   return NBK_OK;
 }
 
-// Another query-bucket size: its items are made at the next lane-per-query search.
+// Another query-bucket size (the autotuner's; the next lane-per-query search makes its items).
 void set_query_bucket(nbk_batch* B, int qb) {
   B->qb = qb;
   dev_free(B->d_items, B->st);
@@ -223,7 +223,8 @@ int batch_build(nbk_batch* B, int b) {
   for (auto& t : B->trees)
     if (t.n > 0) nonempty.push_back(t);
   NBK_TRY(build_forest(nonempty, b, B->d_pos_in, B->d_mass_in, nullptr, B->arr, alloc, st));
-  return NBK_OK;  // the build has synchronised the stream: the host arrays may go
+  // (the build has synchronised the stream: the host arrays may go)
+  return B->wpq ? NBK_OK : make_items(B);
 }
 
 KnnArgs batch_args(nbk_batch* B, int k) {
@@ -532,8 +533,12 @@ int nbk_batch_set_query_mapping(nbk_batch* B, int warp_per_query) {
     set_error("nbk_batch_set_query_mapping: null batch or mapping other than 0 / 1");
     return NBK_ERR_INVALID;
   }
+  BAPI_BEGIN
+  // made here and not by the first search, which may be recorded into a caller's graph
+  if (!warp_per_query) NBK_TRY(make_items(B));
   B->wpq = warp_per_query;
   return NBK_OK;
+  BAPI_END
 }
 
 int nbk_batch_get_query_mapping(const nbk_batch* B, int32_t* warp_per_query) {
