@@ -10,7 +10,7 @@ from tests.helpers import assert_knn_equal, rows_by_id, to_ids
 pytestmark = pytest.mark.gpu
 
 
-def assert_rows_equal(pos, vel, b, k, aniso):
+def assert_rows_equal(pos, vel, b, k, aniso, rows=slice(None)):
     n = len(pos)
     o = oracle.OracleTree(pos, vel, np.ones(n), b, TPHS, 0, 1000, None, backend="port",
                           nthreads=8, aniso=aniso)
@@ -19,7 +19,8 @@ def assert_rows_equal(pos, vel, b, k, aniso):
     nn, d2 = t.FindNearest(k)
     t.close()
     oi, od = o.knn(k, 0)
-    assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), oi, od)
+    assert_knn_equal(rows_by_id(to_ids(nn, perm), perm)[rows], rows_by_id(d2, perm)[rows],
+                     oi[rows], od[rows])
     return d2
 
 
@@ -42,3 +43,32 @@ def test_particles_farther_than_the_search_goes(gpu, port_built, box):
     rng = np.random.default_rng(9)
     d2 = assert_rows_equal(rng.random((3001, 3)) * box, rng.random((3001, 3)), 16, 32, -1)
     assert (d2 == 1e32).any() == (box > 1e17)
+
+
+@pytest.mark.parametrize("n", [2001, 9001])
+def test_queries_without_a_resolved_spacing(gpu, port_built, n):
+    """Twelve particles within 1e-16 of one another, whose plain distances FP32 does not
+    resolve, take the search of a lane each. (A particle whose nearest they are has a metric
+    only if their distances to it do not tie exactly: which one it is taken from is open.)"""
+    rng = np.random.default_rng(11)
+    pos, vel = rng.normal(size=(n, 3)), rng.normal(size=(n, 3))
+    pos[:12], vel[:12] = rng.normal(size=(12, 3)) * 1e-16, rng.normal(size=(12, 3)) * 1e-16
+    x = np.concatenate([pos, vel], axis=1)
+    near = [np.partition(((x - y) ** 2).cumsum(axis=1)[:, 5], (1, 2))[1:3] for y in x]
+    rows = np.array([a != b for a, b in near])
+    assert rows[:12].all() and rows.sum() > n - 5
+    for k in (8, 16):
+        assert_rows_equal(pos, vel, 16, k, 0, rows)
+
+
+def test_more_leftovers_than_their_list_holds(gpu, port_built):
+    """Two of three particles beside one another at 1e-7 in one coordinate: FP32 resolves none
+    of their metrics, and the list of those (an eighth of the particles) is full."""
+    n = 12001
+    rng = np.random.default_rng(13)
+    pos, vel = rng.normal(size=(n, 3)), rng.normal(size=(n, 3))
+    i = np.arange(0, n - 1, 3)
+    pos[i + 1] = pos[i] + rng.normal(size=(i.size, 3)) * 0.01
+    pos[i + 1, 0] = pos[i, 0] + 1e-7
+    vel[i + 1] = vel[i] + rng.normal(size=(i.size, 3)) * 0.01
+    assert_rows_equal(pos, vel, 16, 16, 0)
