@@ -1,12 +1,12 @@
-// Warp-cooperative k-nearest-neighbour search of the batched density's lane-per-query mapping
-// (k_knn_batch, knn.cu).
+// Warp-cooperative k-nearest-neighbour search, a lane per query: the batched density's
+// lane-per-query mapping (k_knn_batch, knn.cu) and points near one another (k_knn_points).
 //
 // Replaces the recursive depth-first search of SplitNode/LeafNode::FindNearestPos
 // (src/KDTree/KDSplitNode.cxx:15-41, 206-231; KDLeafNode.cxx:15-28, 119-130) and its
 // periodic wrapper (KDSplitNode.cxx:1119-1147).
 //
-// Work mapping (the other mapping, a warp per group of particles, is knn_group.cu; the
-// batch's autotuner times both): one warp serves 32 queries that are consecutive in tree order, so they
+// Work mapping (the batch's other mapping, a warp per group of particles, is knn_group.cu; its
+// autotuner times both): one warp serves 32 queries that are next to one another, so they
 // sit in one or two neighbouring leaves and want nearly the same nodes. The warp walks
 // the tree once for all of them (a node is opened when any lane still needs it), stages
 // each opened leaf's FP32 coordinates in shared memory, and every lane tests them against

@@ -1,10 +1,11 @@
 // Warp-per-query k-nearest-neighbour search: the kNN behind CalcDensityParticle,
 // CalcVelDensityParticle, FindNearest / FindNearestPos of given tree particles, the coordinate
-// forms (FindNearest(x), CalcDensityPosition, CalcVelDensityPosition), and the queries that
-// the group search (knn_group.cu) leaves. A warp for 32 consecutive points walked the tree
-// for all of them at once: with points in no spatial order every lane's neighbourhood was
-// opened for the whole warp (250,007 points, k = 40, in 500,009 particles: 145 ms; a warp a
-// point does not depend on their order).
+// forms (FindNearest(x), CalcDensityPosition, CalcVelDensityPosition) but for points near one
+// another with a small k (k_knn_points, knn.cu), and the queries that the group search
+// (knn_group.cu) leaves. A warp for any 32 consecutive points walked the tree for all of them at
+// once: with points in no spatial order every lane's neighbourhood was opened for the whole warp
+// (250,007 points, k = 40, in 500,009 particles: 145 ms; a warp a point does not depend on their
+// order).
 //
 // Replaces the depth-first search of SplitNode/LeafNode::FindNearestPos(target)
 // (src/KDTree/KDSplitNode.cxx:15-41, KDLeafNode.cxx:15-28) with its bounded max-heap

@@ -151,7 +151,8 @@ struct KnnArgs {
   double* vden;
   int* err;
   const double* qv;   // query velocities of coordinate queries (CalcVelDensityPosition)
-  int* fb;            // 1 + nq ints of scratch for the group search (null: a warp per query)
+  int* fb;            // scratch of the leftovers' list: 1 + nq ints for the group search, 5 +
+                      // nq / 16 for points (null: a warp per query)
   int slices, slice;  // kEpiSave over the particles [q0, q0 + nq) of the slice-th of 2^slices
                       // nodes of one level (0, 0: the whole tree)
 };

@@ -341,6 +341,7 @@ int launch_smooth(const SmoothArgs& s0, int which, DevAlloc& alloc, cudaStream_t
   if (which == kSmVelSkew || which == kSmVelKurt) parts.push_back({(void**)&iv, sizeof(V4) * n});
   if (which == kSmMeanOne || which == kSmDispOne) parts.push_back({(void**)&wt, sizeof(double) * n});
   if (every) parts.push_back({(void**)&fb, sizeof(int) * (step + 1)});
+  if (s0.k.qmode == 1) parts.push_back({(void**)&fb, sizeof(int) * (step / 16 + 5)});
   NBK_TRY(alloc.get_block(parts));
   if (sym) NBK_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(double) * width * n, st));
   Phase ph("smooth", st);
