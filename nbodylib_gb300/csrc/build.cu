@@ -102,7 +102,7 @@ struct NodeOut<3> {
     r.count = count;
     x.split_dim = dim;
     x.split_val = split_val;
-    x.pad = 0;
+    x.mixed = 0;
     node[idx] = r;
     nodex[idx] = x;
   }
@@ -1590,6 +1590,40 @@ int64_t count_nodes(int64_t n, int b) {
 }
 
 // Build every tree of the forest. All arrays live on `st`. Returns NBK status.
+// Whether the tree holds places of very different density: what decides, for trees of a middling
+// size, which of the neighbour searches is the faster one (group_lines, knn_group.cu). Such
+// places show in the boxes: the node three levels above one that holds 33 particles has 8 times
+// its volume where the particles lie evenly, and more than 256 times in 1% to 40% of the tree
+// where they are clustered (0 to 0.6% in a uniform box, a plane, a normal distribution). 512
+// places are looked at; the answer comes back with the root's box. (2 us of a build of 270;
+// asked by the search itself, it took 2 to 9 us of each one.)
+constexpr int kMixedSamples = 512, kMixedNode = 33;
+__global__ void __launch_bounds__(kMixedSamples) k_mixed(const NodeRec* node, NodeX* root, int n, int b) {
+  chain_wait();
+  const int i = (int)(((int64_t)threadIdx.x * n) / kMixedSamples);
+  int h = 0, s0 = 0, sz = n, lev = 0;
+  while (sz > b) {
+    const int ls = (sz - 1) / 2 + 1;  // KDTree.cxx:1012, 1025-1030
+    const int right = i >= s0 + ls;
+    if ((right ? sz - ls : ls) < kMixedNode) break;
+    if (right) s0 += ls;
+    sz = right ? sz - ls : ls;
+    h = 2 * h + 1 + right;
+    lev++;
+  }
+  bool mixed = false;
+  if (lev >= 3) {
+    const NodeRec r = node[h], up = node[((h + 1) >> 3) - 1];
+    float v = 1.f;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      if (r.hi[d] > r.lo[d]) v *= (up.hi[d] - up.lo[d]) / (r.hi[d] - r.lo[d]);
+    mixed = v > 256.f;
+  }
+  const int found = __syncthreads_count(mixed);
+  if (threadIdx.x == 0) root->mixed = found > kMixedSamples / 64;
+}
+
 template <int ND>
 static int build_forest_t(const std::vector<TreeSpec>& trees, int b, const double* d_pos_in,
                           const double* d_mass_in, const double* d_vel_in, NodeOut<ND> nout,
@@ -1823,6 +1857,11 @@ static int build_forest_t(const std::vector<TreeSpec>& trees, int b, const doubl
     NBK_TRY(ensure_dyn_smem((const void*)k_local_build<ND>, (int)sm));
     NBK_CUDA_TRY(launch_chain(k_local_build<ND>, (unsigned)nroots, kLocalThreads, sm, st, d_r, Ca,
                               IDa, Cb, IDb, cs, d_mass_in, d_vel_in, b, nout, pout, d_err, (int)p0));
+  }
+  if constexpr (ND == 3) {
+    if (root_out && trees.size() == 1 && trees[0].n >= kGroupSmallest && trees[0].n < kGroupMixedMax)
+      NBK_CUDA_TRY(launch_chain(k_mixed, 1, kMixedSamples, 0, st, nout.node + trees[0].nbase,
+                                nout.nodex + trees[0].nbase, (int)trees[0].n, b));
   }
   if (root_out && root_src)
     NBK_CUDA_TRY(cudaMemcpyAsync(root_out, root_src, root_bytes, cudaMemcpyDeviceToHost, st));

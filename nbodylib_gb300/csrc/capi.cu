@@ -371,6 +371,7 @@ struct nbk_tree {
   double* d_kernel = nullptr;
   float eps = 0;
   float eps6[6] = {0, 0, 0, 0, 0, 0};
+  int mixed = 0;  // k_mixed (build.cu)
   int* d_err = nullptr;
   void* block = nullptr;  // the one device allocation holding every array above
   bool dev() const { return flags & NBK_DEVICE_PTRS; }
@@ -517,6 +518,7 @@ KnnArgs base_args(nbk_tree* t) {
   a.kernel = t->d_kernel;
   a.kernres = t->kernres;
   a.err = t->d_err;
+  a.mixed = t->mixed;
   return a;
 }
 
@@ -818,6 +820,7 @@ int nbk_create(const double* pos, const double* vel, const double* mass, int64_t
     if (treetype == NBK_TVEL) std::swap(d_pos, d_vel);
     NodeX root;
     NBK_TRY(build_forest(trees, bucket_size, d_pos, d_mass, d_vel, A, alloc, st, &root));
+    t->mixed = root.mixed;
     for (int d = 0; d < 3; d++) {
       rlo[d] = root.lo[d];
       rhi[d] = root.hi[d];
@@ -962,7 +965,7 @@ int nbk_knn(nbk_tree* t, int k, int variant, int periodic_mode, int32_t* nn, dou
   a.nq = (int)t->n;
   a.nn = dnn;
   a.d2 = dd2;
-  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
+  if (t->n >= kGroupSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, kEpiNN, t->st));
   NBK_TRY(S.finish());
   if (!t->dev()) NBK_TRY(check_err(t, "nbk_knn"));
@@ -1196,7 +1199,7 @@ static int density_common(nbk_tree* t, int k, int nsmooth, double* rho, double* 
   a.nsmooth = nsmooth;
   a.rho = trho;
   a.vden = tv;
-  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
+  if (t->n >= kGroupSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, epi, t->st));
   if (rho) NBK_TRY(scatter_to_input_order(trho, t->arr.perm, drho, t->n, 1, t->st));
   if (vden) NBK_TRY(scatter_to_input_order(tv, t->arr.perm, dv, t->n, 1, t->st));
@@ -1914,7 +1917,7 @@ int nbk_density_adjoint(nbk_tree* t, int k, const double* w, double* rho, double
   a.nq = (int)t->n;
   a.rho = trho;
   a.nn = nn;
-  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
+  if (t->n >= kGroupSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, kEpiDensSave, t->st));
   k_gather_d<<<(unsigned)((t->n + 255) / 256), 256, 0, t->st>>>(dw, t->arr.perm, tw, t->n);
   note_launch();

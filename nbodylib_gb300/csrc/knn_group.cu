@@ -1061,18 +1061,41 @@ int launch_knn_group_batch(const KnnArgs& a, const BatchArgs& b, cudaStream_t st
   return launch_group_batch<4>(a, b, st);
 }
 
+// From how many particles on the groups are faster than a warp per query, where the particles
+// lie evenly and where they are clustered (k_mixed, build.cu). A group's warp serves its queries
+// one after another, and a group that lies partly in a much denser place takes many times as
+// long as the others: fewer groups than the SMs have room for hide neither. The search's own work
+// decides where: the sums cost a group less than its queries alone, sorted rows and image passes
+// do not, and a warp per query holds more than 64 neighbours in four slots.
+// Measured (time of a warp per query over the groups' time, k = 8, 32, 64; uniform, normal,
+// Plummer sphere, 500 spheres, 8 spheres in a background):
+//   density   16,384: 1.29 1.14 1.60, 1.22 1.07 1.16, 1.03 0.76 0.85, 0.94 0.91 0.88, 0.84 0.71 0.77
+//             49,152: 1.68 1.80 1.58, 1.50 1.47 1.39, 1.27 1.12 1.13, 1.06 1.08 1.13, 0.91 0.87 0.95
+//   rows      24,576: 1.33 1.25 1.30, 1.06 1.06 1.08, 0.88 0.81 0.81, 0.74 0.65 0.74, 0.68 0.64 0.72
+//             98,304: 1.50 1.91 1.50, 1.43 1.53 1.25, 1.28 1.27 1.19, 1.02 1.07 1.07, 0.98 0.91 0.91
+//   images    32,768: 1.13 1.12, 0.92 1.10, 0.71 0.78, 0.82 0.83, 0.65 0.81 (k = 8 and 32)
+//             98,304: 1.41 1.79, 1.34 1.64, 1.25 1.31, 1.09 1.19, 1.03 1.00
+//    k = 48   65,536: 1.18, 1.15, 0.95, 0.87, 0.71; 131,072: 1.25, 1.20, 1.10, 0.92, 0.93
+//   k = 100    8,192: density 5.17 uniform, 2.25 in 500 spheres, 1.25 in 8; images 2.48, 1.54, 1.03
+namespace {
+struct GroupLines {
+  int even, mixed;
+};
+GroupLines group_lines(const KnnArgs& a, int epi) {
+  if (a.kheap > 64) return {kGroupSmallest, kGroupSmallest};
+  if (epi != kEpiNN) return {16384, 49152};
+  if (!a.periodic) return {24576, 98304};
+  return a.kheap <= 33 ? GroupLines{32768, 98304} : GroupLines{65536, 163840};
+}
+}  // namespace
+
 // Every particle of a tree (or a slice of it), none of them given zero-distance or image
 // answers that FP32 offsets cannot tell apart, k within the buffers, squares inside FP32.
-// Below kGrpMin particles there are too few groups to fill the SMs with the warps that a group
-// needs one after another, and a warp per query ends sooner. (Density of clustered particles,
-// group and warp per query: 5,459 with k = 21 69 and 46 us; 20,001 with k = 32 179 and 149;
-// 32,769 with k = 8 128 and 145, k = 32 198 and 192, k = 64 273 and 278, uniform 98 and 178;
-// 65,537 with k = 32 302 and 346; 2^20 3.0 and 5.4 ms.)
-constexpr int kGrpMin = 32768;
-bool group_search_serves(const KnnArgs& a) {
+bool group_search_serves(const KnnArgs& a, int epi) {
   const int K = a.periodic ? a.kheap - 1 : a.kheap;
   return a.qmode == 0 && a.fb && (a.nq == a.tv.n || a.slices > 0) && a.kheap <= 128 && K >= 1 &&
-         a.tv.n >= kGrpMin && a.tv.eps < 1e11f &&
+         a.tv.n >= (a.mixed ? group_lines(a, epi).mixed : group_lines(a, epi).even) &&
+         a.tv.eps < 1e11f &&
          (a.periodic ? a.tv.n <= (1 << kGrpImage) : a.exclude_self != 0);
 }
 

@@ -153,12 +153,15 @@ struct KnnArgs {
   const double* qv;   // query velocities of coordinate queries (CalcVelDensityPosition)
   int* fb;            // scratch of the leftovers' list: 1 + nq ints for the group search, 5 +
                       // nq / 16 for points (null: a warp per query)
+  int mixed;          // places of very different density in the tree (k_mixed)
   int slices, slice;  // kEpiSave over the particles [q0, q0 + nq) of the slice-th of 2^slices
                       // nodes of one level (0, 0: the whole tree)
 };
 int launch_knn(const KnnArgs& a, int epi, cudaStream_t st);
 // The group search (knn_group.cu): every particle of a tree at once.
-bool group_search_serves(const KnnArgs& a);
+constexpr int kGroupSmallest = 8192;    // never below this many particles, and from
+constexpr int kGroupMixedMax = 163840;  // here on whatever the tree holds
+bool group_search_serves(const KnnArgs& a, int epi);
 int launch_knn_group(const KnnArgs& a, int epi, cudaStream_t st);
 
 // ---- phase-space trees (phase.cu)

@@ -48,7 +48,7 @@ struct NodeX {
   double lo[3], hi[3];  // exact FP64 bounding box (min/max of the node's particles)
   double split_val;     // coordinate of the median particle (the reference's cut_val)
   int split_dim;        // -1 for a leaf
-  int pad;
+  int mixed;            // of a root: places of very different density below (k_mixed, build.cu)
 };
 
 // Phase-space (six-dimensional) tree nodes, heap-indexed like the physical ones: the

@@ -1,9 +1,8 @@
-"""Periodic neighbour lists of every particle by the group search (its trees start at 32,768
-particles at the latest): the reference's image gates against the restatement, the minimum
-image against the search of given targets, a warp each, and against brute force; at the slot
-switches of k, sides as short as the lists are wide (a particle's own images among its
-neighbours, groups on both sides of a half period, images searched with larger offsets than the
-group's own) and groups on a wall."""
+"""Periodic neighbour lists of every particle by the group search (70,001 uniform particles):
+the reference's image gates against the restatement, the minimum image against the search of
+given targets, a warp each, and against brute force; at the slot switches of k, sides as short
+as the lists are wide (a particle's own images among its neighbours, groups on both sides of a
+half period, images searched with larger offsets than the group's own) and groups on a wall."""
 import numpy as np
 import pytest
 
@@ -13,7 +12,7 @@ from tests.helpers import assert_knn_equal, d2_ref, reflect_images, rows_by_id, 
 
 pytestmark = pytest.mark.gpu
 
-N = 40009
+N = 70001
 CASES = [([1.0, 1.0, 1.0], 31), ([1.0, 1.0, 1.0], 33), ([1.0, 0.25, 2.0], 32),
          ([1.0, 1.0, 0.01], 32), ([1.0, 1.0, 0.01], 64), ([1.0, 1.0, 2e-3], 31),
          ([1.0, 1.0, 1e-6], 16), ([1.0, 0.02, 0.02], 32), ([1.0, 0.01, 0.03], 100)]

@@ -1,5 +1,5 @@
 """Kernel tables of more cells than 2^20 and 2^21: the cell of every neighbour and with it the
-densities and smoothed fields, by the group search (40,009 particles) and the search below it."""
+densities and smoothed fields, by the group search (70,001 particles) and the search below it."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ from tests.helpers import assert_density_close
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [2001, 40009])
+@pytest.mark.parametrize("n", [2001, 70001])
 @pytest.mark.parametrize("kernres", [(1 << 20) + 7, 3 << 20, (1 << 22) + 5])
 def test_large_tables(gpu, port_built, n, kernres):
     k = 16

@@ -1,4 +1,4 @@
-"""The smoothing family over rows of the group search (40,009 particles), its row lengths at the
+"""The smoothing family over rows of the group search (70,001 particles), its row lengths at the
 slot switches, against the restatement: 1e-12 of the largest magnitude, as the path's."""
 import numpy as np
 import pytest
@@ -19,7 +19,7 @@ def close(got, want, what):
 
 @pytest.mark.parametrize("k", [16, 32, 33, 65])
 def test_every_particle(gpu, port_built, k):
-    pos, mass, vel = syn.clustered_box(40009, 80.0, seed=31 + k, velocities=True)
+    pos, mass, vel = syn.clustered_box(70001, 80.0, seed=31 + k, velocities=True)
     # ten particles too close for FP32: the group search leaves them to its list (no two at one
     # place: which of them is the k-th then is open, and the kurtosis subtracts 3 in each term)
     pos[1000:1010] = pos[1000] + np.random.default_rng(k).normal(size=(10, 3)) * 1e-9
@@ -36,7 +36,7 @@ def test_every_particle(gpu, port_built, k):
           o.smooth_vel_moments(3, k, rho, mean, disp), "CalcSmoothVelKurtosis")
     # the same query's value by the search of given targets, a warp each
     every = t.CalcVelDensityWithPhysDensity(k, k, rho=rho)
-    targets = np.arange(0, 40009, 7, dtype=np.int32)
+    targets = np.arange(0, 70001, 7, dtype=np.int32)
     one = t.CalcVelDensityWithPhysDensityParticle(targets, k, k, rho=rho)
     np.testing.assert_allclose(np.asarray(every)[t.GetPerm()[targets]], one, rtol=1e-12)
     t.close()
