@@ -1704,7 +1704,7 @@ int nbk_fof(nbk_tree* t, double fdist, int32_t minnum, int order, int32_t* group
   int ng = 0;
   // the group count and the error word come back together, in one synchronisation
   PinnedScalars* ps = order == 0 ? pinned_scalars() : nullptr;
-  NBK_TRY(run_fof(a, (int)t->nslots, minnum, order, gtree, ps ? &ps->i[0] : &ng, S.alloc, t->st,
+  NBK_TRY(run_fof(a, minnum, order, gtree, ps ? &ps->i[0] : &ng, S.alloc, t->st,
                   ps != nullptr));
   if (t->n > 0) {
     NBK_CUDA_TRY(launch_chain(k_scatter_i, (unsigned)((t->n + 255) / 256), 256, 0, t->st, gtree,
@@ -1781,7 +1781,7 @@ int nbk_fof_criterion(nbk_tree* t, int comparator, const double* params, int32_t
   a.parent = parent;
   a.err = t->d_err;
   int ng = 0;
-  NBK_TRY(run_fof(a, (int)t->nslots, minnum, order, gtree, &ng, S.alloc, t->st));
+  NBK_TRY(run_fof(a, minnum, order, gtree, &ng, S.alloc, t->st));
   k_scatter_i<<<(unsigned)((t->n + 255) / 256), 256, 0, t->st>>>(gtree, t->arr.perm, dg, t->n);
   note_launch();
   NBK_CUDA_TRY(cudaGetLastError());
@@ -1849,7 +1849,7 @@ static int fof_nn_common(nbk_tree* t, int comparator, const double* params, int 
   for (int k = 0; k < npc; k++) a.pidx[k] = pi[k];
   int ng = 0;
   // groups are numbered by decreasing size, as the reference's (KDFOF.cxx:493-503)
-  NBK_TRY(run_fof(a, (int)t->nslots, minnum, 1, gtree, &ng, S.alloc, t->st));
+  NBK_TRY(run_fof(a, minnum, 1, gtree, &ng, S.alloc, t->st));
   k_scatter_i<<<(unsigned)((t->n + 255) / 256), 256, 0, t->st>>>(gtree, t->arr.perm, dg, t->n);
   note_launch();
   NBK_CUDA_TRY(cudaGetLastError());

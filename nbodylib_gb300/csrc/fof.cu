@@ -1101,9 +1101,8 @@ static int link_fof6d_phase_tree(const FofArgs& a, DevAlloc& alloc, cudaStream_t
   return NBK_OK;
 }
 
-int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tree,
+int run_fof(const FofArgs& a, int minnum, int order, int* d_group_tree,
             int* h_ngroup, DevAlloc& alloc, cudaStream_t st, bool defer_count) {
-  (void)nnodes;
   int n = a.tv.n;
   if (n == 0) {
     *h_ngroup = 0;

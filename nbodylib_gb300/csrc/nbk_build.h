@@ -250,7 +250,7 @@ struct FofArgs {
   int qpw;             // queries per warp of the link kernels (set by run_fof)
   int fp32_weights;    // FOF6d: the weights are normal FP32 numbers (set by run_fof)
 };
-int run_fof(const FofArgs& a, int nnodes, int minnum, int order, int* d_group_tree,
+int run_fof(const FofArgs& a, int minnum, int order, int* d_group_tree,
             int* h_ngroup, DevAlloc& alloc, cudaStream_t st,
             bool defer_count = false);
 

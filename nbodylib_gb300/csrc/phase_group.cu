@@ -50,8 +50,6 @@ constexpr int kPgStack = 192;
 // nodes tested per step (2^18 clustered particles, k = 32: 32 at once 29 ms, 16 13 ms: the
 // frontier grows before the K-th distances have shrunk)
 constexpr int kPgPop = 16;
-// home holds at least this many times K particles (2 and 4 times were no faster)
-constexpr int kPgSeed = 1;
 
 // One query's row in shared memory.
 struct __align__(16) PgQuery {
@@ -368,8 +366,9 @@ __global__ void __launch_bounds__(32 * kPgWpb, 5) k_phase_group(PhaseArgs pa, Pg
   if (g >= (1 << depth)) return;
   constexpr int G = GrpCfg<S>::G;
   const int K = a.kheap;
-  // the group, and the smallest real node around it with more than K (and 8) particles
-  const int want = kPgSeed * max(max(K + 1, G), 9);
+  // the group, and the smallest real node around it with more than K (and 8) particles (2 and 4
+  // times as many were no faster)
+  const int want = max(max(K + 1, G), 9);
   int s0 = 0, sz = tv.n, hh = 0, hs = 0, hn = tv.n, lev = 0;
   for (int i = depth - 1; i >= 0; i--) {
     const int ls0 = (sz - 1) / 2 + 1;
