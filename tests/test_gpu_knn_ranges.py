@@ -38,3 +38,21 @@ def test_rows_and_densities(gpu, port_built, n, box, periodic):
         assert_density_close(np.asarray(batch.density(k, use_graph=False)), want)
     batch.close()
     t.close()
+
+
+@pytest.mark.parametrize("box", [1e-6, 1e-12, 1e-15, 1e-20])
+def test_small_boxes(gpu, port_built, box):
+    """Distances whose squares fall below FP32's range, one tree and a batch."""
+    n, k = 40009, 16
+    pos = np.random.default_rng(22).random((n, 3)) * box
+    o = oracle.OracleTree(pos, None, np.ones(n), 16, 0, 0, 1000, None, backend="port", nthreads=8)
+    t = KDTree(pos, None, np.ones(n), 16, kerntype=0)
+    nn, d2 = t.FindNearest(k)
+    perm = t.GetPerm()
+    assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), *o.knn(k, 0))
+    want = o.density(k)
+    assert_density_close(t.CalcDensity(k), want)
+    t.close()
+    batch = BatchedDensity(pos, np.ones(n), np.array([0, n], np.int64), bucket_size=16)
+    assert_density_close(np.asarray(batch.density(k, use_graph=False)), want)
+    batch.close()
