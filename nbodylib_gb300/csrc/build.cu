@@ -1599,7 +1599,6 @@ int64_t count_nodes(int64_t n, int b) {
 // asked by the search itself, it took 2 to 9 us of each one.)
 constexpr int kMixedSamples = 512, kMixedNode = 33;
 __global__ void __launch_bounds__(kMixedSamples) k_mixed(const NodeRec* node, NodeX* root, int n, int b) {
-  chain_wait();
   const int i = (int)(((int64_t)threadIdx.x * n) / kMixedSamples);
   int h = 0, s0 = 0, sz = n, lev = 0;
   while (sz > b) {
@@ -1611,6 +1610,7 @@ __global__ void __launch_bounds__(kMixedSamples) k_mixed(const NodeRec* node, No
     h = 2 * h + 1 + right;
     lev++;
   }
+  chain_wait();  // (the place's node comes from the tree's sizes alone)
   bool mixed = false;
   if (lev >= 3) {
     const NodeRec r = node[h], up = node[((h + 1) >> 3) - 1];
