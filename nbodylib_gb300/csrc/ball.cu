@@ -16,8 +16,9 @@
 // (in tree order: the leaves ahead of the first inner node are tested, what follows is pushed
 // back), leaf particles are tested a lane each, two leaves at a time, one query after another
 // of those that want the leaf, and one round-to-nearest distance decides outside a band of
-// its own rounding error around the radius: 1.50 ms (both passes; 32 warps per SM, 1.53 ms
-// with 40, which spills).
+// its own rounding error around the radius (FP64 for all where squares leave FP32's range,
+// fp32_band): 1.50 ms (both passes; 32 warps per SM at 64 registers and some 70 bytes of spills;
+// with 40, which spill more, 1.53 ms).
 #include "nbk_build.h"
 
 namespace nbk {

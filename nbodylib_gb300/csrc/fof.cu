@@ -163,7 +163,7 @@ __device__ __forceinline__ bool crit_cmp(int cmp, const double* p, const double 
 // query after another of those that want the leaf: with a query per lane instead, half the
 // lanes had no query that wanted the leaf. A round-to-nearest distance decides outside a
 // band of its own rounding error around the linking length (squared: `near2` and `far2`);
-// pairs inside the band take FP64. 2^20 clustered particles: 1.55 -> 1.01 ms (blocks of 4
+// pairs inside the band, and all pairs where squares leave FP32's range (fp32_band), take FP64. 2^20 clustered particles: 1.55 -> 1.01 ms (blocks of 4
 // warps, 40 warps per SM; 1.23 at 32), bound by instruction issue.
 //
 // CRIT3D: FOFCriterion with FOF3d inside its search region, run as FOF with
@@ -1017,8 +1017,8 @@ __global__ void k_relabel(int* group, const int* newlbl, int n) {
 
 // Queries per warp of the link kernels (a lane each; the other lanes still take nodes and
 // candidates): as many as 32 where that leaves enough warps for every SM (linking 5,003
-// particles: 0.24 ms with 32 a warp, 0.16 with the 2 of this rule; 2^20: 1.23 ms with 32,
-// 1.30 with 16, 1.66 with 8, before the blocks of 4 warps).
+// particles: 0.24 ms with 32 a warp, 0.07 with the 2 of this rule; 65,537: 0.39 and 0.23; 2^20:
+// 1.23 ms with 32, 1.30 with 16, 1.66 with 8, before the blocks of 4 warps).
 constexpr int kQpwMax = 32, kQpwMin = 2;
 int queries_per_warp(int64_t n, int* qpw) {
   int dev = 0, nsm = 0;
