@@ -1052,7 +1052,7 @@ int nbk_knn_points(nbk_tree* t, const double* x, int64_t nq, int k, int periodic
   a.nq = (int)nq;
   a.nn = dnn;
   a.d2 = dd2;
-  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (nq / 16 + 5)));
+  if (nq >= kPointsSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (nq / 16 + 5)));
   NBK_TRY(launch_knn(a, kEpiNN, t->st));
   NBK_TRY(S.finish());
   if (!t->dev()) NBK_TRY(check_err(t, "nbk_knn_points"));
@@ -1093,7 +1093,7 @@ int nbk_knn_coords(nbk_tree* t, const double* x, int64_t nq, int k, int32_t* nn,
     a.nq = (int)nq;
     a.nn = dnn;
     a.d2 = dd2;
-    NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (nq / 16 + 5)));
+    if (nq >= kPointsSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (nq / 16 + 5)));
     NBK_TRY(launch_knn(a, kEpiNN, t->st));
   }
   NBK_TRY(S.finish());
@@ -1574,7 +1574,7 @@ static int positions_common(nbk_tree* t, const double* x, const double* v, int64
   a.nsmooth = nsmooth;
   a.rho = dout;
   a.vden = dout;
-  NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (nq / 16 + 5)));
+  if (nq >= kPointsSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (nq / 16 + 5)));
   NBK_TRY(launch_knn(a, epi, t->st));
   NBK_TRY(S.finish());
   if (!t->dev()) NBK_TRY(check_err(t, "position density"));

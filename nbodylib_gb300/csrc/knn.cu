@@ -211,7 +211,7 @@ constexpr int kPointsHomes = 2;
 // 262,144 1.42 and 1.30, 0.91 and 1.38; 2^20 5.46 and 5.13, 2.29 and 4.77; k = 24, 262,144 1.61
 // and 1.47, 1.28 and 1.68.
 constexpr int kPointsK = 16, kPointsMin = 1 << 19;
-constexpr int kPointsShortK = 12, kPointsShortMin = 1 << 17;
+constexpr int kPointsShortK = 12, kPointsShortMin = kPointsSmallest;
 
 inline bool points_share_warps(const KnnArgs& a) {
   return a.qmode == 1 && a.fb &&

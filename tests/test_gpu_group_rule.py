@@ -56,3 +56,20 @@ def test_with_images(gpu, port_built, kind, n, k):
     nn, d2 = t.FindNearest(k)
     assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), *o.knn(k, 0), kind)
     t.close()
+
+
+@pytest.mark.parametrize("n", [8193, 24577])
+def test_velocity_tree(gpu, port_built, n):
+    """The same searches over velocities, and many points in velocity space."""
+    from nbodylib_gb300.kdtree import TVEL
+    rng = np.random.default_rng(n)
+    pos, vel = rng.random((n, 3)), rng.normal(size=(n, 3))
+    o = oracle.OracleTree(vel, None, np.ones(n), 16, 0, 0, 1000, None, backend="port", nthreads=16)
+    t = KDTree(pos, vel, np.ones(n), 16, treetype=TVEL, kerntype=0)
+    perm = t.GetPerm()
+    nn, d2 = t.FindNearestVel(16)
+    assert_knn_equal(rows_by_id(to_ids(nn, perm), perm), rows_by_id(d2, perm), *o.knn(16, 0))
+    x = np.repeat(vel[perm], (1 << 17) // n + 1, axis=0) + 1e-4
+    nn, d2 = t.FindNearestPoints(x, 8)
+    assert_knn_equal(to_ids(nn, perm), d2, *o.knn_pos(x, 8))
+    t.close()
