@@ -1859,7 +1859,7 @@ static int build_forest_t(const std::vector<TreeSpec>& trees, int b, const doubl
                               IDa, Cb, IDb, cs, d_mass_in, d_vel_in, b, nout, pout, d_err, (int)p0));
   }
   if constexpr (ND == 3) {
-    if (root_out && trees.size() == 1 && trees[0].n >= kGroupSmallest && trees[0].n < kGroupMixedMax)
+    if (root_out && trees.size() == 1 && trees[0].n >= kGroupMixedMin && trees[0].n < kGroupMixedMax)
       NBK_CUDA_TRY(launch_chain(k_mixed, 1, kMixedSamples, 0, st, nout.node + trees[0].nbase,
                                 nout.nodex + trees[0].nbase, (int)trees[0].n, b));
   }

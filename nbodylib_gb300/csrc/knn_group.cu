@@ -1084,9 +1084,9 @@ struct GroupLines {
 };
 GroupLines group_lines(const KnnArgs& a, int epi) {
   if (a.kheap > 64) return {kGroupSmallest, kGroupSmallest};
-  if (epi != kEpiNN) return {16384, 49152};
+  if (epi != kEpiNN) return {kGroupMixedMin, 49152};
   if (!a.periodic) return {24576, 98304};
-  return a.kheap <= 33 ? GroupLines{32768, 98304} : GroupLines{65536, 163840};
+  return a.kheap <= 33 ? GroupLines{32768, 98304} : GroupLines{65536, kGroupMixedMax};
 }
 }  // namespace
 

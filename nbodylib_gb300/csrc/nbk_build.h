@@ -159,8 +159,9 @@ struct KnnArgs {
 };
 int launch_knn(const KnnArgs& a, int epi, cudaStream_t st);
 // The group search (knn_group.cu): every particle of a tree at once.
-constexpr int kGroupSmallest = 8192;    // never below this many particles, and from
-constexpr int kGroupMixedMax = 163840;  // here on whatever the tree holds
+constexpr int kGroupSmallest = 8192;    // never below this many particles; from kGroupMixedMin
+constexpr int kGroupMixedMin = 16384;   // to kGroupMixedMax it depends on what the tree holds
+constexpr int kGroupMixedMax = 163840;
 constexpr int kPointsSmallest = 1 << 17;  // points, from here on, may share warps (knn.cu)
 bool group_search_serves(const KnnArgs& a, int epi);
 int launch_knn_group(const KnnArgs& a, int epi, cudaStream_t st);
