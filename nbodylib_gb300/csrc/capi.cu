@@ -965,7 +965,8 @@ int nbk_knn(nbk_tree* t, int k, int variant, int periodic_mode, int32_t* nn, dou
   a.nq = (int)t->n;
   a.nn = dnn;
   a.d2 = dd2;
-  if (t->n >= kGroupSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
+  if (group_search_serves(a, kEpiNN))
+    NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, kEpiNN, t->st));
   NBK_TRY(S.finish());
   if (!t->dev()) NBK_TRY(check_err(t, "nbk_knn"));
@@ -1199,7 +1200,8 @@ static int density_common(nbk_tree* t, int k, int nsmooth, double* rho, double* 
   a.nsmooth = nsmooth;
   a.rho = trho;
   a.vden = tv;
-  if (t->n >= kGroupSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
+  if (group_search_serves(a, epi))
+    NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, epi, t->st));
   if (rho) NBK_TRY(scatter_to_input_order(trho, t->arr.perm, drho, t->n, 1, t->st));
   if (vden) NBK_TRY(scatter_to_input_order(tv, t->arr.perm, dv, t->n, 1, t->st));
@@ -1917,7 +1919,8 @@ int nbk_density_adjoint(nbk_tree* t, int k, const double* w, double* rho, double
   a.nq = (int)t->n;
   a.rho = trho;
   a.nn = nn;
-  if (t->n >= kGroupSmallest) NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
+  if (group_search_serves(a, kEpiDensSave))
+    NBK_TRY(S.alloc.get((void**)&a.fb, sizeof(int) * (t->n + 1)));
   NBK_TRY(launch_knn(a, kEpiDensSave, t->st));
   k_gather_d<<<(unsigned)((t->n + 255) / 256), 256, 0, t->st>>>(dw, t->arr.perm, tw, t->n);
   note_launch();

@@ -317,7 +317,7 @@ int launch_points(const KnnArgs& a, cudaStream_t st) {
 
 template <int EPI>
 int launch_e(const KnnArgs& a, cudaStream_t st) {
-  if (EPI != kEpiDensPart && EPI != kEpiVelPart && group_search_serves(a, EPI))
+  if (EPI != kEpiDensPart && EPI != kEpiVelPart && a.fb && group_search_serves(a, EPI))
     return launch_knn_group(a, EPI, st);
   if constexpr (EPI == kEpiNN || EPI == kEpiDensPart || EPI == kEpiVelPart || EPI == kEpiSave) {
     if (points_share_warps(a)) return launch_points<kPointsK, EPI>(a, st);

@@ -1096,7 +1096,7 @@ GroupLines group_lines(const KnnArgs& a, int epi) {
 // particles in a box of 1e-14 7.4 ms by groups, 5.8 a warp each).
 bool group_search_serves(const KnnArgs& a, int epi) {
   const int K = a.periodic ? a.kheap - 1 : a.kheap;
-  return a.qmode == 0 && a.fb && (a.nq == a.tv.n || a.slices > 0) && a.kheap <= 128 && K >= 1 &&
+  return a.qmode == 0 && (a.nq == a.tv.n || a.slices > 0) && a.kheap <= 128 && K >= 1 &&
          a.tv.n >= (a.mixed ? group_lines(a, epi).mixed : group_lines(a, epi).even) &&
          a.tv.eps < 1e11f && a.tv.eps > 1e-19f &&
          (a.periodic ? a.tv.n <= (1 << kGrpImage) : a.exclude_self != 0);

@@ -158,7 +158,7 @@ struct KnnArgs {
                       // nodes of one level (0, 0: the whole tree)
 };
 int launch_knn(const KnnArgs& a, int epi, cudaStream_t st);
-// The group search (knn_group.cu): every particle of a tree at once.
+// The group search (knn_group.cu): every particle of a tree at once, with a.fb.
 constexpr int kGroupSmallest = 8192;    // never below this many particles; from kGroupMixedMin
 constexpr int kGroupMixedMin = 16384;   // to kGroupMixedMax it depends on what the tree holds
 constexpr int kGroupMixedMax = 163840;
